@@ -236,8 +236,8 @@ int gtls_set_tuning(gtls_ctx* ctx, const gtls_tuning* t) {
     return fail(ctx, GTLS_E_INVALID, "tile caps must be 0 or multiples of 256 in [256, 65536]");
   if (t->bucket_shift < -3 || t->bucket_shift > 0) return fail(ctx, GTLS_E_INVALID, "bucket_shift must be in [-3, 0]");
   if (t->records_global != 0 && t->records_global != 1) return fail(ctx, GTLS_E_INVALID, "records_global must be 0 or 1");
-  ctx->tile_cap_fp32 = t->tile_cap_fp32 ? t->tile_cap_fp32 : 16384;
-  ctx->tile_cap_fp64 = t->tile_cap_fp64 ? t->tile_cap_fp64 : 8192;
+  ctx->tile_cap_fp32 = t->tile_cap_fp32 ? t->tile_cap_fp32 : kTileCapFp32;
+  ctx->tile_cap_fp64 = t->tile_cap_fp64 ? t->tile_cap_fp64 : kTileCapFp64;
   ctx->bucket_shift = t->bucket_shift;
   ctx->records_global = t->records_global;
   return GTLS_OK;
@@ -293,11 +293,6 @@ int gtls_ctx_create(int device, gtls_ctx** out) {
   c->device = device;
   c->num_sms = prop.multiProcessorCount;
   c->smem_optin = (int)prop.sharedMemPerBlockOptin;
-  if (cudaMalloc(&c->status, 64) != cudaSuccess) {
-    delete c;
-    return fail(nullptr, GTLS_E_NOMEM, "status word allocation failed");
-  }
-  cudaMemset(c->status, 0, 64);
   *out = c;
   return GTLS_OK;
 }
@@ -307,7 +302,6 @@ int gtls_ctx_destroy(gtls_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   if (ctx->arena) cudaFree(ctx->arena);
-  if (ctx->status) cudaFree(ctx->status);
   delete ctx;
   return GTLS_OK;
 }

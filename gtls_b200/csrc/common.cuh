@@ -7,6 +7,11 @@
 
 #include "gtls_b200.h"
 
+namespace gtls {
+// Default tile caps: "the library's own split of a period's starts".
+constexpr int kTileCapFp32 = 16384, kTileCapFp64 = 8192;
+}  // namespace gtls
+
 struct gtls_ctx {
   int device = 0;
   int num_sms = 0;
@@ -14,13 +19,13 @@ struct gtls_ctx {
   std::string err;
   void* arena = nullptr;       // scratch arena (grows on demand)
   size_t arena_bytes = 0;
-  int* status = nullptr;       // device status word(s) written by kernels
   long long launches = 0;      // kernels launched through this context
   size_t chunk_budget = (size_t)8 << 30;   // per-chunk scratch of a search, bytes
-  int tile_cap_fp32 = 16384;   // launch-shape tuning (gtls_set_tuning); results do not depend on it
-  int tile_cap_fp64 = 8192;
+  int tile_cap_fp32 = gtls::kTileCapFp32;   // launch-shape tuning (gtls_set_tuning); results do not depend on it
+  int tile_cap_fp64 = gtls::kTileCapFp64;
   int bucket_shift = 0;
-  int records_global = 0;      // 1: chi2 reads records from global memory for every curve
+  int records_global = 0;      // accepted and reported; the records are always read through L2
+  bool smem_set_fp32 = false, smem_set_fp64 = false;   // the search kernels' shared memory has been allowed
 };
 
 namespace gtls {

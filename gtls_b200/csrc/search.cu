@@ -15,30 +15,24 @@
 //
 //   chi2(d,k) = E + c (2 B_k + c C_k),  B_k = sum_i s_i u_{k+i},  C_k = sum_i s_i^2 w_{k+i}
 //
-// which is what these kernels evaluate.  B and C are sliding correlations of
-// the template with the folded (u, w) records; the work is FMA-bound and runs
-// on the FP64 or FP32 pipes (nothing here is a dense contraction, so no tensor
-// cores).  The mean depth comes from prefix sums of v (FP64; stored as
-// float-float pairs in the FP32 form).  Only starts k that are multiples of
-// skip(d) = w / skip_point (for w > skip_point) are evaluated in the main pass
-// (GPUFun.py:402,409); every other (d,k) carries the value n
-// (GPUFun.py:407,437), which takes part in the minimum like any value.
+// with B and C sliding correlations of the template with the folded (u, w)
+// records.  Only the minimum over (d, k) is wanted, so every start is first
+// bounded from block sums and only those that can hold the minimum get their
+// sums (screen.cuh, chi2.cuh).  A start whose window mean fails the depth test
+// carries the value n (GPUFun.py:407,437), and so do the starts that are not
+// multiples of skip(d) = w / skip_point (for w > skip_point) in the main pass
+// (GPUFun.py:402,409).
 //
 // Kernels:
-//   curve_setup_kernel   (v, w) records per original sample and E.
-//   prepare_kernel       one CTA per period: FP64 fold (GPUFun.py:30-41),
-//                        stable bucket ranking of the phases (cupy argsort),
-//                        each ranked sample written straight to its place in
-//                        the padded sorted record array (patchData
-//                        GPUFun.py:110-129), then the prefix of v.
-//   chi2_kernel          one CTA per (period, tile of starts): the tile of
-//                        records is staged in shared memory, warps pull
-//                        (duration, start-group) tasks from a CTA-local queue,
-//                        register-blocked correlations produce B, C for R
-//                        starts at a time, each CTA keeps its (min, argmin).
-//   finish_kernel        per-period minimum over tiles (first occurrence).
+//   curve_setup_kernel   (v, w) records per original sample and their sums.
+//   prepare_kernel       one CTA per period: FP64 fold (GPUFun.py:30-41) and
+//                        stable bucket ranking of the phases (cupy argsort):
+//                        the original index of every sorted position.
+//   chi2_kernel          one CTA per (period, range of starts): (min, argmin).
+//   finish_kernel        per-period minimum over ranges (first occurrence).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdint>
@@ -47,7 +41,7 @@
 
 #include "chi2_core.cuh"
 #include "common.cuh"
-#include "tma.cuh"
+#include "screen.cuh"
 
 namespace gtls {
 
@@ -61,55 +55,18 @@ constexpr int kMaxRounds = 32;      // rounds of the shared-memory prepare path
 constexpr int kRoundShift = 20;     // hist entries of that path: position | round << kRoundShift
 constexpr int kPosMask = (1 << kRoundShift) - 1;
 constexpr int kPrepStaticSmem = 4096;  // static shared memory of prepare_kernel, rounded up
-constexpr int kChiThreads = 512;
-constexpr int kSplitMinSkip = 32;  // skip >= this: lanes split the block offset rho
-// Split-path task: a window of kWin consecutive starts of one duration.  Its
-// starts are first put through the depth test; the starts that pass are then
-// covered by groups of kR consecutive starts (each beginning at the first
-// uncovered start that passes), and only those groups are correlated.
-constexpr int kWin = 6 * kR;
-// All-starts pass, lane-path task of a width of at least kLaneGateMinW: a
-// window of 32 * kLaneG groups of kR consecutive starts; the groups whose
-// starts all fail the depth test are dropped and the others are dealt out to
-// the lanes round by round.  (For shorter widths, and for the main pass's
-// lane-path widths, measured: a group's sums cost about what its depth tests
-// do, and the task is the plain 32 groups.)
-constexpr int kLaneG = 6;            // (2 and 4 measured slower)
-constexpr int kLaneGateMinW = 64;
-// Zeroed records after each shared-memory tile: a skip-1 group whose kR
-// starts all lie in the tile reads at most kR - 2 records past it (only ever
-// against zero template entries), so those groups need no clamping.
-constexpr int kTilePad = 16;
-
-// float-float helpers (Knuth two-sum; no multiplications, so no contraction)
-__device__ __forceinline__ float2 ff_add(float2 a, float2 b) {
-  float s = a.x + b.x;
-  float bb = s - a.x;
-  float e = (a.x - (s - bb)) + (b.x - bb);
-  e += a.y + b.y;
-  float hi = s + e;
-  return make_float2(hi, e - (hi - s));
-}
-__device__ __forceinline__ float2 ff_from_double(double v) {
-  float hi = (float)v;
-  return make_float2(hi, (float)(v - (double)hi));
-}
-// Store prefix value v at pre[r] through the FP64 view of the prefix array:
-// as a double (FP64 form) or as the float-float pair (hi, lo) occupying the
-// same 8 bytes (FP32 form; hi at the lower address).  Streaming stores: the
-// chi2 kernel reads them back only after the whole chunk is prepared.
-template <typename Real>
-__device__ __forceinline__ void store_prefix(double* pre, int r, double v) {
-  if constexpr (sizeof(Real) == 8) {
-    __stcs(pre + r, v);
-  } else {
-    const float2 f = ff_from_double(v);
-    const unsigned long long bits = ((unsigned long long)__float_as_uint(f.y) << 32) | __float_as_uint(f.x);
-    __stcs(pre + r, __longlong_as_double((long long)bits));
-  }
-}
-
 // ------------------------------------------------------------ descriptors
+// Sums over a curve.  vscale and wscale are powers of two that bring v and w
+// to the order of one for the FP32 bounds (screen.cuh): u scales with both,
+// delta with dscale = vscale^2 wscale.
+struct CurveConst {
+  double ebase;            // sum v^2 w
+  double vscale, wscale, dscale;
+  float wbar, qbar;        // mean of the scaled w and u^2
+  float prefix_err;        // rounding of a difference of two prefix values, relative to the largest of them
+  int uniform;             // all weights equal
+};
+
 // Per-light-curve parameters and buffers on the device.  A search covers one
 // or many light curves; every kernel finds its curve through these.
 template <typename Real>
@@ -121,26 +78,26 @@ struct CurveDev {
   double* chi2_out;             // [np]
   int64_t* loc_out;             // [np] or NULL
   double2* vw;                  // [n] (v, w) per original sample (scratch)
-  double* ebase;                // sum v^2 w (scratch)
-  int* wmin;                    // [np] duration range (scratch)
-  int* wmax;
+  CurveConst* cst;              // sums over the curve (scratch)
+  double* sums;                 // [setup blocks * kSetupSums] their parts (scratch)
+  int* arrived;                 // setup blocks done (0 at first)
   const int* widths;            // [D]
   const double* overshoot;      // [D]
   const double* templates;      // [D * max_width]
   const int* skips;             // [D]
   const int* trow_off;          // [D] offsets into trows
-  const int* trow_len;          // [D]
-  typename Tr<Real>::R2* trows; // template rows (s, s^2), zero-padded
+  typename Tr<Real>::R2* trows; // template rows (s, s^2), w_d entries each
+  ScreenRow* srows;             // [2 D] bounds of the chi2 of a start: constants per duration and table,
+  ScreenCell* scells;           // its cells,
+  const int* sends;             // and their ends
   int* union_cnt;               // [nbatch]
   int* union_list;              // [nbatch * D] ascending duration indices
-  short* cost_order;            // [nbatch * D] positions in union_list, longest task first
   long long np;
-  int n, maxd, M, Mrec, D, max_width, batch, nbatch;
-  int tile, ntiles, nb_log2;
+  int n, maxd, D, max_width, batch, nbatch;
+  int tile, ntiles, nb_log2;    // starts of a chi2 CTA, CTAs of a period, bucket bits (global-scatter ordering)
   int rnb_log2, rcap;           // shared-memory prepare path: bucket bits and round capacity (0: off)
-  int global_rec;               // 1: chi2 reads the records from global memory (no shared tile)
-  int maxd_l;                   // > 0 (global records, main pass): the lane path's records, the tile
-                                // plus this halo (its longest width), are staged in shared memory
+  int coarse, vstride;          // chi2: step of the coarse prefix (0: none), row of the prefix of v of a CTA
+  int max_cell;                 // longest cell (samples)
   float span;
 };
 
@@ -153,10 +110,8 @@ struct Run {
   int count;          // periods in the run
   int tile0;          // first chi2 CTA of the run in its chunk
   long long pidx0;    // index of the run's first period within its curve
-  long long slot_off; // element offsets of the run's first row in each scratch array
-  long long rec_off;
-  long long pv_off;
-  long long part_off;
+  long long slot_off; // element offset of the run's first row of sorted indices (and of slots)
+  long long v_off;    // element offset of the run's first row of prefixes of v
 };
 
 // Largest i in [lo, hi) with key(i) <= x (keys ascending, key(lo) <= x).
@@ -172,32 +127,84 @@ __device__ __forceinline__ int upper_find(int lo, int hi, long long x, F key) {
 
 // ------------------------------------------------------------ curve set-up
 // (v, w) per original sample: v = y - 1 (exact), w = 1/(dy*dy)
-// (calcInverseSquaredPatchedDy GPUFun.py:134-142), and E = sum v^2 w
-// (calculate_base_error GPUFun.py:293-312 summed over the n samples).
+// (calcInverseSquaredPatchedDy GPUFun.py:134-142), and the curve's sums, E =
+// sum v^2 w (calculate_base_error GPUFun.py:293-312 summed over the n samples)
+// first.  One CTA per kSetupItems samples (one CTA per curve took 25 us on
+// 70,000 samples); the last of a curve's CTAs adds their parts, in order.
+constexpr int kSetupThreads = 256;
+constexpr int kSetupItems = 1024;
+constexpr int kSetupSums = 6;   // E, sum v^2, sum w, sum u^2, min w, max w
+
+__device__ __forceinline__ double sums_join(int k, double x, double y) {
+  return k < 4 ? x + y : (k == 4 ? fmin(x, y) : fmax(x, y));
+}
+
+// Power of two that brings x to [1, 2), or 1 where there is none.
+__device__ __forceinline__ double unit_scale(double x) {
+  if (!(x > 1e-290 && x < 1e290)) return 1.0;
+  return exp2(-(double)ilogb(x));
+}
+
 template <typename Real>
-__global__ void __launch_bounds__(1024) curve_setup_kernel(const CurveDev<Real>* __restrict__ cds) {
-  __shared__ double red[1024];
-  const CurveDev<Real>& C = cds[blockIdx.x];
-  const double* __restrict__ y = C.y;
-  const double* __restrict__ dy = C.dy;
-  double2* __restrict__ vw = C.vw;
-  const int n = C.n;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    double v = y[i] - 1.0;
-    double d = dy[i];
-    double w = 1.0 / (d * d);
-    vw[i] = make_double2(v, w);
-    double diff = 1.0 - y[i];
-    acc += diff * diff * w;
+__device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
+  __shared__ double red[kSetupSums][kSetupThreads / 32];
+  __shared__ int last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double s[kSetupSums] = {0, 0, 0, 0, INFINITY, -INFINITY};
+  for (int i = blk * kSetupItems + threadIdx.x; i < min(C.n, (blk + 1) * kSetupItems); i += kSetupThreads) {
+    const double v = C.y[i] - 1.0;
+    const double d = C.dy[i];
+    const double w = 1.0 / (d * d);
+    C.vw[i] = make_double2(v, w);
+    s[0] += v * v * w;
+    s[1] += v * v;
+    s[2] += w;
+    s[3] += (v * w) * (v * w);
+    s[4] = fmin(s[4], w);
+    s[5] = fmax(s[5], w);
   }
-  red[threadIdx.x] = acc;
+#pragma unroll
+  for (int k = 0; k < kSetupSums; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[k] = sums_join(k, s[k], __shfl_xor_sync(0xffffffffu, s[k], o));
+    if (lane == 0) red[k][wid] = s[k];
+  }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x < kSetupSums) {
+    double x = red[threadIdx.x][0];
+    for (int i = 1; i < kSetupThreads / 32; ++i) x = sums_join(threadIdx.x, x, red[threadIdx.x][i]);
+    C.sums[(size_t)blk * kSetupSums + threadIdx.x] = x;
+    __threadfence();
   }
-  if (threadIdx.x == 0) *C.ebase = red[0];
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(C.arrived, 1) == nblk - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (wid < kSetupSums) {
+    const int k = wid;
+    double x = k < 4 ? 0.0 : (k == 4 ? INFINITY : -INFINITY);
+    for (int b = lane; b < nblk; b += 32) x = sums_join(k, x, __ldcg(&C.sums[(size_t)b * kSetupSums + k]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = sums_join(k, x, __shfl_xor_sync(0xffffffffu, x, o));
+    if (lane == 0) red[k][0] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    CurveConst cc;
+    cc.ebase = red[0][0];
+    cc.vscale = unit_scale(sqrt(red[1][0] / C.n));
+    cc.wscale = unit_scale(red[2][0] / C.n);
+    cc.dscale = cc.vscale * cc.vscale * cc.wscale;
+    cc.wbar = (float)(red[2][0] * cc.wscale / C.n);
+    cc.qbar = (float)(red[3][0] * (cc.vscale * cc.wscale) * (cc.vscale * cc.wscale) / C.n);
+    // a prefix value carries some 20 roundings of a batch's scan, each of at
+    // most the largest prefix value times 2^-23, and one batch's more for each
+    // batch that a cell spans
+    cc.prefix_err = 0x1p-18f * (4.f + C.max_cell / 2048);
+    cc.uniform = red[4][0] == red[5][0];
+    *C.cst = cc;
+  }
 }
 
 // ------------------------------------------------------------ block scans
@@ -298,90 +305,6 @@ __device__ __forceinline__ void rank_bucket_warp(const uint2* __restrict__ slot,
   }
 }
 
-// Prefix of v in place over pre[1..M], accumulated in FP64 for both forms
-// (the FP32 form then stores each prefix as a float-float pair (hi, lo) in
-// the same 8 bytes): each warp scans a contiguous range (coalesced), then
-// adds the sum of the ranges before it.  pre[0] = 0.  wsum: 32 doubles.
-template <typename Real>
-__device__ void prefix_of_v(double* pre_d, int M, double* wsum) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int per = (M + nwarp - 1) / nwarp;
-  const int beg = 1 + min(M, wid * per);
-  const int end = 1 + min(M, (wid + 1) * per);
-  double acc = 0.0;
-  for (int r = beg + lane; r < end; r += 32) acc += pre_d[r];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) wsum[wid] = acc;
-  __syncthreads();
-  double carry = 0.0;
-  for (int w = 0; w < wid; ++w) carry += wsum[w];
-  if (wid == 0 && lane == 0) store_prefix<Real>(pre_d, 0, 0.0);
-  for (int r0 = beg; r0 < end; r0 += 32) {
-    const int r = r0 + lane;
-    double x = r < end ? pre_d[r] : 0.0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double yv = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += yv;
-    }
-    if (r < end) store_prefix<Real>(pre_d, r, carry + x);
-    carry += __shfl_sync(0xffffffffu, x, 31);
-  }
-}
-
-// Prefix value at pre[r] as a double (the inverse of store_prefix; in the
-// FP32 form the float-float pair is summed back in FP64).
-template <typename Real>
-__device__ __forceinline__ double load_prefix(const double* pre, int r) {
-  if constexpr (sizeof(Real) == 8) {
-    return pre[r];
-  } else {
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(pre[r]);
-    return (double)__uint_as_float((unsigned)bits) + (double)__uint_as_float((unsigned)(bits >> 32));
-  }
-}
-
-// Inclusive prefix of src[0, cnt) (shared memory, FP64) plus carry0, stored
-// at pre[dst0 + q] for q < cnt; returns, in every thread, the last stored
-// value (carry0 when cnt == 0).  Thread i sums its own chunk of K
-// consecutive entries (K odd, so that the lanes' strided reads fall in
-// distinct banks), the chunk sums are scanned across the block (shuffles,
-// then the warp totals), each thread rewrites its chunk in place as the
-// running prefix, and the block stores the result coalesced.  wsum: 32
-// doubles.  Ends with a barrier, after which src may be overwritten.
-template <typename Real>
-__device__ double scan_store(double* src, int cnt, double carry0, double* pre_d, int dst0, double* wsum) {
-  if (cnt <= 0) return carry0;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int K = ((cnt + blockDim.x - 1) / blockDim.x) | 1;
-  const int beg = min(cnt, (int)threadIdx.x * K), end = min(cnt, beg + K);
-  double acc = 0.0;
-  for (int r = beg; r < end; ++r) acc += src[r];
-  // exclusive prefix of the chunk sums: within the warp, then over the warps
-  double inc = acc;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const double yv = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += yv;
-  }
-  if (lane == 31) wsum[wid] = inc;
-  __syncthreads();
-  double exc = __shfl_up_sync(0xffffffffu, inc, 1);
-  double run = carry0;
-  for (int w = 0; w < wid; ++w) run += wsum[w];
-  if (lane > 0) run += exc;
-  for (int r = beg; r < end; ++r) {
-    run += src[r];
-    src[r] = run;
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < cnt; q += blockDim.x) store_prefix<Real>(pre_d, dst0 + q, src[q]);
-  const double last = src[cnt - 1];
-  __syncthreads();
-  return last;
-}
-
 // Round tables of the shared-memory prepare path.
 struct RoundTables {
   int nrounds;               // rounds; -1: the period takes the global-scatter path
@@ -399,30 +322,21 @@ struct RoundTables {
 // coalesced).  Each round then
 //   (a) reads its words (coalesced) into shared-memory slots by bucket,
 //   (b) ranks every slot within its bucket (the stable argsort order of
-//       the fold, as slot_less defines it) and writes the record of the
-//       resulting sorted position (close to the slot's, so nearly
-//       coalesced), with its v into shared memory, and
-//   (c) stores the FP64 prefix of v over its positions,
-// so that nothing is scattered through global memory.  Afterwards the
-// wrapped copy of the first maxd positions (patchData, GPUFun.py:110-129)
-// gets its prefix from pre[n] + pre[q + 1].  Returns false, having written
-// nothing, when a single bucket holds more than `cap` samples or more than
-// kMaxRounds rounds would be needed; the caller then takes the global path.
-// Dynamic shared memory: hist [NB] ints, slots [cap] words, vbuf [cap]
-// doubles.
-template <typename Real, bool kOrder>
-__device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, double* wsum, int* big, int* nbig, RoundTables& rt,
-                               const double* __restrict__ t, const double2* __restrict__ vw, int n, int maxd,
-                               double P, int nb_log2, int cap, uint2* __restrict__ stage,
-                               typename Tr<Real>::R2* __restrict__ out, double* __restrict__ pre_d,
-                               int* __restrict__ ord) {
-  using R2 = typename Tr<Real>::R2;
+//       the fold, as slot_less defines it) and writes its original index at
+//       the resulting sorted position (close to the slot's, so nearly
+//       coalesced),
+// so that nothing is scattered through global memory.  Returns false, having
+// written nothing, when a single bucket holds more than `cap` samples or more
+// than kMaxRounds rounds would be needed; the caller then takes the global
+// path.  Dynamic shared memory: hist [NB] ints, slots [cap] words.
+__device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int* nbig, RoundTables& rt,
+                               const double* __restrict__ t, int n, double P, int nb_log2, int cap,
+                               uint2* __restrict__ stage, int* __restrict__ ord) {
   const int nb = 1 << nb_log2;
   const double scale = (double)nb;
   constexpr unsigned imask = (unsigned)(kPackedMaxN - 1);
   int* hist = dyn;
   uint2* slots = reinterpret_cast<uint2*>(dyn + nb);
-  double* vbuf = reinterpret_cast<double*>(slots + cap);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   constexpr int kB = 2;   // elements per thread in flight in each pass (4 and 8 measured slower)
   const int stride = blockDim.x * kB;
@@ -518,7 +432,6 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, double* wsum,
     }
   }
   __syncthreads();
-  double carry = 0.0;   // prefix of v up to the current round (FP64)
   for (int r = 0; r < nr; ++r) {
     const int rs = rt.rpos[r], cnt = rt.rpos[r + 1] - rs;
     const int b0 = rt.rb[r], b1 = rt.rb[r + 1];
@@ -553,13 +466,11 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, double* wsum,
       for (uintptr_t a = lo + (uintptr_t)threadIdx.x * 128; a < hi; a += (uintptr_t)blockDim.x * 128)
         asm volatile("discard.global.L2 [%0], 128;" ::"l"(a) : "memory");
     }
-    // (b) ranks, and the records at once: the entry of sorted position p
-    //     (round-local q = p - rs) and original sample i gets its record
-    //     (u, w) at p (and at p + n when p < maxd: the wrap of patchData,
-    //     GPUFun.py:110-129) and its v at vbuf[q]; i is clamped so that a
-    //     malformed input can never address outside the curve.  Buckets of
-    //     more than kSmallBucketSm entries are listed and ranked by whole warps
-    //     (unless the list overflows); every other slot by its own thread.
+    // (b) ranks: the entry of sorted position p and original sample i puts
+    //     i, clamped so that a malformed input can never address outside the
+    //     curve, at ord[p].  Buckets of more than kSmallBucketSm entries are
+    //     listed and ranked by whole warps (unless the list overflows); every
+    //     other slot by its own thread.
     for (int b = b0 + (int)threadIdx.x; b < b1; b += blockDim.x) {
       const int k = H(b) - (b == 0 ? 0 : H(b - 1));
       if (k > kSmallBucketSm) {
@@ -570,21 +481,7 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, double* wsum,
     __syncthreads();
     const int nbg = *nbig;
     const bool warp_ranked = nbg <= kBigBuckets;
-    auto emit = [&](int q, int i) {
-      i = min(max(i, 0), n - 1);
-      const int p = rs + q;
-      if constexpr (kOrder) {
-        ord[p] = i;
-        return;
-      }
-      const double2 g = vw[i];
-      R2 o;
-      o.x = (Real)(g.x * g.y);
-      o.y = (Real)g.y;
-      __stcs(out + p, o);
-      if (p < maxd) __stcs(out + p + n, o);
-      vbuf[q] = g.x;
-    };
+    auto emit = [&](int q, int i) { ord[rs + q] = min(max(i, 0), n - 1); };
     if (warp_ranked)
       for (int q = wid; q < nbg; q += nwarp) {
         const int b = big[q];
@@ -623,89 +520,48 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, double* wsum,
           }
         }
       }
-      // the gathers of the kB entries in flight together
-      if constexpr (kOrder) {
 #pragma unroll
-        for (int u = 0; u < kB; ++u)
-          if (pos[u] >= 0) emit(pos[u], idx[u]);
-      } else {
-        double2 g[kB];
-#pragma unroll
-        for (int u = 0; u < kB; ++u) g[u] = pos[u] >= 0 ? vw[min(max(idx[u], 0), n - 1)] : make_double2(0.0, 0.0);
-#pragma unroll
-        for (int u = 0; u < kB; ++u) {
-          if (pos[u] >= 0) {
-            const int p = rs + pos[u];
-            R2 o;
-            o.x = (Real)(g[u].x * g[u].y);
-            o.y = (Real)g[u].y;
-            __stcs(out + p, o);
-            if (p < maxd) __stcs(out + p + n, o);
-            vbuf[pos[u]] = g[u].x;
-          }
-        }
-      }
+      for (int u = 0; u < kB; ++u)
+        if (pos[u] >= 0) emit(pos[u], idx[u]);
     }
     __syncthreads();
-    // (c) pre[rs + q + 1] = carry + v[0..q] (ends with a barrier)
-    if constexpr (!kOrder) carry = scan_store<Real>(vbuf, cnt, carry, pre_d, rs + 1, wsum);
-  }
-  if constexpr (!kOrder) {
-    // pre[0] = 0, and the wrapped copy: pre[n + 1 + q] = pre[n] + pre[q + 1]
-    if (threadIdx.x == 0) store_prefix<Real>(pre_d, 0, 0.0);
-    const int nw = min(maxd, n);
-    for (int q = threadIdx.x; q < nw; q += blockDim.x)
-      store_prefix<Real>(pre_d, n + 1 + q, carry + load_prefix<Real>(pre_d, q + 1));
   }
   return true;
 }
 
-// kOrder: write only the stable fold order of each period (order_out[rec_off
-// + local * n + p] = original index of sorted position p) instead of the
-// records and prefix (gtls_fold_order).  kThreads: kPrepThreads (one CTA per
+// The stable fold order of each period: order[slot_off + local * n + p] = the
+// original index of sorted position p.  kThreads: kPrepThreads (one CTA per
 // SM), or kPrepThreadsSmall for curves of at most kPrepSmallMaxN samples
 // (two CTAs per SM, each with half the shared memory: the barriers of one
 // overlap the other's work, which pays on short curves).
-template <typename Real, bool kOrder = false, int kThreads = kPrepThreads>
+template <typename Real, int kThreads = kPrepThreads>
 __global__ void __launch_bounds__(kThreads, kPrepThreads / kThreads)
 prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, int nruns,
-               uint2* __restrict__ scr_slot, typename Tr<Real>::R2* __restrict__ rec,
-               typename Tr<Real>::Pv* __restrict__ pv, int* __restrict__ order_out = nullptr) {
-  using R2 = typename Tr<Real>::R2;
-  using Pv = typename Tr<Real>::Pv;
+               uint2* __restrict__ scr_slot, int* __restrict__ order, int* __restrict__ tau = nullptr) {
   extern __shared__ int hist[];
   __shared__ int wtmp_i[32];
-  __shared__ double wsum[32];
   __shared__ int big[kBigBuckets];
   __shared__ int nbig;
   const int item = blockIdx.x;
+  if (tau && threadIdx.x == 0) tau[item] = 0x7f800000;   // infinity: the chi2 kernel's first bound
   const int ri = upper_find(0, nruns, item, [&](int i) { return (long long)runs[i].item0; });
   const Run& R = runs[ri];
   const CurveDev<Real>& C = cds[R.curve];
   const int local = item - R.item0;
   const double* __restrict__ t = C.t;
-  const double2* __restrict__ vw = C.vw;
   const int n = C.n;
-  const int maxd = C.maxd;
   const int nb_log2 = C.nb_log2;
   const int nb = 1 << nb_log2;
   const double scale = (double)nb;
   const bool packed = n <= kPackedMaxN && nb_log2 <= 32 - kPackedShift;
   const unsigned imask = packed ? (unsigned)(kPackedMaxN - 1) : 0xffffffffu;
   const double P = C.periods[R.pidx0 + local];
-  const int M = C.M;
-  const int Mrec = C.Mrec;
-  uint2* slot = scr_slot + R.slot_off + (size_t)local * n;
-  R2* out = kOrder ? nullptr : rec + R.rec_off + (size_t)local * Mrec;
-  Pv* pre = kOrder ? nullptr : pv + R.pv_off + (size_t)local * (M + 1);
-  double* pre_d = reinterpret_cast<double*>(pre);   // FP64 view during the scan (Pv is 8 bytes)
-  int* ord = kOrder ? order_out + R.rec_off + (size_t)local * n : nullptr;
+  uint2* slot = scr_slot + R.slot_off - runs[0].slot_off + (size_t)local * n;
+  int* ord = order + R.slot_off + (size_t)local * n;
   constexpr int kB = 4;   // elements per thread in flight in each pass
   const int stride = blockDim.x * kB;
   __shared__ RoundTables rt;
-  if (C.rnb_log2 > 0 && prepare_rounds<Real, kOrder>(hist, wtmp_i, wsum, big, &nbig, rt, t, vw, n, maxd, P,
-                                                     C.rnb_log2, C.rcap, slot, out, pre_d, ord))
-    return;
+  if (C.rnb_log2 > 0 && prepare_rounds(hist, wtmp_i, big, &nbig, rt, t, n, P, C.rnb_log2, C.rcap, slot, ord)) return;
   // global path: buckets scattered through the scratch row
 
   for (int b = threadIdx.x; b < nb; b += blockDim.x) hist[b] = 0;
@@ -749,28 +605,9 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
     }
   }
   __syncthreads();
-  // (3) ranking within buckets.  The entry of final sorted position p and
-  //     original sample i is emitted at once: its record (u, w) at p, v at
-  //     pre[p + 1] for the scan, and the same at n + p when p < maxd (the
-  //     wrap of patchData, GPUFun.py:110-129); i is clamped so that a
-  //     malformed input can never address outside the curve.
-  auto emit = [&](int p, int i) {
-    i = min(max(i, 0), n - 1);
-    if constexpr (kOrder) {
-      ord[p] = i;
-      return;
-    }
-    const double2 g = vw[i];
-    R2 o;
-    o.x = (Real)(g.x * g.y);
-    o.y = (Real)g.y;
-    out[p] = o;
-    pre_d[p + 1] = g.x;
-    if (p < maxd) {
-      out[p + n] = o;
-      pre_d[p + n + 1] = g.x;
-    }
-  };
+  // (3) ranking within buckets: the entry of sorted position p and original
+  //     sample i puts i, clamped as above, at ord[p].
+  auto emit = [&](int p, int i) { ord[p] = min(max(i, 0), n - 1); };
   //     (a) buckets of more than kSmallBucket entries (clustered phases, as
   //         when the period is close to a multiple of a regular cadence) are
   //         listed, from the shared-memory counts alone;
@@ -825,619 +662,13 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
       }
     }
   }
-  __syncthreads();
-  if constexpr (kOrder) return;
-  // (5) prefix of v in place over pre[1..M] (accumulated in FP64; the FP32
-  //     form stores float-float pairs)
-  prefix_of_v<Real>(pre_d, M, wsum);
 }
 
-// ------------------------------------------------------------------ chi2
-struct Best {
-  double v;
-  long long loc;
-};
-__device__ __forceinline__ void best_update(Best& b, double v, long long loc) {
-  if (v < b.v || (v == b.v && loc < b.loc)) {
-    b.v = v;
-    b.loc = loc;
-  }
-}
+}  // namespace gtls
 
-struct Chi2Args {
-  int pass;                 // GTLS_PASS_MAIN / GTLS_PASS_ALL
-  int nruns;
-  double depth_min;
-  int* status;              // device status word (bit 0: tile copy did not complete)
-  double* part_v;           // [chunk tiles]
-  long long* part_loc;      // [chunk tiles]
-  unsigned long long* work; // NULL, or [2]: multiply-adds of the starts passing the depth test, and issued
-};
+#include "chi2.cuh"
 
-// Mean depth of the window [k, k+w): -(sum v)/w  (calcAverageFromCumsum, GPUFun.py:366-375),
-// with 1/w computed once per duration.
-// From the two prefix values a = pre[k + w] and b = pre[k]:
-__device__ __forceinline__ double window_mean_of(double a, double b, double inv_w) { return -(a - b) * inv_w; }
-__device__ __forceinline__ float window_mean_of(float2 a, float2 b, float inv_w) {
-  // two-diff of the high parts, then the low parts
-  float s = a.x - b.x;
-  float bb = s - a.x;
-  float e = (a.x - (s - bb)) - (b.x + bb);
-  e += a.y - b.y;
-  return -(s + e) * inv_w;
-}
-template <typename Pv, typename Real>
-__device__ __forceinline__ Real window_mean(const Pv* pre, int k, int w, Real inv_w) {
-  return window_mean_of(pre[k + w], pre[k], inv_w);
-}
-
-// Value of start k for duration d from its sums (B, C).
-template <typename Real>
-__device__ __forceinline__ void eval_mean(Best& best, Real mean, Real os, Real B, Real C, double depth_min,
-                                          double ebase, double sentinel, long long loc) {
-  if ((double)mean > depth_min) {
-    Real c = mean * os * (Real)2;
-    Real delta = c * ((Real)2 * B + c * C);
-    best_update(best, ebase + (double)delta, loc);
-  } else {
-    best_update(best, sentinel, loc);
-  }
-}
-template <typename Real>
-__device__ __forceinline__ void eval_start(Best& best, const typename Tr<Real>::Pv* pre, int k, int w, Real inv_w,
-                                           Real os, Real B, Real C, double depth_min, double ebase,
-                                           double sentinel, long long loc) {
-  eval_mean<Real>(best, window_mean(pre, k, w, inv_w), os, B, C, depth_min, ebase, sentinel, loc);
-}
-
-// Butterfly reduce-scatter of 2*kR = 18 per-lane values over the warp
-// (9 + 5 + 3 + 2 + 1 shuffles): value i ends, summed over all lanes, in lane
-// kLaneOf[i].  Returns this lane's value (meaningful only in those lanes).
-__constant__ int kLaneOf[2 * kR] = {0, 1, 2, 4, 5, 8, 9, 10, 12, 16, 17, 18, 20, 21, 24, 25, 26, 28};
-
-template <typename Real>
-__device__ __forceinline__ Real warp_reduce_scatter18(const typename Tr<Real>::R2 (&acc)[kR]) {
-  const int lane = threadIdx.x & 31;
-  Real v[18];
-#pragma unroll
-  for (int r = 0; r < kR; ++r) {
-    v[r] = acc[r].x;
-    v[kR + r] = acc[r].y;
-  }
-  // level xor 16: keep 9 of 18
-  {
-    const bool hi = lane & 16;
-    Real nv[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      Real send = hi ? v[i] : v[9 + i];
-      Real recv = __shfl_xor_sync(0xffffffffu, send, 16);
-      nv[i] = (hi ? v[9 + i] : v[i]) + recv;
-    }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) v[i] = nv[i];
-  }
-  // level xor 8: keep 5 of 9 (v[9] = 0 pad)
-  {
-    const bool hi = lane & 8;
-    v[9] = (Real)0;
-    Real nv[5];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-      Real send = hi ? v[i] : v[5 + i];
-      Real recv = __shfl_xor_sync(0xffffffffu, send, 8);
-      nv[i] = (hi ? v[5 + i] : v[i]) + recv;
-    }
-#pragma unroll
-    for (int i = 0; i < 5; ++i) v[i] = nv[i];
-  }
-  // level xor 4: keep 3 of 5 (v[5] = 0 pad)
-  {
-    const bool hi = lane & 4;
-    v[5] = (Real)0;
-    Real nv[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      Real send = hi ? v[i] : v[3 + i];
-      Real recv = __shfl_xor_sync(0xffffffffu, send, 4);
-      nv[i] = (hi ? v[3 + i] : v[i]) + recv;
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) v[i] = nv[i];
-  }
-  // level xor 2: keep 2 of 3 (v[3] = 0 pad)
-  {
-    const bool hi = lane & 2;
-    v[3] = (Real)0;
-    Real nv[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      Real send = hi ? v[i] : v[2 + i];
-      Real recv = __shfl_xor_sync(0xffffffffu, send, 2);
-      nv[i] = (hi ? v[2 + i] : v[i]) + recv;
-    }
-    v[0] = nv[0];
-    v[1] = nv[1];
-  }
-  // level xor 1: keep 1 of 2
-  {
-    const bool hi = lane & 1;
-    Real send = hi ? v[0] : v[1];
-    Real recv = __shfl_xor_sync(0xffffffffu, send, 1);
-    v[0] = (hi ? v[1] : v[0]) + recv;
-  }
-  return v[0];
-}
-
-// correlate() with the template entries of the offset rho taken from the
-// lanes instead of memory: lane q (q < Q) holds T[q*s + rho] in tl, and step
-// q reads it by shuffle.  The products and their order are those of
-// correlate(); only where the template value comes from differs.  All 32
-// lanes must call it (lanes without starts read clamped records and discard
-// the sums).
-template <typename Real, bool kTwoLevel>
-__device__ __forceinline__ void correlate_bc(const typename Tr<Real>::R2* __restrict__ tile, int L, int base, int s,
-                                             typename Tr<Real>::R2 tl, int Q, typename Tr<Real>::R2 (&acc)[kR]) {
-  using R2 = typename Tr<Real>::R2;
-  R2 xs[kR];
-  const int last = L - 1;
-#pragma unroll
-  for (int i = 0; i < kR - 1; ++i) xs[i] = tile[min(base + i * s, last)];
-  R2 pr[kR];
-#pragma unroll
-  for (int r = 0; r < kR; ++r) pr[r] = kTwoLevel ? zero_pair<R2>() : acc[r];
-  int pos = base + (kR - 1) * s;
-  for (int q0 = 0; q0 < Q; q0 += kR) {
-#pragma unroll
-    for (int qq = 0; qq < kR; ++qq) {
-      if (q0 + qq >= Q) break;
-      xs[(qq + kR - 1) % kR] = tile[min(pos, last)];
-      R2 tq;
-      tq.x = __shfl_sync(0xffffffffu, tl.x, q0 + qq);
-      tq.y = __shfl_sync(0xffffffffu, tl.y, q0 + qq);
-      pos += s;
-#pragma unroll
-      for (int r = 0; r < kR; ++r) fma_pair(tq, xs[(qq + r) % kR], pr[r]);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < kR; ++r) {
-    if (kTwoLevel)
-      add_pair(acc[r], pr[r]);
-    else
-      acc[r] = pr[r];
-  }
-}
-
-// Dynamic shared memory of one chi2 CTA: the record tile (rounded up to 16
-// bytes) followed by the per-duration table (overshoot, width | skip << 16,
-// template row offset).
-template <typename Real>
-__host__ __device__ __forceinline__ size_t chi2_tile_bytes(int tile, int maxd) {
-  return ((size_t)(tile + maxd + kTilePad) * sizeof(typename Tr<Real>::R2) + 15) & ~(size_t)15;
-}
-template <typename Real>
-__host__ __device__ __forceinline__ size_t chi2_smem_bytes(int tile, int maxd, int D) {
-  return chi2_tile_bytes<Real>(tile, maxd) + (size_t)D * (sizeof(Real) + 2 * sizeof(int));
-}
-
-// kAllStarts: the instance for the all-starts pass (every skip is 1), which
-// alone carries the unclamped skip-1 path, so that the main-pass instance
-// keeps its register allocation.  kGlobal: the records are read from global
-// memory (through L1/L2) instead of a shared-memory tile, for curves whose
-// longest duration leaves no room for a tile in shared memory (or when the
-// caller asks for it); results are the same either way.
-template <typename Real, bool kAllStarts, bool kGlobal>
-__global__ void __launch_bounds__(kChiThreads, 1)
-chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs,
-            const typename Tr<Real>::R2* __restrict__ rec, const typename Tr<Real>::Pv* __restrict__ pv,
-            Chi2Args a) {
-  using R2 = typename Tr<Real>::R2;
-  using Pv = typename Tr<Real>::Pv;
-  constexpr bool kTwoLevel = sizeof(Real) == 4;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  R2* tile = reinterpret_cast<R2*>(smem_raw);
-  __shared__ int task_pre[GTLS_MAX_DURATIONS + 1];
-  __shared__ short task_dur[GTLS_MAX_DURATIONS];
-  __shared__ int task_next;
-  __shared__ Best red[kChiThreads / 32];
-  __shared__ __align__(8) uint64_t tile_bar;
-  __shared__ int tile_ok;
-  __shared__ unsigned long long work_sm[2];
-
-  const int cta = blockIdx.x;
-  const int ri = upper_find(0, a.nruns, cta, [&](int i) { return (long long)runs[i].tile0; });
-  const Run& R = runs[ri];
-  const CurveDev<Real>& C = cds[R.curve];
-  const int local = (cta - R.tile0) / C.ntiles;
-  const int tix = (cta - R.tile0) - local * C.ntiles;
-  const long long pg = R.pidx0 + local;       // period index within the curve
-  const int bidx = (int)(pg / C.batch);
-  const int D = C.D;
-  const int n = C.n;
-  const int ucnt = C.union_cnt[bidx];
-  const int* ulist = C.union_list + (size_t)bidx * D;
-  const int k0 = tix * C.tile;
-  const int k1 = min(n, k0 + C.tile);
-  const int L = (k1 - k0) + C.maxd - 1;
-  const R2* src = rec + R.rec_off + (size_t)local * C.Mrec + k0;
-  const Pv* pre = pv + R.pv_off + (size_t)local * (C.M + 1);
-  const double ebase = *C.ebase;
-  const double sentinel = (double)n;
-  const int* __restrict__ skips = C.skips;
-  const int lane = threadIdx.x & 31;
-  // per-duration table after the tile: overshoot, (width | skip << 16), template row offset
-  // staged records: the whole tile and halo, or (global records) only what
-  // the lane path reads, when the host made room for it
-  const bool stage = !kGlobal || C.maxd_l > 0;
-  const int Lt = kGlobal ? (k1 - k0) + C.maxd_l - 1 : L;
-  Real* dtab_os = reinterpret_cast<Real*>(
-      smem_raw + (kGlobal ? (C.maxd_l > 0 ? chi2_tile_bytes<Real>(C.tile, C.maxd_l) : 0)
-                          : chi2_tile_bytes<Real>(C.tile, C.maxd)));
-  int* dtab_ws = reinterpret_cast<int*>(dtab_os + D);
-  int* dtab_row = dtab_ws + D;
-  const R2* __restrict__ trows = C.trows;
-  if (threadIdx.x >= 32)
-    for (int d = (int)threadIdx.x - 32; d < D; d += (int)blockDim.x - 32) {
-      dtab_os[d] = (Real)C.overshoot[d];
-      dtab_ws[d] = C.widths[d] | (skips[d] << 16);
-      dtab_row[d] = C.trow_off[d];
-    }
-
-  // stage the records [k0, k0 + L) in shared memory with one bulk (TMA) copy;
-  // the byte count is rounded up to 16 (the record rows are padded for it)
-  const uint32_t tile_bytes = (uint32_t)(((size_t)Lt * sizeof(R2) + 15) & ~(size_t)15);
-  if (stage && threadIdx.x == 0) {
-    mbar_init(&tile_bar, 1);
-    mbar_arrive_expect_tx(&tile_bar, tile_bytes);
-    bulk_g2s(tile, src, tile_bytes, &tile_bar);
-  }
-  // task table (warp 0, overlapping the copy): the batch's durations in the
-  // precomputed cost order (longest task first, so the CTA's last tasks are short)
-  const short* corder = C.cost_order + (size_t)bidx * D;
-  if (threadIdx.x < 32) {
-    int carry = 0;
-    for (int u0 = 0; u0 < ucnt; u0 += 32) {
-      const int u = u0 + lane;
-      int nt = 0;
-      if (u < ucnt) {
-        task_dur[u] = corder[u];
-        const int d = ulist[corder[u]];
-        const int sk = skips[d];
-        const int jlo = (k0 + sk - 1) / sk, jhi = (k1 + sk - 1) / sk;
-        const int nj = max(0, jhi - jlo);
-        const int wd = C.widths[d];
-        nt = (sk >= kSplitMinSkip) ? (nj + kWin - 1) / kWin
-             : (kAllStarts && wd >= kLaneGateMinW ? (nj + 32 * kR * kLaneG - 1) / (32 * kR * kLaneG)
-                                    : (nj + 32 * kR - 1) / (32 * kR));
-      }
-      int inc = nt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int yv = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += yv;
-      }
-      if (u < ucnt) task_pre[u] = carry + inc - nt;
-      carry += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    if (lane == 0) {
-      task_pre[ucnt] = carry;
-      task_next = 0;
-      work_sm[0] = work_sm[1] = 0;
-      if (!stage || kGlobal) {
-        tile_ok = 1;   // global records: the warps that need the lane path's tile wait for it
-      } else {
-        tile_ok = mbar_wait_bounded(&tile_bar, 0, 1LL << 22) ? 1 : 0;
-        if (!tile_ok) {
-          // The copy into this CTA's shared memory may still be in flight:
-          // record the failure, then wait for it again (bounded, 16x longer)
-          // before the CTA goes on to evaluate nothing and exit, so that the
-          // copy does not land in shared memory that a later CTA owns.
-          atomicOr(a.status, 1);
-          mbar_wait_bounded(&tile_bar, 0, 1LL << 26);
-        }
-      }
-    }
-  }
-  __syncthreads();
-  if (stage && !kGlobal) {
-    // zero the pad after the tile's Lt records (the copy's rounding to 16 bytes
-    // may have brought in one record past them, possibly an unwritten one)
-    for (int i = Lt + (int)threadIdx.x; i < Lt + kTilePad; i += blockDim.x) {
-      R2 zr;
-      zr.x = (Real)0;
-      zr.y = (Real)0;
-      tile[i] = zr;
-    }
-  }
-  __syncthreads();
-  const R2* recs = kGlobal ? src : tile;   // the records [k0, k0 + L)
-  const R2* recl = stage ? tile : src;     // the lane path's: [k0, k0 + Ll)
-  const int Ll = stage ? Lt : L;
-
-  Best best{INFINITY, 0x7fffffffffffffffLL};
-  // the first start skipped by k % skip != 0 carries the value n (GPUFun.py:407,409)
-  if (a.pass == GTLS_PASS_MAIN && k0 == 0 && threadIdx.x == 0 && n > 1) {
-    for (int u = 0; u < ucnt; ++u)
-      if (skips[ulist[u]] > 1) {
-        best_update(best, sentinel, (long long)u * n + 1);
-        break;
-      }
-  }
-  const int ntask = tile_ok ? task_pre[ucnt] : 0;
-  const bool count_work = a.work != nullptr;
-  // global records with a staged lane-path tile: the split path starts at
-  // once; a warp waits for the tile (bounded) before its first lane-path task
-  bool lane_tile = !(kGlobal && stage);
-  bool lane_skip = false;
-  while (true) {
-    int tk = 0;
-    if (lane == 0) tk = atomicAdd(&task_next, 1);
-    tk = __shfl_sync(0xffffffffu, tk, 0);
-    if (tk >= ntask) break;
-    // binary search: the entry u with task_pre[u] <= tk < task_pre[u + 1]
-    int lo = 0, hi = ucnt - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (task_pre[mid] <= tk) lo = mid;
-      else hi = mid - 1;
-    }
-    const int u = lo;
-    const int sub = tk - task_pre[u];
-    const int upos = task_dur[u];        // position in ascending union order
-    const int d = ulist[upos];
-    const int ws = dtab_ws[d];
-    const int w = ws & 0xffff;
-    const int s = ws >> 16;
-    const int Q = (w + s - 1) / s;
-    const int jlo = (k0 + s - 1) / s;
-    const int jhi = (k1 + s - 1) / s;
-    const R2* trow = trows + dtab_row[d];
-    const Real os = dtab_os[d];
-    const Real inv_w = (Real)1 / (Real)w;
-    const long long locb = (long long)upos * n;
-    const int Qr = (Q + kR - 1) / kR * kR;
-    R2 acc[kR];
-    if (s >= kSplitMinSkip) {
-      // lanes split the offset rho inside a skip block.  (1) the depth test
-      // of the window's starts (one start per lane); a start that fails it
-      // takes the value n here and needs no sums (GPUFun.py:407,437)
-      const int jw = jlo + sub * kWin;
-      const int jend = min(jhi, jw + kWin);
-      unsigned long long act = 0;
-#pragma unroll
-      for (int i0 = 0; i0 < kWin; i0 += 32) {
-        const int j = jw + i0 + lane;
-        bool on = false;
-        if (i0 + lane < kWin && j < jend) {
-          const int k = j * s;
-          on = (double)window_mean(pre, k, w, inv_w) > a.depth_min;
-          if (!on) best_update(best, sentinel, locb + k);
-        }
-        act |= (unsigned long long)__ballot_sync(0xffffffffu, on) << i0;
-      }
-      if (count_work && lane == 0) atomicAdd(&work_sm[0], (unsigned long long)__popcll(act) * 2ULL * (unsigned)w);
-      // (2) groups of kR consecutive starts, each from the first start of the
-      //     window that passes and is not yet covered (moved back so that it
-      //     ends inside the window: the starts it then re-covers are either
-      //     covered already or fail the test)
-      while (act) {
-        const int off = min(__ffsll((long long)act) - 1, kWin - kR);
-        act &= ~(((1ULL << kR) - 1ULL) << off);
-        const int jb = jw + off;
-#pragma unroll
-        for (int r = 0; r < kR; ++r) acc[r] = zero_pair<R2>();
-        // every load of the group inside the tile: no clamping needed
-        if ((jb + Qr + kR - 1) * s - k0 <= L) {
-          if (!kTwoLevel && Qr == kR) {
-            correlate_rounds<Real>(recs, jb * s - k0, s, trow, lane, acc);
-          } else {
-            for (int rho = lane; rho < s; rho += 32)
-              correlate_pre<Real, kTwoLevel, false>(recs, L, jb * s + rho - k0, s, trow, rho, Q, acc);
-          }
-        } else {
-          for (int rho = lane; rho < s; rho += 32)
-            correlate_pre<Real, kTwoLevel, true>(recs, L, jb * s + rho - k0, s, trow, rho, Q, acc);
-        }
-        if (count_work && lane == 0) atomicAdd(&work_sm[1], (unsigned long long)kR * 2ULL * (unsigned)(Qr * s));
-        const Real mine = warp_reduce_scatter18<Real>(acc);
-        // lane kLaneOf[r] holds B_r, lane kLaneOf[kR + r] holds C_r
-        int r = -1;
-#pragma unroll
-        for (int i = 0; i < kR; ++i)
-          if (lane == kLaneOf[i]) r = i;
-        const int srcl = r >= 0 ? kLaneOf[kR + r] : lane;
-        const Real C = __shfl_sync(0xffffffffu, mine, srcl);
-        if (r >= 0) {
-          const int j = jb + r;
-          if (j < jend) {
-            const int k = j * s;
-            eval_start<Real>(best, pre, k, w, inv_w, os, mine, C, a.depth_min, ebase, sentinel, locb + k);
-          }
-        }
-      }
-    } else if (kAllStarts && w >= kLaneGateMinW) {
-      // lanes own groups of kR consecutive starts.  (1) the depth test of the
-      // window's groups, kLaneG per lane (a start that fails it takes the value
-      // n here); (2) the groups with a passing start, dealt out 32 at a time
-      const int g0 = sub * 32 * kLaneG;
-      unsigned masks[kLaneG];
-      int total = 0;
-#pragma unroll
-      for (int i = 0; i < kLaneG; ++i) {
-        const int jb = jlo + (g0 + 32 * i + lane) * kR;
-        bool any = false;
-        if (jb < jhi) {
-          Pv p0[kR], pw[kR];
-#pragma unroll
-          for (int r = 0; r < kR; ++r) {
-            const int k = min(jb + r, jhi - 1) * s;
-            p0[r] = pre[k];
-            pw[r] = pre[k + w];
-          }
-#pragma unroll
-          for (int r = 0; r < kR; ++r) {
-            if (jb + r < jhi) {
-              const bool on = (double)window_mean_of(pw[r], p0[r], inv_w) > a.depth_min;
-              any |= on;
-              if (!on) best_update(best, sentinel, locb + (long long)(jb + r) * s);
-            }
-          }
-        }
-        masks[i] = __ballot_sync(0xffffffffu, any);
-        total += __popc(masks[i]);
-      }
-      for (int q0 = 0; q0 < total; q0 += 32) {
-        const int q = q0 + lane;
-        int jb = jhi;   // no group for lanes past the last one
-        if (q < total) {
-          int before = 0;
-#pragma unroll
-          for (int i = 0; i < kLaneG; ++i) {
-            const int c = __popc(masks[i]);
-            if (q >= before && q < before + c) jb = jlo + (g0 + 32 * i + (int)__fns(masks[i], 0, q - before + 1)) * kR;
-            before += c;
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < kR; ++r) acc[r] = zero_pair<R2>();
-        if (jb < jhi) {
-          if (kAllStarts && !kGlobal && s == 1 && jb + kR <= jhi) {
-            correlate_s1<Real, kTwoLevel>(recl, jb - k0, trow, Qr, acc);
-          } else {
-            for (int rho = 0; rho < s; ++rho)
-              correlate<Real, kTwoLevel>(recl, Ll, jb * s + rho - k0, s, trow, rho, Q, acc);
-          }
-          Pv p0[kR], pw[kR];
-#pragma unroll
-          for (int r = 0; r < kR; ++r) {
-            const int k = min(jb + r, jhi - 1) * s;
-            p0[r] = pre[k];
-            pw[r] = pre[k + w];
-          }
-#pragma unroll
-          for (int r = 0; r < kR; ++r) {
-            const int j = jb + r;
-            if (j < jhi) {
-              const int k = j * s;
-              eval_mean<Real>(best, window_mean_of(pw[r], p0[r], inv_w), os, acc[r].x, acc[r].y, a.depth_min, ebase,
-                              sentinel, locb + k);
-            }
-          }
-        }
-        if (count_work) {
-          const unsigned ng = __popc(__ballot_sync(0xffffffffu, jb < jhi));
-          if (lane == 0) atomicAdd(&work_sm[1], (unsigned long long)ng * kR * 2ULL * (unsigned)(Qr * s));
-        }
-      }
-      if (count_work) {
-        // starts passing the depth test, counted from the prefix values again
-        unsigned nact = 0;
-        for (int i = 0; i < kLaneG; ++i) {
-          const int jb = jlo + (g0 + 32 * i + lane) * kR;
-          for (int r = 0; r < kR && jb + r < jhi; ++r)
-            nact += (double)window_mean(pre, (jb + r) * s, w, inv_w) > a.depth_min;
-        }
-        nact = __reduce_add_sync(0xffffffffu, nact);
-        if (lane == 0) atomicAdd(&work_sm[0], (unsigned long long)nact * 2ULL * (unsigned)w);
-      }
-    } else {
-      if constexpr (kGlobal) {
-        if (!lane_tile) {
-          int ok = 1;
-          if (lane == 0) {
-            ok = mbar_wait_bounded(&tile_bar, 0, 1LL << 22) ? 1 : 0;
-            if (!ok) atomicOr(a.status, 1);
-          }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          lane_skip = !ok;
-          if (ok)
-            for (int i = Lt + lane; i < Lt + kTilePad; i += 32) tile[i] = zero_pair<R2>();
-          __syncwarp();
-          lane_tile = true;
-        }
-        if (lane_skip) continue;   // the status word reports it
-      }
-#pragma unroll
-      for (int r = 0; r < kR; ++r) acc[r] = zero_pair<R2>();
-      // each lane takes kR consecutive start blocks and every rho
-      const int jb = jlo + (sub * 32 + lane) * kR;
-      if (!kAllStarts && Q <= 32) {
-        // the main pass (Q <= 16 here): every lane, the template entries of each
-        // offset held across the lanes, the next offset's loaded ahead
-        R2 tcur = lane < Q ? trow[lane * s] : zero_pair<R2>();
-        for (int rho = 0; rho < s; ++rho) {
-          const R2 tnx = (lane < Q && rho + 1 < s) ? trow[rho + 1 + lane * s] : zero_pair<R2>();
-          correlate_bc<Real, kTwoLevel>(recl, Ll, min(jb, jhi) * s + rho - k0, s, tcur, Q, acc);
-          tcur = tnx;
-        }
-      }
-      if (jb < jhi) {
-        if (kAllStarts && !kGlobal && s == 1 && jb + kR <= jhi) {
-          correlate_s1<Real, kTwoLevel>(recl, jb - k0, trow, Qr, acc);
-        } else if (kAllStarts || Q > 32) {
-          for (int rho = 0; rho < s; ++rho)
-            correlate<Real, kTwoLevel>(recl, Ll, jb * s + rho - k0, s, trow, rho, Q, acc);
-        }
-        // the prefix values of the lane's kR starts, all loads in flight
-        // together (indices clamped to the last start of the tile; values of
-        // starts past it are discarded)
-        Pv p0[kR], pw[kR];
-#pragma unroll
-        for (int r = 0; r < kR; ++r) {
-          const int k = min(jb + r, jhi - 1) * s;
-          p0[r] = pre[k];
-          pw[r] = pre[k + w];
-        }
-#pragma unroll
-        for (int r = 0; r < kR; ++r) {
-          const int j = jb + r;
-          if (j < jhi) {
-            const int k = j * s;
-            eval_mean<Real>(best, window_mean_of(pw[r], p0[r], inv_w), os, acc[r].x, acc[r].y, a.depth_min, ebase,
-                            sentinel, locb + k);
-          }
-        }
-      }
-      if (count_work) {
-        // work counters: the lanes' starts, and those passing the depth test
-        unsigned nst = 0, nact = 0;
-        if (jb < jhi)
-          for (int r = 0; r < kR && jb + r < jhi; ++r) {
-            ++nst;
-            nact += (double)window_mean(pre, (jb + r) * s, w, inv_w) > a.depth_min;
-          }
-        nst = __reduce_add_sync(0xffffffffu, nst);
-        nact = __reduce_add_sync(0xffffffffu, nact);
-        if (lane == 0) {
-          atomicAdd(&work_sm[0], (unsigned long long)nact * 2ULL * (unsigned)w);
-          atomicAdd(&work_sm[1], (unsigned long long)((nst + kR - 1) / kR * kR) * 2ULL * (unsigned)(Qr * s));
-        }
-      }
-    }
-  }
-  // a staged copy that no warp waited for must land before the CTA exits
-  if (kGlobal && stage && threadIdx.x == 0) mbar_wait_bounded(&tile_bar, 0, 1LL << 26);
-  // CTA minimum (value, then location)
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double v = __shfl_xor_sync(0xffffffffu, best.v, o);
-    long long l = __shfl_xor_sync(0xffffffffu, best.loc, o);
-    best_update(best, v, l);
-  }
-  if (lane == 0) red[threadIdx.x >> 5] = best;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    Best b = red[0];
-    for (int i = 1; i < kChiThreads / 32; ++i) best_update(b, red[i].v, red[i].loc);
-    a.part_v[cta] = b.v;
-    a.part_loc[cta] = b.loc;
-    if (a.work) {
-      atomicAdd(a.work, work_sm[0]);
-      atomicAdd(a.work + 1, work_sm[1]);
-    }
-  }
-}
+namespace gtls {
 
 template <typename Real>
 __global__ void finish_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, int nruns,
@@ -1447,6 +678,7 @@ __global__ void finish_kernel(const CurveDev<Real>* __restrict__ cds, const Run*
   const int ri = upper_find(0, nruns, item, [&](int i) { return (long long)runs[i].item0; });
   const Run& R = runs[ri];
   const CurveDev<Real>& C = cds[R.curve];
+  if (C.ntiles == 1) return;   // written by the chi2 kernel
   const int local = item - R.item0;
   const long long pg = R.pidx0 + local;
   Best b{INFINITY, 0x7fffffffffffffffLL};
@@ -1490,93 +722,194 @@ __global__ void duration_range_kernel(const double* __restrict__ periods, long l
   duration_range(periods[i], span, n, &wmin[i], &wmax[i]);
 }
 
-// Duration ranges of every period of every curve (period offsets p_off).
+// The ascending list of durations valid for at least one period of union
+// batch b of the curve (durationsGrid and durationBool GPUFun.py:47-105,
+// OR-ed as core.py:704-716).  Widths ascend, so a period's valid ones are a run:
+// its ends are counted up and down, and a duration is in the union where the
+// running count is not 0.
 template <typename Real>
-__global__ void duration_range_batch_kernel(const CurveDev<Real>* __restrict__ cds,
-                                            const long long* __restrict__ p_off, int n_curves) {
-  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (g >= p_off[n_curves]) return;
-  const int c = upper_find(0, n_curves, g, [&](int i) { return p_off[i]; });
-  const CurveDev<Real>& C = cds[c];
-  const long long i = g - p_off[c];
-  duration_range(C.periods[i], C.span, C.n, &C.wmin[i], &C.wmax[i]);
-}
-
-// One CTA per union batch (batch offsets b_off): the ascending list of
-// durations valid for at least one period of the batch (durationBool
-// GPUFun.py:91-105 OR-ed as core.py:704-716), and the same entries ordered by
-// the cost of one chi2 task, longest first (cost_order holds positions in
-// the ascending list).
-template <typename Real>
-__global__ void union_kernel(const CurveDev<Real>* __restrict__ cds, const long long* __restrict__ b_off,
-                             int n_curves, int all_durations) {
-  __shared__ int flags[GTLS_MAX_DURATIONS];
-  __shared__ int cost[GTLS_MAX_DURATIONS];
-  __shared__ short pos[GTLS_MAX_DURATIONS];
-  const long long gb = blockIdx.x;
-  const int c = upper_find(0, n_curves, gb, [&](int i) { return b_off[i]; });
-  const CurveDev<Real>& C = cds[c];
-  const long long b = gb - b_off[c];
+__device__ void duration_union(const CurveDev<Real>& C, long long b, int all_durations) {
+  __shared__ int edge[GTLS_MAX_DURATIONS + 1];
   const int D = C.D;
   const long long p0 = b * C.batch;
   const long long p1 = min(C.np, p0 + C.batch);
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    int w = C.widths[d];
-    int any = 0;
-    for (long long p = p0; p < p1 && !any; ++p) any = (w >= C.wmin[p]) && (w <= C.wmax[p]);
-    flags[d] = any || (all_durations && p1 > p0);
+  for (int d = threadIdx.x; d <= D; d += blockDim.x) edge[d] = 0;
+  __syncthreads();
+  const int* __restrict__ widths = C.widths;
+  auto first_from = [&](int w) {   // first duration of at least w samples
+    int lo = 0, hi = D;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (widths[mid] >= w) hi = mid;
+      else lo = mid + 1;
+    }
+    return lo;
+  };
+  for (long long p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+    int wmin = 0, wmax = INT32_MAX - 1;
+    if (!all_durations) duration_range(C.periods[p], C.span, C.n, &wmin, &wmax);
+    const int lo = first_from(wmin), hi = wmax == INT32_MAX ? D : first_from(wmax + 1);
+    if (lo < hi) {
+      atomicAdd(&edge[lo], 1);
+      atomicAdd(&edge[hi], -1);
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int cnt = 0;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
     int* ulist = C.union_list + b * D;
-    for (int d = 0; d < D; ++d)
-      if (flags[d]) {
-        ulist[cnt] = d;
-        const int sk = C.skips[d];
-        const int Qb = ((C.widths[d] + sk - 1) / sk + kR - 1) / kR;
-        // per-lane work of one task: every rho (thread-group path) or rho / 32 (split path)
-        cost[cnt] = (sk >= kSplitMinSkip ? (sk + 31) / 32 * 5 / 4 : sk) * Qb;
-        pos[cnt] = (short)cnt;
-        ++cnt;
+    int cnt = 0, open = 0;
+    for (int d0 = 0; d0 < D; d0 += 32) {
+      int run = d0 + lane < D ? edge[d0 + lane] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += y;
       }
-    C.union_cnt[b] = cnt;
-    // insertion sort by cost, descending (ties: wider first)
-    for (int i = 1; i < cnt; ++i) {
-      int cv = cost[i];
-      short pv = pos[i];
-      int j = i - 1;
-      while (j >= 0 && (cost[j] < cv || (cost[j] == cv && pos[j] < pv))) {
-        cost[j + 1] = cost[j];
-        pos[j + 1] = pos[j];
-        --j;
-      }
-      cost[j + 1] = cv;
-      pos[j + 1] = pv;
+      run += open;
+      const bool in = d0 + lane < D && run > 0;
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in) ulist[cnt + __popc(m & ((1u << lane) - 1u))] = d0 + lane;
+      cnt += __popc(m);
+      open = __shfl_sync(0xffffffffu, run, 31);
     }
-    for (int i = 0; i < cnt; ++i) C.cost_order[b * D + i] = pos[i];
+    if (lane == 0) C.union_cnt[b] = cnt;
   }
 }
 
-// Template rows in the layout the chi2 kernel reads: row d holds (s_i, s_i^2)
-// for i < w_d and zeros up to its length.  One CTA per (curve, duration).
+// Template rows as the exact sums read them, (s_i, s_i^2) for i < w_d, and the
+// cells of the bounds (screen.cuh): a warp per cell, kTemplateParts CTAs per
+// (duration, table).  A row's sums over its cells are added up in memory
+// (their last bits depend on the order; the bounds leave room for more).
+constexpr int kTemplateParts = 4;
 template <typename Real>
-__global__ void template_rows_kernel(const CurveDev<Real>* __restrict__ cds, const long long* __restrict__ d_off,
-                                     int n_curves) {
-  const long long gd = blockIdx.x;
-  const int c = upper_find(0, n_curves, gd, [&](int i) { return d_off[i]; });
-  const CurveDev<Real>& C = cds[c];
-  const int d = (int)(gd - d_off[c]);
+__device__ void template_part(const CurveDev<Real>& C, int d, int table, int part) {
   const int w = C.widths[d];
-  const int len = C.trow_len[d];
-  typename Tr<Real>::R2* row = C.trows + C.trow_off[d];
-  for (int i = threadIdx.x; i < len; i += blockDim.x) {
-    double sv = i < w ? C.templates[(size_t)d * C.max_width + i] : 0.0;
-    typename Tr<Real>::R2 o;
-    o.x = (Real)sv;
-    o.y = (Real)(sv * sv);
-    row[i] = o;
+  const double* __restrict__ T = C.templates + (size_t)d * C.max_width;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  if (table == 0) {
+    typename Tr<Real>::R2* row = C.trows + C.trow_off[d];
+    for (int i = part * blockDim.x + threadIdx.x; i < w; i += kTemplateParts * blockDim.x) {
+      const double sv = T[i];
+      typename Tr<Real>::R2 o;
+      o.x = (Real)sv;
+      o.y = (Real)(sv * sv);
+      row[i] = o;
+    }
   }
+  ScreenRow& row = C.srows[2 * d + table];
+  const int first = row.first, m = row.m;   // set by the host, the sums to 0
+  const int g = w <= kRingMaxW ? 1 : C.coarse;
+  const int* __restrict__ ends = C.sends + first;
+  auto at = [&](int i) { return i >= 0 && i < w ? T[i] : 0.0; };
+  auto sum_over = [&](double x) { return warp_sum(x); };
+  for (int q = part * nwarp + wid; q < m; q += kTemplateParts * nwarp) {
+    const int e0 = (q > 0 ? ends[q - 1] : 0) * g, e1 = ends[q] * g, l = e1 - e0;
+    // mean of the template over the cell for a window that starts with the
+    // cells, and g - 1 samples after them (coarse rows): the line between is a + b offset
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 4
+    for (int x = e0 + lane; x < e1; x += 32) {
+      s0 += at(x);
+      s1 += at(x - (g - 1));
+    }
+    const double mean0 = sum_over(s0) / l, mean1 = sum_over(s1) / l;
+    const float a = (float)mean0, b = g > 1 ? (float)((mean0 - mean1) / (g - 1)) : 0.f;
+    double rc2 = 0.0, rb = 0.0, mn = INFINITY, mx = 0.0;
+    if (g == 1) {
+      double s2 = 0.0;
+      for (int x = e0 + lane; x < e1; x += 32) {
+        const double r = at(x) - (double)a, sq = at(x) * at(x);
+        s2 += r * r;
+        mn = fmin(mn, sq);
+        mx = fmax(mx, sq);
+      }
+      rc2 = sum_over(s2);                    // about a, so at least the centred square
+      rb = fabs(mean0 - (double)a);          // the mean's rounding
+    } else {
+      for (int off = lane; off < g; off += 32) {   // a lane per offset of the window's start in its first step
+        const double ae = (double)a - (double)b * off;
+        double r1 = 0.0, r2 = 0.0;
+#pragma unroll 8
+        for (int x = e0 - off; x < e1 - off; ++x) {
+          const double s = at(x), r = s - ae, sq = s * s;
+          r1 += r;
+          r2 += r * r;
+          mn = fmin(mn, sq);
+          mx = fmax(mx, sq);
+        }
+        rc2 = fmax(rc2, fmax(r2 - r1 * r1 / l, 0.0) + 1e-14 * r2);
+        rb = fmax(rb, fabs(r1 / l));
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      rc2 = fmax(rc2, __shfl_xor_sync(0xffffffffu, rc2, o));
+      rb = fmax(rb, __shfl_xor_sync(0xffffffffu, rb, o));
+      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) {
+      ScreenCell cell;
+      cell.a = a;
+      cell.b = b;
+      cell.rc = (float)(sqrt(rc2) * 1.000001);
+      cell.rb = (float)(rb * 1.000001);
+      cell.mn = (float)mn;
+      cell.mx = table == 0 ? __int_as_float(ends[q]) : (float)mx;   // the first table has no use for it
+      cell.l = (float)l;
+      cell.inv_l = (float)(1.0 / l * (1.0 - 0x1p-10));
+      C.scells[first + q] = cell;
+      atomicAdd(&row.asum, (float)((fabs((double)a) + fabs((double)b) * (g - 1) + rb) * 1.0001));
+      atomicAdd(&row.smn, (float)mn);
+      atomicAdd(&row.smx, (float)(mx * 1.0001));
+      atomicAdd(&row.lmn, (float)(mn * l));
+      atomicAdd(&row.lmx, (float)(mx * l));
+    }
+  }
+  if (part == 0 && wid == 0) {
+    double t2 = 0.0;
+#pragma unroll 8
+    for (int i = lane; i < w; i += 32) t2 += T[i] * T[i];
+    t2 = sum_over(t2);
+    if (lane == 0) {
+      row.inv_w = (float)(1.0 / w);
+      row.os2 = (float)(2.0 * C.overshoot[d]);
+      row.tn = (float)(sqrt(t2) * 1.000001);
+      row.t2 = (float)t2;
+    }
+  }
+}
+
+// Everything a search prepares before its periods, in one launch: the CTAs of
+// the curves' set-up, of the unions, and of the templates (five launches one
+// after the other took 36 us on a 1,499-sample curve).
+struct SetupArgs {
+  const int* blk_off;        // [n_curves + 1] set-up CTAs of the curves
+  const long long* b_off;    // [n_curves + 1] union batches
+  const long long* d_off;    // [n_curves + 1] durations
+  int n_curves, n_blk, all_durations;
+  long long n_batch;
+};
+template <typename Real>
+__global__ void __launch_bounds__(kSetupThreads) setup_kernel(const CurveDev<Real>* __restrict__ cds, SetupArgs a) {
+  long long i = blockIdx.x;
+  if (i < a.n_blk) {
+    const int c = upper_find(0, a.n_curves, i, [&](int k) { return (long long)a.blk_off[k]; });
+    curve_setup(cds[c], (int)i - a.blk_off[c], a.blk_off[c + 1] - a.blk_off[c]);
+    return;
+  }
+  i -= a.n_blk;
+  if (i < a.n_batch) {
+    const int c = upper_find(0, a.n_curves, i, [&](int k) { return a.b_off[k]; });
+    duration_union(cds[c], i - a.b_off[c], a.all_durations);
+    return;
+  }
+  i -= a.n_batch;
+  const int part = (int)(i % kTemplateParts), table = (int)(i / kTemplateParts & 1);
+  i /= 2 * kTemplateParts;
+  const int c = upper_find(0, a.n_curves, i, [&](int k) { return a.d_off[k]; });
+  template_part(cds[c], (int)(i - a.d_off[c]), table, part);
 }
 
 // ------------------------------------------------------------------ host
@@ -1590,11 +923,9 @@ static int nb_log2_for(int n, int shift) {
 
 // Shared-memory prepare path of a curve of n samples: NB = 2^(ceil(log2 n) -
 // 2) buckets (at most 2^14, about four samples a bucket), and the largest
-// round capacity that fits the CTA's shared memory next to them (16 bytes a
-// sample: slot word and v).  Off (0) for curves beyond the packed slot
-// words or when fewer than 1,024 samples fit a round.  The rounds fix the
-// summation order of the prefix, so they depend on n and the device alone
-// (not on the tuning, which must not change a result).
+// round capacity that fits the CTA's shared memory next to them (8 bytes a
+// sample: the slot word).  Off (0) for curves beyond the packed slot words or
+// when fewer than 1,024 samples fit a round.
 template <typename Real>
 static void rounds_params(CurveDev<Real>& C, int smem_optin) {
   C.rnb_log2 = 0;
@@ -1606,7 +937,7 @@ static void rounds_params(CurveDev<Real>& C, int smem_optin) {
   const int nbl = std::max(1, std::min(14, k - 2));
   // two CTAs per SM for short curves: each gets half the shared memory
   const long long budget = (n <= kPrepSmallMaxN ? smem_optin / 2 : smem_optin) - kPrepStaticSmem;
-  const long long c = std::min<long long>((budget - (4LL << nbl)) / 16, n);
+  const long long c = std::min<long long>((budget - (4LL << nbl)) / 8, n);
   if (c < 1024 && c < n) return;
   C.rnb_log2 = nbl;
   C.rcap = (int)c;
@@ -1617,7 +948,7 @@ static void rounds_params(CurveDev<Real>& C, int smem_optin) {
 template <typename Real>
 static size_t prep_smem_bytes(const CurveDev<Real>& C) {
   size_t b = sizeof(int) << C.nb_log2;
-  if (C.rnb_log2 > 0) b = std::max(b, (sizeof(int) << C.rnb_log2) + 16 * (size_t)C.rcap);
+  if (C.rnb_log2 > 0) b = std::max(b, (sizeof(int) << C.rnb_log2) + sizeof(uint2) * (size_t)C.rcap);
   return b;
 }
 
@@ -1634,59 +965,129 @@ struct CurveHost {
   float span;
 };
 
+// Dynamic shared memory the kernels may ask for, set once per context.
+template <typename Real>
+static cudaError_t allow_smem(int optin) {
+  const int chi = (int)kChiSmemMax;
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto* k, int bytes) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  };
+  set(prepare_kernel<Real>, optin - kPrepStaticSmem);
+  set(prepare_kernel<Real, kPrepThreadsSmall>, optin - kPrepStaticSmem);
+  set(chi2_kernel<Real, false>, chi);
+  set(chi2_kernel<Real, true>, chi);
+  return e;
+}
+
+// Host copies of small arrays, gathered so that one copy takes them all to the
+// start of the arena (each pageable copy costs the host 5 to 10 us).
+struct Upload {
+  std::vector<char> host;
+  template <typename T>
+  size_t add(const T* src, size_t count) {
+    const size_t at = align_up(host.size(), 256);
+    host.resize(at + count * sizeof(T));
+    if (count) std::memcpy(host.data() + at, src, count * sizeof(T));
+    return at;
+  }
+};
+
 template <typename Real>
 static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int precision_pass, int skip_point,
                       double depth_min, int flags, gtls_timing* tm, cudaStream_t st) {
   using R2 = typename Tr<Real>::R2;
-  using Pv = typename Tr<Real>::Pv;
   const bool all = precision_pass == GTLS_PASS_ALL;
-  const size_t smem_budget = (size_t)ctx->smem_optin - 12 * 1024;   // static shared memory ~10.5 KB
+  const size_t list_cap = (all ? kListAll : kList) + kRedo;
+  bool& allowed = sizeof(Real) == 8 ? ctx->smem_set_fp64 : ctx->smem_set_fp32;
+  if (!allowed) {
+    GTLS_TRY_CUDA(ctx, allow_smem<Real>(ctx->smem_optin));
+    allowed = true;
+  }
 
-  // ---- per-curve layout on the host
+  // ---- the curves' widths
   std::vector<CurveDev<Real>> cd(n_curves);
-  std::vector<std::vector<int>> hw(n_curves), hskip(n_curves), hoff(n_curves), hlen(n_curves);
   std::vector<long long> p_off(n_curves + 1, 0), b_off(n_curves + 1, 0), d_off(n_curves + 1, 0);
-  size_t fixed = 0, rows_total = 0;
-  for (int c = 0; c < n_curves; ++c) {
-    const CurveHost& h = ch[c];
-    const int D = h.D;
-    hw[c].resize(D);
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(hw[c].data(), h.widths, sizeof(int) * D, cudaMemcpyDeviceToHost, st));
+  std::vector<int> blk_off(n_curves + 1, 0);
+  for (int c = 0; c < n_curves; ++c) d_off[c + 1] = d_off[c] + ch[c].D;
+  const size_t d_total = (size_t)d_off[n_curves];
+  std::vector<int> widths(d_total);
+  for (int c = 0, c1; c < n_curves; c = c1) {   // runs of curves whose arrays follow one another: one copy
+    for (c1 = c + 1; c1 < n_curves && ch[c1].widths == ch[c].widths + (d_off[c1] - d_off[c]); ++c1) {}
+    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(widths.data() + d_off[c], ch[c].widths, sizeof(int) * (d_off[c1] - d_off[c]),
+                                       cudaMemcpyDeviceToHost, st));
   }
   GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
+
+  // ---- ranges of starts per chi2 CTA.  The whole period, unless widths that
+  // the ring does not hold would make the coarse prefix coarser than
+  // kCoarseStep samples, or the caller set a cap.
+  const int cap_default = sizeof(Real) == 4 ? kTileCapFp32 : kTileCapFp64;
+  const int cap = sizeof(Real) == 4 ? ctx->tile_cap_fp32 : ctx->tile_cap_fp64;
+  long long ctas = 0, np_total = 0;
+  for (int c = 0; c < n_curves; ++c) {
+    const CurveHost& h = ch[c];
+    long long tile = std::min(h.n, 1 << 26);   // the blocks of the all-starts pass are numbered in 31 bits
+    if (h.max_width > kRingMaxW)
+      tile = std::max<long long>(kCoarseStep * (kCoarseCap - 8) - h.max_width, 4LL * h.max_width);
+    // the all-starts pass screens 8 or more times as many starts: shorter
+    // ranges even out its CTAs (600 of a whole period's third each, two to an SM, are three rounds)
+    if (all) tile = std::min<long long>(tile, std::max(8192, h.max_width));
+    if (cap != cap_default) tile = std::min<long long>(tile, cap);
+    cd[c].ntiles = (int)((h.n + tile - 1) / tile);
+    ctas += h.np * cd[c].ntiles;
+    np_total += h.np;
+  }
+  // small searches (the candidates, the harmonics, the best period): narrower
+  // ranges, so that the launch still fills the SMs (two CTAs each; aiming at two
+  // waves took 30% longer on 350 periods of 1,499 samples; a start's value does
+  // not depend on the range it is in)
+  const long long want = 2LL * ctx->num_sms;
+  const long long per = np_total > 0 && ctas < want ? (want + np_total - 1) / np_total : 1;
+  for (int c = 0; c < n_curves; ++c) {
+    const long long tiles = std::max<long long>(cd[c].ntiles, std::min<long long>(per, (ch[c].n + 511) / 512));
+    const long long tile = ((ch[c].n + tiles - 1) / tiles + 31) / 32 * 32;
+    cd[c].tile = (int)tile;
+    cd[c].ntiles = (int)((ch[c].n + tile - 1) / tile);
+  }
+
+  // ---- per-curve layout on the host
+  std::vector<int> skips(d_total), trow_off(d_total), ends;
+  std::vector<ScreenRow> srows(2 * d_total);
+  std::vector<size_t> cell_off(n_curves + 1, 0), row_off(n_curves + 1, 0);
   for (int c = 0; c < n_curves; ++c) {
     const CurveHost& h = ch[c];
     const int n = h.n, D = h.D, maxd = h.max_width;
     CurveDev<Real>& C = cd[c];
-    std::memset(&C, 0, sizeof(C));
-    hskip[c].resize(D);
-    hoff[c].resize(D);
-    hlen[c].resize(D);
-    int rows = 0;
+    const int* hw = widths.data() + d_off[c];
+    size_t rows = 0, cells = (size_t)D * kLaneCells;
+    C.coarse = coarse_step(C.tile, maxd);
+    C.max_cell = 0;
     for (int i = 0; i < D; ++i) {
-      const int w = hw[c][i];
-      if (w < 1 || w > maxd || (i > 0 && w <= hw[c][i - 1]))
+      const int w = hw[i];
+      if (w < 1 || w > maxd || (i > 0 && w <= hw[i - 1]))
         return fail(ctx, GTLS_E_INVALID, "widths must be ascending, >= 1 and <= max_width");
-      const int sk = (!all && w > skip_point) ? w / skip_point : 1;
-      const int Q = (w + sk - 1) / sk;
-      const int Qr = (Q + kR - 1) / kR * kR;
-      hskip[c][i] = sk;
-      hoff[c][i] = rows;
-      hlen[c][i] = (Qr + 1) * sk;   // one extra zero block: the one-step template prefetch reads it
-      rows += hlen[c][i];
+      skips[d_off[c] + i] = (!all && w > skip_point) ? w / skip_point : 1;
+      trow_off[d_off[c] + i] = (int)rows;
+      rows += w;
+      const int g = w <= kRingMaxW ? 1 : C.coarse;
+      // the two tables of cells: the first kLaneCells apart, the second after them
+      for (int k = 0; k < 2; ++k) {
+        std::vector<int> e;
+        screen_cells(w, g, k == 0, e);
+        ScreenRow r = {};
+        r.first = k == 0 ? i * kLaneCells : (int)cells;
+        r.m = (int)e.size();
+        srows[2 * (d_off[c] + i) + k] = r;
+        if (k == 1) cells += e.size();
+        ends.resize(cell_off[c] + cells);
+        std::copy(e.begin(), e.end(), ends.begin() + cell_off[c] + r.first);
+        for (size_t q = 0; q < e.size(); ++q) C.max_cell = std::max(C.max_cell, (e[q] - (q ? e[q - 1] : 0)) * g);
+      }
     }
     if (maxd > 0xffff) return fail(ctx, GTLS_E_RANGE, "max_width above 65535");
-    const size_t table = (size_t)D * (sizeof(Real) + 2 * sizeof(int)) + 16;
-    const long long cap = sizeof(Real) == 4 ? ctx->tile_cap_fp32 : ctx->tile_cap_fp64;
-    long long tile = ((long long)((smem_budget - table) / sizeof(R2)) - maxd - kTilePad) / 256 * 256;
-    // records in global memory when the longest duration leaves no room for a
-    // shared-memory tile of at least 256 starts (or when the caller asks for it)
-    // (the all-starts pass keeps the tile: its dense skip-1 sums reuse each
-    // record many times, and it measured faster on the tile)
-    const bool global_rec = (ctx->records_global && !all) || tile < 256;
-    if (global_rec) tile = cap;
-    tile = std::min<long long>(tile, cap);
-    if (tile > n) tile = (n + 255) / 256 * 256;
+    cell_off[c + 1] = ends.size();
+    row_off[c + 1] = row_off[c] + rows;
     C.t = h.t;
     C.y = h.y;
     C.dy = h.dy;
@@ -1699,61 +1100,17 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     C.np = h.np;
     C.n = n;
     C.maxd = maxd;
-    C.M = n + maxd;
-    C.Mrec = (C.M + 1) & ~1;
     C.D = D;
     C.max_width = maxd;
     C.batch = h.batch;
     C.nbatch = (int)((h.np + h.batch - 1) / h.batch);
-    C.tile = (int)tile;
-    C.ntiles = (int)((n + tile - 1) / tile);
+    C.vstride = C.coarse > 0 ? (C.tile + maxd + 2 * C.coarse + 8) / 8 * 8 : 0;
     C.nb_log2 = nb_log2_for(n, ctx->bucket_shift);
     rounds_params(C, ctx->smem_optin);
-    C.global_rec = global_rec ? 1 : 0;
-    C.maxd_l = 0;
-    if (global_rec && !all) {
-      int mx = 0;
-      for (int i = 0; i < D; ++i)
-        if (hskip[c][i] < kSplitMinSkip) mx = std::max(mx, hw[c][i]);
-      if (mx > 0 && chi2_smem_bytes<Real>((int)tile, mx, D) <= smem_budget) C.maxd_l = mx;
-    }
     C.span = h.span;
     p_off[c + 1] = p_off[c] + h.np;
     b_off[c + 1] = b_off[c] + C.nbatch;
-    d_off[c + 1] = d_off[c] + D;
-    carve_size<double2>(fixed, n);
-    carve_size<double>(fixed, 1);
-    carve_size<int>(fixed, h.np);
-    carve_size<int>(fixed, h.np);
-    carve_size<int>(fixed, (size_t)C.nbatch);
-    carve_size<int>(fixed, (size_t)C.nbatch * D);
-    carve_size<short>(fixed, (size_t)C.nbatch * D);
-    carve_size<int>(fixed, 3 * (size_t)D);
-    carve_size<R2>(fixed, (size_t)rows);
-    rows_total += rows;
-  }
-
-  // ---- small searches (a few periods: the harmonics, the best period):
-  // narrower tiles, so that the chi2 launch still has about two CTAs per SM
-  // (a start's value does not depend on the width of its tile)
-  {
-    long long ctas = 0, np_total = 0;
-    for (int c = 0; c < n_curves; ++c) {
-      ctas += cd[c].np * cd[c].ntiles;
-      np_total += cd[c].np;
-    }
-    const long long want = 2LL * ctx->num_sms;
-    if (np_total > 0 && ctas < want) {
-      const long long per = (want + np_total - 1) / np_total;   // tiles wanted per period
-      for (int c = 0; c < n_curves; ++c) {
-        CurveDev<Real>& C = cd[c];
-        const long long narrow = std::max<long long>(256, ((C.n + per - 1) / per + 255) / 256 * 256);
-        if (narrow < C.tile) {
-          C.tile = (int)narrow;
-          C.ntiles = (int)((C.n + narrow - 1) / narrow);
-        }
-      }
-    }
+    blk_off[c + 1] = blk_off[c] + (n + kSetupItems - 1) / kSetupItems;
   }
 
   // ---- chunks of the period list (curve after curve) and their runs
@@ -1761,43 +1118,45 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
   std::vector<Run> runs;
   std::vector<int> chunk_r0, chunk_items, chunk_tiles;
   std::vector<size_t> chunk_smem_prep, chunk_smem_chi;
-  std::vector<int> chunk_global;   // per chunk: records of all its curves in global memory (1) or tiles (0)
   std::vector<int> chunk_small;    // per chunk: all its curves take the two-per-SM prepare shape
-  size_t max_slot = 0, max_rec = 0, max_pv = 0, max_part = 0;
+  size_t max_slot = 0, max_v = 0, max_part = 0, max_items = 0;
   {
-    size_t slot = 0, rec = 0, pvs = 0, bytes = 0;
+    size_t slot = 0, vs = 0, bytes = 0;
     int items = 0, tiles = 0;
     size_t sm_prep = 0, sm_chi = 0;
     int mode = -1;
     chunk_r0.push_back(0);
     auto close_chunk = [&]() {
       if (items == 0) return;
-      chunk_global.push_back(mode & 1);
-      chunk_small.push_back(mode >> 1);
+      chunk_small.push_back(mode);
       chunk_items.push_back(items);
       chunk_tiles.push_back(tiles);
       chunk_smem_prep.push_back(sm_prep);
       chunk_smem_chi.push_back(sm_chi);
       max_slot = std::max(max_slot, slot);
-      max_rec = std::max(max_rec, rec);
-      max_pv = std::max(max_pv, pvs);
+      max_v = std::max(max_v, vs);
       max_part = std::max(max_part, (size_t)tiles);
+      max_items = std::max(max_items, (size_t)items);
       chunk_r0.push_back((int)runs.size());
-      slot = rec = pvs = bytes = 0;
+      slot = vs = bytes = 0;
       items = tiles = 0;
       sm_prep = sm_chi = 0;
       mode = -1;
     };
     for (int c = 0; c < n_curves; ++c) {
       const CurveDev<Real>& C = cd[c];
-      const size_t per = (size_t)C.n * 8 + (size_t)C.Mrec * sizeof(R2) + (size_t)(C.M + 1) * sizeof(Pv) +
-                         (size_t)C.ntiles * 16;
+      const size_t per = (size_t)C.n * (sizeof(uint2) + sizeof(int)) +
+                         (size_t)C.ntiles * (sizeof(float) * C.vstride + list_cap * sizeof(Waiting) + 16) + 4;
+      // the smallest budget a period is accepted with (as documented: slots, a
+      // record and a prefix value per sample and wrapped sample)
+      const size_t least = (size_t)C.n * 8 + (size_t)(C.n + C.maxd + 1) * (sizeof(R2) + 8);
       long long p = 0;
-      // one records mode and one prepare shape per chunk
-      const int cmode = C.global_rec | (C.n <= kPrepSmallMaxN ? 2 : 0);
+      // one prepare shape per chunk
+      const int cmode = C.n <= kPrepSmallMaxN ? 1 : 0;
       if (C.np > 0 && mode != -1 && mode != cmode) close_chunk();
       while (p < C.np) {
         long long fit = (long long)((budget > bytes ? budget - bytes : 0) / per);
+        if (items == 0) fit = budget < least ? 0 : std::max<long long>(fit, 1);
         fit = std::min<long long>(fit, (long long)INT32_MAX - items);
         fit = std::min<long long>(fit, ((1LL << 31) - 1 - tiles) / C.ntiles);
         if (fit <= 0) {
@@ -1813,20 +1172,15 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
         r.tile0 = tiles;
         r.pidx0 = p;
         r.slot_off = (long long)slot;
-        r.rec_off = (long long)rec;
-        r.pv_off = (long long)pvs;
-        r.part_off = tiles;
+        r.v_off = (long long)vs;
         runs.push_back(r);
         slot += (size_t)take * C.n;
-        rec += (size_t)take * C.Mrec;
-        pvs += (size_t)take * (C.M + 1);
+        vs += (size_t)take * C.ntiles * C.vstride;
         bytes += (size_t)take * per;
         items += (int)take;
         tiles += (int)(take * C.ntiles);
         sm_prep = std::max(sm_prep, prep_smem_bytes(C));
-        sm_chi = std::max(sm_chi, C.global_rec ? (C.maxd_l > 0 ? chi2_smem_bytes<Real>(C.tile, C.maxd_l, C.D)
-                                                                : (size_t)C.D * (sizeof(Real) + 2 * sizeof(int)))
-                                               : chi2_smem_bytes<Real>(C.tile, C.maxd, C.D));
+        sm_chi = std::max(sm_chi, chi2_smem_bytes(C.coarse > 0, C.D));
         mode = cmode;
         p += take;
       }
@@ -1834,71 +1188,76 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     close_chunk();
   }
   const int nchunks = (int)chunk_items.size();
-  const int nruns_total = (int)runs.size();
 
-  // ---- arena: fixed per-curve buffers, descriptors, and one chunk of scratch
-  size_t total = fixed;
-  carve_size<CurveDev<Real>>(total, n_curves);
-  carve_size<Run>(total, std::max(1, nruns_total));
-  carve_size<long long>(total, 3 * (size_t)(n_curves + 1));
+  // ---- arena: the uploaded arrays, per-curve buffers, and one chunk of scratch
+  Upload up;
+  const size_t at_cd = up.add((const CurveDev<Real>*)cd.data(), n_curves);   // filled in below
+  const size_t at_runs = up.add(runs.data(), runs.size());
+  const size_t at_boff = up.add(b_off.data(), b_off.size());
+  const size_t at_doff = up.add(d_off.data(), d_off.size());
+  const size_t at_blk = up.add(blk_off.data(), blk_off.size());
+  const size_t at_skips = up.add(skips.data(), skips.size());
+  const size_t at_trow = up.add(trow_off.data(), trow_off.size());
+  const size_t at_ends = up.add(ends.data(), ends.size());
+  const size_t at_srows = up.add(srows.data(), srows.size());
+  const std::vector<int> zeros(n_curves, 0);
+  const size_t at_arrived = up.add(zeros.data(), zeros.size());
+  size_t total = up.host.size();
+  for (int c = 0; c < n_curves; ++c) {
+    const CurveDev<Real>& C = cd[c];
+    carve_size<double2>(total, C.n);
+    carve_size<CurveConst>(total, 1);
+    carve_size<double>(total, (size_t)(blk_off[c + 1] - blk_off[c]) * kSetupSums);
+    carve_size<int>(total, (size_t)C.nbatch);
+    carve_size<int>(total, (size_t)C.nbatch * C.D);
+  }
+  carve_size<R2>(total, row_off[n_curves]);
+  carve_size<ScreenCell>(total, ends.size());
   carve_size<uint2>(total, max_slot);
-  carve_size<R2>(total, max_rec);
-  carve_size<Pv>(total, max_pv);
+  carve_size<int>(total, max_slot);
+  carve_size<float>(total, max_v);
   carve_size<double>(total, max_part);
   carve_size<long long>(total, max_part);
+  carve_size<Waiting>(total, max_part * list_cap);
+  carve_size<int>(total, max_items);
   carve_size<unsigned long long>(total, 2);
   total += 32 * 256;
   void* mem = arena(ctx, total);
   if (!mem) return fail(ctx, GTLS_E_NOMEM, "scratch allocation failed");
+  char* base = static_cast<char*>(mem);
   Carver cv(mem);
+  cv.take<char>(up.host.size());
   for (int c = 0; c < n_curves; ++c) {
     CurveDev<Real>& C = cd[c];
     C.vw = cv.take<double2>(C.n);
-    C.ebase = cv.take<double>(1);
-    C.wmin = cv.take<int>(C.np);
-    C.wmax = cv.take<int>(C.np);
+    C.cst = cv.take<CurveConst>(1);
+    C.sums = cv.take<double>((size_t)(blk_off[c + 1] - blk_off[c]) * kSetupSums);
+    C.arrived = reinterpret_cast<int*>(base + at_arrived) + c;
     C.union_cnt = cv.take<int>(C.nbatch);
     C.union_list = cv.take<int>((size_t)C.nbatch * C.D);
-    C.cost_order = cv.take<short>((size_t)C.nbatch * C.D);
-    int* dint = cv.take<int>(3 * (size_t)C.D);
-    C.skips = dint;
-    C.trow_off = dint + C.D;
-    C.trow_len = dint + 2 * C.D;
-    int rows = 0;
-    for (int i = 0; i < C.D; ++i) rows += hlen[c][i];
-    C.trows = cv.take<R2>(rows);
-    std::vector<int> tmp(3 * (size_t)C.D);
-    std::copy(hskip[c].begin(), hskip[c].end(), tmp.begin());
-    std::copy(hoff[c].begin(), hoff[c].end(), tmp.begin() + C.D);
-    std::copy(hlen[c].begin(), hlen[c].end(), tmp.begin() + 2 * C.D);
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(dint, tmp.data(), sizeof(int) * tmp.size(), cudaMemcpyHostToDevice, st));
+    C.skips = reinterpret_cast<const int*>(base + at_skips) + d_off[c];
+    C.trow_off = reinterpret_cast<const int*>(base + at_trow) + d_off[c];
+    C.sends = reinterpret_cast<const int*>(base + at_ends) + cell_off[c];
+    C.srows = reinterpret_cast<ScreenRow*>(base + at_srows) + 2 * d_off[c];
   }
-  CurveDev<Real>* d_cd = cv.take<CurveDev<Real>>(n_curves);
-  Run* d_runs = cv.take<Run>(std::max(1, nruns_total));
-  long long* d_offs = cv.take<long long>(3 * (size_t)(n_curves + 1));
+  R2* trows = cv.take<R2>(row_off[n_curves]);
+  ScreenCell* scells = cv.take<ScreenCell>(ends.size());
+  for (int c = 0; c < n_curves; ++c) {
+    cd[c].trows = trows + row_off[c];
+    cd[c].scells = scells + cell_off[c];
+  }
   uint2* scr_slot = cv.take<uint2>(max_slot);
-  R2* rec = cv.take<R2>(max_rec);
-  Pv* pv = cv.take<Pv>(max_pv);
+  int* order = cv.take<int>(max_slot);
+  float* vpre = cv.take<float>(max_v);
   double* part_v = cv.take<double>(max_part);
   long long* part_loc = cv.take<long long>(max_part);
+  Waiting* list = cv.take<Waiting>(max_part * list_cap);
+  int* tau = cv.take<int>(max_items);
   unsigned long long* work = cv.take<unsigned long long>(2);
-  {
-    std::vector<long long> offs(3 * (size_t)(n_curves + 1));
-    std::copy(p_off.begin(), p_off.end(), offs.begin());
-    std::copy(b_off.begin(), b_off.end(), offs.begin() + (n_curves + 1));
-    std::copy(d_off.begin(), d_off.end(), offs.begin() + 2 * (n_curves + 1));
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(d_cd, cd.data(), sizeof(CurveDev<Real>) * n_curves, cudaMemcpyHostToDevice,
-                                       st));
-    if (nruns_total)
-      GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(d_runs, runs.data(), sizeof(Run) * nruns_total, cudaMemcpyHostToDevice,
-                                         st));
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(d_offs, offs.data(), sizeof(long long) * offs.size(), cudaMemcpyHostToDevice,
-                                       st));
-  }
-  const long long* d_poff = d_offs;
-  const long long* d_boff = d_offs + (n_curves + 1);
-  const long long* d_doff = d_offs + 2 * (n_curves + 1);
-
+  std::memcpy(up.host.data() + at_cd, cd.data(), sizeof(CurveDev<Real>) * n_curves);
+  GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(base, up.host.data(), up.host.size(), cudaMemcpyHostToDevice, st));
+  const CurveDev<Real>* d_cd = reinterpret_cast<const CurveDev<Real>*>(base + at_cd);
+  const Run* d_runs = reinterpret_cast<const Run*>(base + at_runs);
   // ---- optional stage timing with CUDA events on the call's stream
   cudaEvent_t ev[2] = {nullptr, nullptr};
   std::vector<cudaEvent_t> evc;
@@ -1906,42 +1265,28 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     std::memset(tm, 0, sizeof(*tm));
     for (auto& e : ev) GTLS_TRY_CUDA(ctx, cudaEventCreate(&e));
     GTLS_TRY_CUDA(ctx, cudaEventRecord(ev[0], st));
+    GTLS_TRY_CUDA(ctx, cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), st));
   }
-  GTLS_TRY_CUDA(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), st));
-  if (tm) GTLS_TRY_CUDA(ctx, cudaMemsetAsync(work, 0, 2 * sizeof(unsigned long long), st));
-  curve_setup_kernel<Real><<<n_curves, 1024, 0, st>>>(d_cd);
-  if (p_off[n_curves] > 0)
-    duration_range_batch_kernel<Real><<<(unsigned)((p_off[n_curves] + 255) / 256), 256, 0, st>>>(d_cd, d_poff,
-                                                                                                 n_curves);
-  if (b_off[n_curves] > 0)
-    union_kernel<Real><<<(unsigned)b_off[n_curves], 256, 0, st>>>(d_cd, d_boff, n_curves,
-                                                                   (flags & GTLS_SEARCH_ALL_DURATIONS) ? 1 : 0);
-  template_rows_kernel<Real><<<(unsigned)d_off[n_curves], 256, 0, st>>>(d_cd, d_doff, n_curves);
-  ctx->launches += 4;
+  SetupArgs sa;
+  sa.blk_off = reinterpret_cast<const int*>(base + at_blk);
+  sa.b_off = reinterpret_cast<const long long*>(base + at_boff);
+  sa.d_off = reinterpret_cast<const long long*>(base + at_doff);
+  sa.n_curves = n_curves;
+  sa.n_blk = blk_off[n_curves];
+  sa.all_durations = (flags & GTLS_SEARCH_ALL_DURATIONS) ? 1 : 0;
+  sa.n_batch = b_off[n_curves];
+  const long long setup_ctas = sa.n_blk + sa.n_batch + 2LL * kTemplateParts * d_off[n_curves];
+  if (setup_ctas > INT32_MAX) return fail(ctx, GTLS_E_RANGE, "too many periods, samples and durations in one call");
+  setup_kernel<Real><<<(unsigned)setup_ctas, kSetupThreads, 0, st>>>(d_cd, sa);
+  ctx->launches += 1;
   GTLS_TRY_CUDA(ctx, cudaGetLastError());
   if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(ev[1], st));
 
-  size_t max_prep = 0, max_chi = 0;
-  for (int k = 0; k < nchunks; ++k) {
-    max_prep = std::max(max_prep, chunk_smem_prep[k]);
-    max_chi = std::max(max_chi, chunk_smem_chi[k]);
-  }
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(prepare_kernel<Real, false, kPrepThreadsSmall>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(max_prep, 1)));
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(prepare_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)std::max<size_t>(max_prep, 1)));
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(chi2_kernel<Real, false, false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(max_chi, 1)));
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(chi2_kernel<Real, true, false>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(max_chi, 1)));
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(chi2_kernel<Real, false, true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(max_chi, 1)));
-  GTLS_TRY_CUDA(ctx, cudaFuncSetAttribute(chi2_kernel<Real, true, true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(max_chi, 1)));
   Chi2Args ca;
-  ca.pass = precision_pass;
   ca.depth_min = depth_min;
-  ca.status = ctx->status;
+  ca.vpre = vpre;
+  ca.list = list;
+  ca.tau = tau;
   ca.part_v = part_v;
   ca.part_loc = part_loc;
   ca.work = tm ? work : nullptr;
@@ -1954,28 +1299,31 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
       GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[0], st));
     }
     if (chunk_small[k])
-      prepare_kernel<Real, false, kPrepThreadsSmall><<<items, kPrepThreadsSmall, chunk_smem_prep[k], st>>>(
-          d_cd, d_runs + r0, nr, scr_slot, rec, pv);
+      prepare_kernel<Real, kPrepThreadsSmall><<<items, kPrepThreadsSmall, chunk_smem_prep[k], st>>>(
+          d_cd, d_runs + r0, nr, scr_slot, order, tau);
     else
-      prepare_kernel<Real><<<items, kPrepThreads, chunk_smem_prep[k], st>>>(d_cd, d_runs + r0, nr, scr_slot, rec, pv);
+      prepare_kernel<Real><<<items, kPrepThreads, chunk_smem_prep[k], st>>>(d_cd, d_runs + r0, nr, scr_slot, order,
+                                                                             tau);
     if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[1], st));
     ca.nruns = nr;
-    using ChiKernel = void (*)(const CurveDev<Real>*, const Run*, const R2*, const Pv*, Chi2Args);
-    const ChiKernel kern = all ? (chunk_global[k] ? &chi2_kernel<Real, true, true> : &chi2_kernel<Real, true, false>)
-                               : (chunk_global[k] ? &chi2_kernel<Real, false, true>
-                                                  : &chi2_kernel<Real, false, false>);
-    kern<<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, rec, pv, ca);
+    if (all)
+      chi2_kernel<Real, true><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
+    else
+      chi2_kernel<Real, false><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
     if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[2], st));
-    finish_kernel<Real><<<(items + 127) / 128, 128, 0, st>>>(d_cd, d_runs + r0, nr, items, part_v, part_loc);
+    if (tiles > items) {   // some periods are split
+      finish_kernel<Real><<<(items + 127) / 128, 128, 0, st>>>(d_cd, d_runs + r0, nr, items, part_v, part_loc);
+      ctx->launches += 1;
+    }
     if (tm) {
       GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[3], st));
       for (auto& e : e3) evc.push_back(e);
     }
-    ctx->launches += 3;
+    ctx->launches += 2;
     GTLS_TRY_CUDA(ctx, cudaGetLastError());
   }
+  GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
   if (tm) {
-    GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
     float ms = 0;
     GTLS_TRY_CUDA(ctx, cudaEventElapsedTime(&ms, ev[0], ev[1]));
     tm->setup_ms = ms;
@@ -2000,11 +1348,11 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
       for (long long b = 0; b < C.nbatch; ++b) {
         long long np_b = std::min<long long>(C.batch, C.np - b * C.batch);
         for (int u = 0; u < hc[b]; ++u) {
-          int dd = hl[(size_t)b * C.D + u];
-          long long sk = hskip[c][dd];
+          const size_t dd = d_off[c] + hl[(size_t)b * C.D + u];
+          long long sk = skips[dd];
           long long js = (C.n + sk - 1) / sk;
           starts += np_b * js;
-          fma += np_b * js * 2LL * hw[c][dd];
+          fma += np_b * js * 2LL * widths[dd];
         }
       }
     }
@@ -2014,14 +1362,6 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     GTLS_TRY_CUDA(ctx, cudaMemcpy(hwk, work, sizeof(hwk), cudaMemcpyDeviceToHost));
     tm->chi2_active_fma = (long long)hwk[0];
     tm->chi2_issued_fma = (long long)hwk[1];
-  }
-  // device status word: a tile copy that did not complete within its bound
-  int hst = 0;
-  GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(&hst, ctx->status, sizeof(int), cudaMemcpyDeviceToHost, st));
-  GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
-  if (hst != 0) {
-    char msg[200];
-    return fail(ctx, gtls_decode_status(hst, msg, sizeof(msg)), msg);
   }
   return GTLS_OK;
 }
@@ -2140,8 +1480,6 @@ extern "C" int gtls_fold_order(gtls_ctx* ctx, const double* t, int32_t n, const 
   C.periods = periods;
   C.np = n_periods;
   C.n = n;
-  C.M = n;
-  C.Mrec = (n + 1) & ~1;
   C.nb_log2 = nb_log2_for(n, ctx->bucket_shift);
   rounds_params(C, ctx->smem_optin);
   // chunks of periods sized to the scratch budget (8 bytes of slots per sample and period)
@@ -2153,7 +1491,7 @@ extern "C" int gtls_fold_order(gtls_ctx* ctx, const double* t, int32_t n, const 
     std::memset(&r, 0, sizeof(r));
     r.count = (int)std::min<long long>(per_chunk, n_periods - p0);
     r.pidx0 = p0;
-    r.rec_off = p0 * n;   // offset of the run's rows in order_out
+    r.slot_off = p0 * n;   // offset of the run's rows in order_out
     runs.push_back(r);
   }
   size_t total = 0;
@@ -2169,18 +1507,16 @@ extern "C" int gtls_fold_order(gtls_ctx* ctx, const double* t, int32_t n, const 
   GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(d_cd, &C, sizeof(C), cudaMemcpyHostToDevice, st));
   GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(d_runs, runs.data(), sizeof(Run) * runs.size(), cudaMemcpyHostToDevice, st));
   const size_t smem = prep_smem_bytes(C);
-  const bool small = n <= kPrepSmallMaxN;
-  GTLS_TRY_CUDA(ctx, small ? cudaFuncSetAttribute(prepare_kernel<double, true, kPrepThreadsSmall>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                           : cudaFuncSetAttribute(prepare_kernel<double, true>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (!ctx->smem_set_fp64) {
+    GTLS_TRY_CUDA(ctx, allow_smem<double>(ctx->smem_optin));
+    ctx->smem_set_fp64 = true;
+  }
   for (size_t k = 0; k < runs.size(); ++k) {
-    if (small)
-      prepare_kernel<double, true, kPrepThreadsSmall><<<runs[k].count, kPrepThreadsSmall, smem, st>>>(
-          d_cd, d_runs + k, 1, slots, nullptr, nullptr, order_out);
+    if (n <= kPrepSmallMaxN)
+      prepare_kernel<double, kPrepThreadsSmall><<<runs[k].count, kPrepThreadsSmall, smem, st>>>(d_cd, d_runs + k, 1,
+                                                                                                slots, order_out);
     else
-      prepare_kernel<double, true><<<runs[k].count, kPrepThreads, smem, st>>>(d_cd, d_runs + k, 1, slots, nullptr,
-                                                                               nullptr, order_out);
+      prepare_kernel<double><<<runs[k].count, kPrepThreads, smem, st>>>(d_cd, d_runs + k, 1, slots, order_out);
     ctx->launches += 1;
     GTLS_TRY_CUDA(ctx, cudaGetLastError());
   }

@@ -61,12 +61,10 @@ const char* gtls_last_error(const gtls_ctx* ctx);
 /* ABI version compiled into the library (GTLS_ABI_VERSION). */
 int gtls_abi_version(void);
 
-/* Meaning of a search's device status word (no counterpart in the
- * reference, whose kernels have no error path).  The search kernels set bits
- * of a per-context word instead of hanging: bit 0 = a chi2 CTA's
- * shared-memory tile copy did not complete within its bounded wait (the CTA
- * then waited, bounded again, for the copy in flight, evaluated nothing and
- * left its period's minimum at +inf).  Returns GTLS_OK for 0 and
+/* Meaning of a device status word (no counterpart in the reference, whose
+ * kernels have no error path), kept for callers that stored one: bit 0 = a
+ * chi2 CTA's shared-memory tile copy did not complete within its bounded wait.
+ * The present kernels wait for no copy and set no bit.  Returns GTLS_OK for 0 and
  * GTLS_E_DEVICE otherwise, and writes a NUL-terminated message of at most
  * `cap` bytes to `msg` (host; msg may be NULL). */
 int gtls_decode_status(int32_t word, char* msg, size_t cap);
@@ -75,8 +73,8 @@ int gtls_decode_status(int32_t word, char* msg, size_t cap);
  * (no counterpart in the reference; used to account for device work). */
 int64_t gtls_launch_count(const gtls_ctx* ctx);
 
-/* Bytes of per-chunk scratch a search may use (fold records, prefix sums,
- * sort slots; default 8 GiB).  Periods are processed in chunks that fit it;
+/* Bytes of per-chunk scratch a search may use (sort slots, fold order, lists
+ * of starts; default 8 GiB).  A period is accepted from 48 bytes a sample on.  Periods are processed in chunks that fit it;
  * results do not depend on it.  No counterpart in the reference, whose
  * batch size comes from the free-memory formula of core.py:620-628.
  * bytes must be >= 1 MiB. */
@@ -88,17 +86,16 @@ int gtls_set_chunk_budget(gtls_ctx* ctx, uint64_t bytes);
  * gtls_b200.tune) may time a few settings on its own data and keep the
  * fastest.  A zero field means the default. */
 typedef struct gtls_tuning {
-  int32_t tile_cap_fp32;      /* max starts per chi2 tile (CTA), FP32 form: a multiple of 256 in
-                                 [256, 65536], or 0 = 16384.  The shared-memory size caps it too. */
-  int32_t tile_cap_fp64;      /* the same for the FP64 form, 0 = 8192                        */
+  int32_t tile_cap_fp32;      /* max starts of a chi2 CTA, FP32 form: a multiple of 256 in
+                                 [256, 65536]; 0, or 16384 = the library's own split (by the
+                                 curve's samples and longest duration)                       */
+  int32_t tile_cap_fp64;      /* the same for the FP64 form; 0, or 8192 = the library's own split */
   int32_t bucket_shift;       /* phase buckets of the global-scatter fold ordering (curves above
                                  2^17 samples, and periods whose phases cluster beyond what the
                                  shared-memory ordering holds) = 2^min(15, ceil(log2 N) + shift),
                                  shift in [-3, 0] (0 = default)                               */
-  int32_t records_global;     /* 1: the main pass's chi2 kernel reads the folded records from
-                                 global memory (L1/L2) for every curve; 0: from a shared-memory
-                                 tile when the curve's longest duration leaves room for one
-                                 (default).  The all-starts pass always uses the tile when it fits */
+  int32_t records_global;     /* 0 or 1, kept for callers: the folded records are read through L2
+                                 by every setting                                             */
 } gtls_tuning;
 
 int gtls_set_tuning(gtls_ctx* ctx, const gtls_tuning* tuning);
@@ -145,20 +142,19 @@ typedef struct gtls_timing {
   int32_t chunks;             /* period chunks (one prepare + chi2 launch each) */
   int32_t reserved;
   double setup_ms;            /* curve set-up, duration ranges, unions, template rows */
-  double prepare_ms;          /* fold + ranking + gather + prefix, all chunks   */
+  double prepare_ms;          /* fold + ranking, all chunks                     */
   double chi2_ms;             /* chi2 kernel, all chunks                        */
-  double finish_ms;           /* per-period minimum, all chunks                 */
-  int64_t chi2_starts;        /* (duration, start) evaluations done by the chi2 kernel */
-  int64_t chi2_fma;           /* multiply-adds of B and C over every evaluated start
+  double finish_ms;           /* per-period minimum of split periods, all chunks */
+  int64_t chi2_starts;        /* (duration, start) pairs the minimum is over      */
+  int64_t chi2_fma;           /* multiply-adds of B and C over every one of them
                                  (2 * width per start, whether or not its window
                                  passes the depth test)                          */
   int64_t chi2_active_fma;    /* the same over the starts whose window mean passes
                                  the depth test: the only starts whose sums enter
                                  the result (the reference's in-transit loop runs
                                  for these alone, GPUFun.py:409-424)            */
-  int64_t chi2_issued_fma;    /* multiply-adds the kernel performed (register
-                                 groups of consecutive starts, padded template
-                                 blocks included)                                */
+  int64_t chi2_issued_fma;    /* multiply-adds of the starts that were summed:
+                                 those their bounds did not rule out             */
 } gtls_timing;
 
 /*
