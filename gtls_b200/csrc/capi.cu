@@ -1,6 +1,7 @@
 // C-ABI entry points of gtls_b200: context, period grid, spectra.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -71,151 +72,6 @@ __global__ void period_reverse_kernel(const double* __restrict__ tmp, const int*
   long long cnt = hi >= lo ? (long long)(hi - lo + 1) : 0;
   long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (j < cnt) out[j] = tmp[hi - j];
-}
-
-// ---------------------------------------------------------------- spectra
-// stats.spectra (stats.py:95-122) with numpy.ma semantics for masked entries
-// (SpecState and the kernel declarations are in spectra.cuh).
-
-__device__ __forceinline__ bool unmasked(const uint8_t* mask, long long i) { return !mask || !mask[i]; }
-
-// Deterministic single-CTA reductions (fixed tree).
-template <typename Op>
-__device__ double block_reduce(double v, Op op, double* sh) {
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] = op(sh[threadIdx.x], sh[threadIdx.x + s]);
-    __syncthreads();
-  }
-  double r = sh[0];
-  __syncthreads();
-  return r;
-}
-struct OpAdd { __device__ double operator()(double a, double b) const { return a + b; } };
-// NaN-propagating like numpy's min/max
-struct OpMin {
-  __device__ double operator()(double a, double b) const { return (a != a) ? a : ((b != b) ? b : fmin(a, b)); }
-};
-struct OpMax {
-  __device__ double operator()(double a, double b) const { return (a != a) ? a : ((b != b) ? b : fmax(a, b)); }
-};
-
-__global__ void __launch_bounds__(1024) spectra_raw_kernel(const double* __restrict__ chi2,
-                                                           const uint8_t* __restrict__ mask, long long n,
-                                                           double* __restrict__ sr, double* __restrict__ praw,
-                                                           SpecState* st) {
-  __shared__ double sh[1024];
-  double mn = INFINITY, cnt = 0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x)
-    if (unmasked(mask, i)) {
-      mn = OpMin()(mn, chi2[i]);
-      cnt += 1;
-    }
-  mn = block_reduce(mn, OpMin(), sh);
-  cnt = block_reduce(cnt, OpAdd(), sh);
-  double s = 0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    double v = mn / chi2[i];
-    sr[i] = v;
-    if (unmasked(mask, i)) s += v;
-  }
-  double mean = block_reduce(s, OpAdd(), sh) / cnt;
-  double q = 0, mx = -INFINITY;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x)
-    if (unmasked(mask, i)) {
-      double dv = sr[i] - mean;
-      q += dv * dv;
-      mx = OpMax()(mx, dv);
-    }
-  double sd = sqrt(block_reduce(q, OpAdd(), sh) / cnt);
-  mx = block_reduce(mx, OpMax(), sh);
-  double sde_raw = (1 - mean) / sd;
-  double scale = sde_raw / mx;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) praw[i] = (sr[i] - mean) * scale;
-  if (threadIdx.x == 0) {
-    st->mean_sr = mean;
-    st->std_sr = sd;
-    st->sde_raw = sde_raw;
-    st->scale_raw = scale;
-    st->count = (int)cnt;
-  }
-}
-
-// Running median (helpers.py:91-106): window rows i = 0..n-k, median of the
-// unmasked values of praw[i, i+k) as numpy.ma.median takes it ((lo+hi)/2 of
-// the middle pair), then edge rows repeated to length n.
-__global__ void running_median_kernel(const double* __restrict__ praw, const uint8_t* __restrict__ mask,
-                                      long long n, int k, double* __restrict__ med) {
-  long long rows = n - k + 1;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= rows) return;
-  int cnt = 0;
-  for (int j = 0; j < k; ++j) cnt += unmasked(mask, i + j);
-  double out = NAN;
-  if (cnt > 0) {
-    int h = cnt / 2;
-    int lo_r = (cnt & 1) ? h : h - 1;
-    int hi_r = h;
-    double lo = NAN, hi = NAN;
-    // rank of element j among the unmasked window values, ties broken by position
-    for (int j = 0; j < k; ++j) {
-      if (!unmasked(mask, i + j)) continue;
-      double v = praw[i + j];
-      int r = 0;
-      for (int m = 0; m < k; ++m) {
-        if (!unmasked(mask, i + m)) continue;
-        double x = praw[i + m];
-        r += (x < v) || (x == v && m < j);
-      }
-      if (r == lo_r) lo = v;
-      if (r == hi_r) hi = v;
-    }
-    out = (lo + hi) / 2.0;
-  }
-  long long front = (n - rows) / 2;
-  med[front + i] = out;
-}
-
-__global__ void median_pad_kernel(double* med, long long n, long long rows) {
-  long long front = (n - rows) / 2;
-  long long back = n - rows - front;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < front) med[i] = med[front];
-  if (i < back) med[front + rows + i] = med[front + rows - 1];
-}
-
-__global__ void __launch_bounds__(1024) spectra_final_kernel(const double* __restrict__ praw,
-                                                             const uint8_t* __restrict__ mask,
-                                                             const double* __restrict__ med, long long n,
-                                                             double* __restrict__ power, SpecState* st) {
-  __shared__ double sh[1024];
-  const double cnt = st->count;
-  double s = 0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    double p = praw[i] - med[i];
-    power[i] = p;
-    if (unmasked(mask, i)) s += p;
-  }
-  double mean = block_reduce(s, OpAdd(), sh) / cnt;
-  double q = 0;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    double p = power[i] - mean;
-    power[i] = p;
-    if (unmasked(mask, i)) q += p * p;
-  }
-  double sd = sqrt(block_reduce(q, OpAdd(), sh) / cnt);
-  double mx = -INFINITY, mxp = -INFINITY;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x)
-    if (unmasked(mask, i)) {
-      mx = OpMax()(mx, power[i] / sd);
-      mxp = OpMax()(mxp, power[i]);
-    }
-  double sde = block_reduce(mx, OpMax(), sh);
-  mxp = block_reduce(mxp, OpMax(), sh);
-  double scale = sde / mxp;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) power[i] = power[i] * scale;
-  if (threadIdx.x == 0) st->sde = sde;
 }
 
 }  // namespace gtls
@@ -340,38 +196,28 @@ int gtls_spectra(gtls_ctx* ctx, const double* chi2, const uint8_t* mask, int64_t
   if (!ctx) return GTLS_E_INVALID;
   if (!chi2 || !sr || !power_raw || !power || !sde_raw || !sde || n < 1)
     return fail(ctx, GTLS_E_INVALID, "bad arguments to gtls_spectra");
-  double kd = oversampling_factor * 30;
-  if (kd != std::floor(kd) || kd < 1) return fail(ctx, GTLS_E_INVALID, "oversampling_factor * 30 must be an integer");
-  long long k = (long long)kd;
-  if (k % 2 == 0) k += 1;
+  const long long k = spectra_window(oversampling_factor);
+  if (k == 0) return fail(ctx, GTLS_E_INVALID, "oversampling_factor * 30 must be an integer");
   GTLS_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  size_t bytes = align_up(sizeof(double) * n, 256) + align_up(sizeof(SpecState), 256) + 256;
-  void* mem = arena(ctx, bytes);
+  size_t bytes = 0;
+  carve_size<double>(bytes, kSpecParts);
+  carve_size<SpecState>(bytes, 1);
+  carve_size<double>(bytes, n);
+  void* mem = arena(ctx, bytes + 256);
   if (!mem) return fail(ctx, GTLS_E_NOMEM, "scratch allocation failed");
   Carver cv(mem);
-  double* med = cv.take<double>(n);
-  SpecState* dst = cv.take<SpecState>(1);
-  spectra_raw_kernel<<<1, 1024, 0, st>>>(chi2, mask, n, sr, power_raw, dst);
-  ctx->launches += 1;
+  SpecScratch s;
+  s.part = cv.take<double>(kSpecParts);
+  s.state = cv.take<SpecState>(1);
+  s.med = cv.take<double>(n);
+  // (a window of more than n / 2 periods is never taken)
+  ctx->launches += spectra_launch(chi2, mask, n, (int)std::min<long long>(k, n), sr, power_raw, power, s, st);
+  GTLS_TRY_CUDA(ctx, cudaGetLastError());
   SpecState hs;
-  if (n > 2 * k) {
-    long long rows = n - k + 1;
-    running_median_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(power_raw, mask, n, (int)k, med);
-    median_pad_kernel<<<(unsigned)((n - rows + 255) / 256 + 1), 256, 0, st>>>(med, n, rows);
-    spectra_final_kernel<<<1, 1024, 0, st>>>(power_raw, mask, med, n, power, dst);
-    ctx->launches += 3;
-    GTLS_TRY_CUDA(ctx, cudaGetLastError());
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
-    *sde = hs.sde;
-  } else {
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(power, power_raw, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-    GTLS_TRY_CUDA(ctx, cudaGetLastError());
-    GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
-    *sde = hs.sde_raw;
-  }
+  GTLS_TRY_CUDA(ctx, cudaMemcpyAsync(&hs, s.state, sizeof(hs), cudaMemcpyDeviceToHost, st));
+  GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
+  *sde = n > 2 * k ? hs.sde : hs.sde_raw;
   *sde_raw = hs.sde_raw;
   return GTLS_OK;
 }

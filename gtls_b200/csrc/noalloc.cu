@@ -12,7 +12,8 @@
 //
 // Costs and limits of that choice:
 //  * the array is part of this library's device image, so every GPU that
-//    loads the library holds GTLS_NOALLOC_SCRATCH_BYTES until the process exits;
+//    loads the library holds GTLS_NOALLOC_SCRATCH_BYTES, and 28 KB of partial
+//    sums, until the process exits;
 //  * at most GTLS_NOALLOC_MAX_PERIODS periods per call; larger inputs are
 //    rejected with GTLS_E_RANGE before anything is launched;
 //  * all calls on one device share the array: calls that overlap on the GPU
@@ -42,8 +43,10 @@ namespace {
 constexpr size_t kMedBytes = sizeof(double) * (size_t)GTLS_NOALLOC_MAX_PERIODS;
 constexpr size_t kStateOff = (kMedBytes + 255) / 256 * 256;
 static_assert(kStateOff + sizeof(SpecState) <= GTLS_NOALLOC_SCRATCH_BYTES, "scratch too small");
+constexpr size_t kPartOff = (GTLS_NOALLOC_SCRATCH_BYTES + 255) / 256 * 256;   // the launches' partial results follow it
+constexpr size_t kTotalBytes = kPartOff + sizeof(double) * kSpecParts;
 
-__device__ __align__(256) unsigned char g_noalloc_scratch[GTLS_NOALLOC_SCRATCH_BYTES];
+__device__ __align__(256) unsigned char g_noalloc_scratch[kTotalBytes];
 
 constexpr int kMaxDevices = 64;
 std::atomic<void*> g_scratch_ptr[kMaxDevices];
@@ -92,33 +95,23 @@ extern "C" int gtls_spectra_noalloc(const double* chi2, const uint8_t* mask, int
     return noalloc_fail(GTLS_E_RANGE, "gtls_spectra_noalloc: n = " + std::to_string(n) +
                                           " exceeds GTLS_NOALLOC_MAX_PERIODS = " +
                                           std::to_string((long long)GTLS_NOALLOC_MAX_PERIODS));
-  const double kd = oversampling_factor * 30;
-  if (kd != std::floor(kd) || kd < 1)
-    return noalloc_fail(GTLS_E_INVALID, "oversampling_factor * 30 must be an integer");
-  long long k = (long long)kd;
-  if (k % 2 == 0) k += 1;
+  const long long k = spectra_window(oversampling_factor);
+  if (k == 0) return noalloc_fail(GTLS_E_INVALID, "oversampling_factor * 30 must be an integer");
   void* base = nullptr;
   int rc = scratch_on_current_device(&base);
   if (rc != GTLS_OK) return rc;
-  double* med = static_cast<double*>(base);
-  SpecState* dst = reinterpret_cast<SpecState*>(static_cast<unsigned char*>(base) + kStateOff);
+  unsigned char* const b = static_cast<unsigned char*>(base);
+  SpecScratch s;
+  s.med = reinterpret_cast<double*>(b);
+  s.state = reinterpret_cast<SpecState*>(b + kStateOff);
+  s.part = reinterpret_cast<double*>(b + kPartOff);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-
-  spectra_raw_kernel<<<1, 1024, 0, st>>>(chi2, mask, n, sr, power_raw, dst);
+  spectra_launch(chi2, mask, n, (int)(k < n ? k : n), sr, power_raw, power, s, st);
   SpecState hs;
   cudaError_t e;
-  if (n > 2 * k) {
-    long long rows = n - k + 1;
-    running_median_kernel<<<(unsigned)((rows + 127) / 128), 128, 0, st>>>(power_raw, mask, n, (int)k, med);
-    median_pad_kernel<<<(unsigned)((n - rows + 255) / 256 + 1), 256, 0, st>>>(med, n, rows);
-    spectra_final_kernel<<<1, 1024, 0, st>>>(power_raw, mask, med, n, power, dst);
-  } else {
-    e = cudaMemcpyAsync(power, power_raw, sizeof(double) * n, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return noalloc_fail(GTLS_E_CUDA, std::string("cudaMemcpyAsync: ") + cudaGetErrorString(e));
-  }
   e = cudaGetLastError();
   if (e != cudaSuccess) return noalloc_fail(GTLS_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
-  e = cudaMemcpyAsync(&hs, dst, sizeof(hs), cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(&hs, s.state, sizeof(hs), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return noalloc_fail(GTLS_E_CUDA, std::string("readback: ") + cudaGetErrorString(e));
   *sde_raw = hs.sde_raw;

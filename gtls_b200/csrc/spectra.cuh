@@ -1,23 +1,38 @@
-// Spectra kernels (defined in capi.cu), shared with the allocation-free entry point.
+// Spectra (spectra.cu), shared by gtls_spectra and its allocation-free form.
 #pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
 #include <cstdint>
 
 namespace gtls {
 
 struct SpecState {
-  double mean_sr, std_sr, sde_raw, scale_raw;
-  double sde;
-  int count;
-  int has_median;
+  double count, mean_sr, mean_power;
+  double sde_raw, sde;
 };
 
-__global__ void spectra_raw_kernel(const double* __restrict__ chi2, const uint8_t* __restrict__ mask, long long n,
-                                   double* __restrict__ sr, double* __restrict__ praw, SpecState* st);
-__global__ void running_median_kernel(const double* __restrict__ praw, const uint8_t* __restrict__ mask,
-                                      long long n, int k, double* __restrict__ med);
-__global__ void median_pad_kernel(double* med, long long n, long long rows);
-__global__ void spectra_final_kernel(const double* __restrict__ praw, const uint8_t* __restrict__ mask,
-                                     const double* __restrict__ med, long long n, double* __restrict__ power,
-                                     SpecState* st);
+constexpr int kSpecCtas = 4 * 148;                   // CTAs of a launch, at most
+constexpr size_t kSpecParts = 6 * (size_t)kSpecCtas; // partial results of the launches
+
+struct SpecScratch {
+  double* part;       // [kSpecParts]
+  SpecState* state;
+  double* med;        // [n], read and written for windows of more than 512 periods only
+};
+
+// Launches the spectra of n periods with a running median over k (none when n
+// <= 2 k: state->sde is then not set).  Returns the number of launches.
+int spectra_launch(const double* chi2, const uint8_t* mask, long long n, int k, double* sr, double* praw,
+                   double* power, SpecScratch s, cudaStream_t st);
+
+// Window of the running median for an oversampling factor: 30 times it, made
+// odd (stats.py:108-112); 0 when that is no whole number of at least 1.
+inline long long spectra_window(double oversampling_factor) {
+  const double kd = oversampling_factor * 30;
+  if (!(kd >= 1 && kd <= 1e15) || kd != (double)(long long)kd) return 0;
+  const long long k = (long long)kd;
+  return k + 1 - k % 2;
+}
 
 }  // namespace gtls
