@@ -157,22 +157,22 @@ __device__ __forceinline__ int nth_bit(unsigned w, int r) {
 // middle pair); the first and last rows' are repeated to the ends.
 //
 // A CTA sorts a tile of M consecutive values once (bitonic, a value per
-// thread) and then slides the window as a bit set over the sorted places: a
-// warp holds it (32 places a lane), a row moves two bits and finds the middle
-// one by counting, some 50 warp instructions where ranking the window by
-// all pairs took k^2 / 32 steps.  M is the smallest tile of at least twice the
-// window.
+// thread) and then slides the window as a bit set over the sorted places. M / 32
+// lanes hold it (32 places each, so 32 runs of rows at once); a row moves two
+// bits and finds the middle one by counting, some 70 instructions of a few
+// lanes where ranking the window by all pairs took k^2 steps of one.  M is
+// the smallest tile of at least twice the window.
 template <int M>
 __global__ void __launch_bounds__(M) spec_median_kernel(const double* __restrict__ sr, const uint8_t* __restrict__ mask,
                                                         long long n, int k, int raw_parts, double* __restrict__ praw,
                                                         double* __restrict__ power, SpecScratch s) {
-  constexpr int kWords = M / 32;   // lanes of the bit set, and warps
+  constexpr int kWords = M / 32;   // words and lanes of a bit set
   __shared__ double sh[32];
   __shared__ double key_sm[M];               // while sorting, then the sorted values
   __shared__ unsigned short idx_sm[M];       // and their places in the tile (0xffff: not in any window)
   __shared__ unsigned short rank_sm[M];      // sorted place of each place (0xffff likewise)
   __shared__ double raw_sm[M], med_sm[M];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   double sde_raw;
   const double scale = raw_scale(s, raw_parts, &sde_raw, sh), mean = s.state->mean_sr;
   const long long rows = n - k + 1, front = (n - rows) / 2;
@@ -226,49 +226,40 @@ __global__ void __launch_bounds__(M) spec_median_kernel(const double* __restrict
     idx_sm[tid] = (unsigned short)idx;
     if (idx != 0xffff) rank_sm[idx] = (unsigned short)tid;
     __syncthreads();
-    // rows a..b-1 of the tile by this warp
-    const int per = (nrow + kWords - 1) / kWords, a = min(nrow, wid * per), b = min(nrow, a + per);
-    if (a < b) {
-      unsigned word = 0;
-      if (lane < kWords)
-        for (int q = 0; q < 32; ++q) {
-          const int place = idx_sm[32 * lane + q];
-          if (place != 0xffff && place >= a && place < a + k) word |= 1u << q;
-        }
-      int cnt = (int)__reduce_add_sync(0xffffffffu, __popc(word));
-      for (int row = a; row < b; ++row) {
-        if (row > a) {   // the window moves on
-          const int out = rank_sm[row - 1], inn = rank_sm[row + k - 1];
-          if (out != 0xffff) {
-            if (lane == out >> 5) word &= ~(1u << (out & 31));
-            --cnt;
-          }
-          if (inn != 0xffff) {
-            if (lane == inn >> 5) word |= 1u << (inn & 31);
-            ++cnt;
-          }
-        }
-        const int pc = __popc(word);
-        int inc = pc;
-#pragma unroll
-        for (int o = 1; o < kWords; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += y;
-        }
-        const int before = inc - pc;
-        const int hi_r = cnt / 2, lo_r = (cnt & 1) ? hi_r : hi_r - 1;
-        auto value_of = [&](int r) {   // the r-th smallest of the window
-          const unsigned has = __ballot_sync(0xffffffffu, r >= before && r < inc);
-          const int at = has >> lane & 1 ? 32 * lane + nth_bit(word, r - before) : 0;
-          return has ? key_sm[__shfl_sync(0xffffffffu, at, __ffs(has) - 1)] : NAN;
-        };
-        double med = NAN;
-        if (cnt > 0) {
-          const double lo = value_of(lo_r), hi = (cnt & 1) ? lo : value_of(hi_r);
-          med = (lo + hi) / 2.0;
-        }
-        if (lane == 0) med_sm[row] = med;
+    // rows a..b-1 of the tile by this lane's group of kWords lanes
+    const int gl = tid % kWords, per = (nrow + 31) / 32;   // 32 groups
+    const int a = min(nrow, tid / kWords * per), b = min(nrow, a + per);
+    const unsigned group = (kWords == 32 ? 0xffffffffu : ((1u << kWords) - 1u)) << (lane - gl);
+    unsigned word = 0;
+#pragma unroll 4
+    for (int q = 0; q < 32; ++q) {
+      const int place = idx_sm[32 * gl + q];
+      if (place != 0xffff && place >= a && place < a + k) word |= 1u << q;
+    }
+    for (int row = a; row < a + per; ++row) {   // the whole warp keeps step
+      if (row > a && row < b) {   // the window moves on
+        const int out = rank_sm[row - 1], inn = rank_sm[row + k - 1];
+        if (out != 0xffff && gl == out >> 5) word &= ~(1u << (out & 31));
+        if (inn != 0xffff && gl == inn >> 5) word |= 1u << (inn & 31);
       }
+      const int pc = __popc(word);
+      int inc = pc;
+#pragma unroll
+      for (int o = 1; o < kWords; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o, kWords);
+        if (gl >= o) inc += y;
+      }
+      const int before = inc - pc, cnt = __shfl_sync(0xffffffffu, inc, kWords - 1, kWords);
+      const int hi_r = cnt / 2, lo_r = (cnt & 1) ? hi_r : hi_r - 1;
+      // the middle one or two of the window, from the lanes that hold them
+      const bool has_lo = lo_r >= before && lo_r < inc, has_hi = hi_r >= before && hi_r < inc;
+      double lo = 0, hi = 0;
+      if (has_lo) lo = key_sm[32 * gl + nth_bit(word, lo_r - before)];
+      if (has_hi) hi = hi_r == lo_r ? lo : key_sm[32 * gl + nth_bit(word, hi_r - before)];
+      const unsigned lo_at = __ballot_sync(0xffffffffu, has_lo) & group, hi_at = __ballot_sync(0xffffffffu, has_hi) & group;
+      lo = __shfl_sync(0xffffffffu, lo, lo_at ? __ffs(lo_at) - 1 : lane);
+      hi = __shfl_sync(0xffffffffu, hi, hi_at ? __ffs(hi_at) - 1 : lane);
+      if (gl == 0 && row < b) med_sm[row] = cnt > 0 ? (lo + hi) * 0.5 : NAN;
     }
     __syncthreads();
     // a thread per place: its row is the one that it is the middle of, or the nearest
@@ -375,8 +366,8 @@ __global__ void __launch_bounds__(kSpecThreads) spec_scale_kernel(long long n, d
 
 int spectra_launch(const double* chi2, const uint8_t* mask, long long n, int k, double* sr, double* praw,
                    double* power, SpecScratch s, cudaStream_t st) {
-  // at most kSpecCtas CTAs; eight values a thread, so that a short spectrum is few CTAs
-  const int ctas = (int)std::min<long long>(kSpecCtas, (n + 8 * kSpecThreads - 1) / (8 * kSpecThreads));
+  // two values a thread, at most kSpecCtas CTAs
+  const int ctas = (int)std::min<long long>(kSpecCtas, (n + 2 * kSpecThreads - 1) / (2 * kSpecThreads));
   int launches = 3;
   spec_min_kernel<<<ctas, kSpecThreads, 0, st>>>(chi2, mask, n, s);
   spec_sr_kernel<<<ctas, kSpecThreads, 0, st>>>(chi2, mask, n, sr, s);
