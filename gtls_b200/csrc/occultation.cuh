@@ -1,7 +1,7 @@
 // Occultation of a star with quadratic limb darkening by an opaque disk, by
 // the quadrature of gtls_b200/ldmodel.py (96-node Gauss-Legendre after the
 // substitution r = m + h sin(theta)), in forms shared by the adjoint model
-// (adjoint.cu, with dual-number derivatives in (z, p)) and the transit
+// (adjoint.cu, with derivatives in (z, p)) and the transit
 // template generator (templates.cu).  ldmodel stands in for the batman light
 // curve of the reference (src/gputls/transit.py:8-42).
 #pragma once
@@ -59,91 +59,48 @@ static const GLTable& gl_table() {
   return g;
 }
 
-// value and derivatives with respect to (z, p)
-struct D2 {
-  double v, z, p;
-};
-__device__ __forceinline__ D2 d2(double v) { return {v, 0.0, 0.0}; }
-__device__ __forceinline__ D2 operator+(D2 a, D2 b) { return {a.v + b.v, a.z + b.z, a.p + b.p}; }
-__device__ __forceinline__ D2 operator-(D2 a, D2 b) { return {a.v - b.v, a.z - b.z, a.p - b.p}; }
-__device__ __forceinline__ D2 operator*(D2 a, D2 b) {
-  return {a.v * b.v, a.v * b.z + b.v * a.z, a.v * b.p + b.v * a.p};
-}
-__device__ __forceinline__ D2 operator*(D2 a, double s) { return {a.v * s, a.z * s, a.p * s}; }
-__device__ __forceinline__ D2 operator/(D2 a, D2 b) {
-  const double q = a.v / b.v;
-  return {q, (a.z - q * b.z) / b.v, (a.p - q * b.p) / b.v};
-}
-// value of double inputs: the same expressions without derivatives
-__device__ __forceinline__ double dval(double a) { return a; }
-__device__ __forceinline__ double dval(D2 a) { return a.v; }
-
-// mu = sqrt(max(1 - r^2, 0)) and its derivative (0 where clamped)
+// mu = sqrt(max(1 - r^2, 0))
 __device__ __forceinline__ double mu_of(double r) {
   const double x = 1.0 - r * r;
   return x > 0.0 ? sqrt(x) : 0.0;
 }
-__device__ __forceinline__ D2 mu_of(D2 r) {
-  const double x = 1.0 - r.v * r.v;
-  if (!(x > 0.0)) return d2(0.0);
-  const double m = sqrt(x);
-  const double k = -r.v / m;
-  return {m, k * r.z, k * r.p};
-}
-// acos of c clamped to [-1, 1] (derivative 0 where clamped)
+// acos of c clamped to [-1, 1]
 __device__ __forceinline__ double acos_clamped(double c) {
   return c >= 1.0 ? 0.0 : (c <= -1.0 ? kPi : acos(c));
 }
-__device__ __forceinline__ D2 acos_clamped(D2 c) {
-  if (c.v >= 1.0) return d2(0.0);
-  if (c.v <= -1.0) return d2(kPi);
-  const double s = 1.0 - c.v * c.v;
-  const double k = s > 0.0 ? -1.0 / sqrt(s) : 0.0;
-  return {acos(c.v), k * c.z, k * c.p};
-}
-
-// Constants of either scalar type.
-template <typename T> __device__ __forceinline__ T cst(double v);
-template <> __device__ __forceinline__ double cst<double>(double v) { return v; }
-template <> __device__ __forceinline__ D2 cst<D2>(double v) { return d2(v); }
 
 // Moments M0..M2 of the occulted flux: lambda = (M0 - u1 M1 - u2 M2) / (pi K),
 // Mk = int (1 - mu)^k x (2 pi r over the covered disk, 2 r acos(c) over the
-// partly covered annuli) dr, both by the quadrature of ldmodel.occulted_fraction.
-template <typename T>
-__device__ __forceinline__ void occultation_moments(T Z, T Pp, const GLTable& g, T (&M)[3]) {
+// partly covered annuli) dr, both by the quadrature of ldmodel.occulted_fraction
+// (its nodes j0, j0 + step, ...).
+__device__ __forceinline__ void occultation_moments(double z, double p, const GLTable& g, double (&M)[3], int j0 = 0,
+                                                    int step = 1) {
 #pragma unroll
-  for (int k = 0; k < 3; ++k) M[k] = cst<T>(0.0);
-  const double z = dval(Z), p = dval(Pp);
-  const T one = cst<T>(1.0);
+  for (int k = 0; k < 3; ++k) M[k] = 0.0;
   // region fully covered by the planet: r in [0, min(p - z, 1)]
   if (p - z > 0.0) {
-    const T ih = p - z > 1.0 ? one : Pp - Z;
-    const T half = ih * 0.5;
-    for (int j = 0; j < kGLN; ++j) {
-      const T r = half + half * g.s[j];
-      const T wt = half * g.jw[j];
-      const T om = one - mu_of(r);
-      const T f = r * wt * (2.0 * kPi);
+    const double half = (p - z > 1.0 ? 1.0 : p - z) * 0.5;
+    for (int j = j0; j < kGLN; j += step) {
+      const double r = half + half * g.s[j];
+      const double om = 1.0 - mu_of(r);
+      const double f = r * (half * g.jw[j]) * (2.0 * kPi);
       M[0] = M[0] + f;
       M[1] = M[1] + f * om;
       M[2] = M[2] + f * om * om;
     }
   }
   // partially covered annuli: r in [|z - p|, min(1, z + p)]
-  const T lo = z >= p ? Z - Pp : Pp - Z;
-  const T hi = z + p > 1.0 ? one : Z + Pp;
-  if (dval(hi) > dval(lo)) {
-    const T mid = (lo + hi) * 0.5;
-    const T half = (hi - lo) * 0.5;
-    const T zs = z > 1e-300 ? Z : cst<T>(1e-300);
-    const T zp2 = zs * zs - Pp * Pp;
-    for (int j = 0; j < kGLN; ++j) {
-      const T r = mid + half * g.s[j];
-      const T wt = half * g.jw[j];
-      const T c = (r * r + zp2) / (r * zs * 2.0);
-      const T om = one - mu_of(r);
-      const T f = r * acos_clamped(c) * wt * 2.0;
+  const double lo = z >= p ? z - p : p - z;
+  const double hi = z + p > 1.0 ? 1.0 : z + p;
+  if (hi > lo) {
+    const double mid = (lo + hi) * 0.5, half = (hi - lo) * 0.5;
+    const double zs = z > 1e-300 ? z : 1e-300;
+    const double zp2 = zs * zs - p * p;
+    for (int j = j0; j < kGLN; j += step) {
+      const double r = mid + half * g.s[j];
+      const double c = (r * r + zp2) / (r * zs * 2.0);
+      const double om = 1.0 - mu_of(r);
+      const double f = r * acos_clamped(c) * (half * g.jw[j]) * 2.0;
       M[0] = M[0] + f;
       M[1] = M[1] + f * om;
       M[2] = M[2] + f * om * om;
@@ -151,13 +108,81 @@ __device__ __forceinline__ void occultation_moments(T Z, T Pp, const GLTable& g,
   }
 }
 
+// N = M0 - u1 M1 - u2 M2 with its derivatives in (z, p), and M1, M2 (which are
+// minus its derivatives in u1, u2): the derivatives of the discrete quadrature
+// itself, through the nodes, the limits and c.  Written out by hand, with one
+// reciprocal per node where general dual numbers divide five times; where a
+// square root or the acos is clamped its derivative is 0.
+struct OccultationGrad {
+  double N, Nz, Np, M1, M2;
+};
+__device__ __forceinline__ OccultationGrad occultation_grad(double z, double p, double u1, double u2,
+                                                            const GLTable& g, int j0, int step) {
+  OccultationGrad o{0.0, 0.0, 0.0, 0.0, 0.0};
+  // one node: f and its derivatives times the intensity at r
+  auto add = [&](double r, double rz, double rp, double f, double fz, double fp) {
+    const double x = 1.0 - r * r;
+    double mu = 0.0, k = 0.0;   // mu and r / mu = -dmu/dr
+    if (x > 0.0) {
+      const double s = rsqrt(x);
+      mu = x * s;
+      k = r * s;
+    }
+    const double om = 1.0 - mu;
+    const double I = 1.0 - om * (u1 + u2 * om), Ir = -(u1 + 2.0 * u2 * om) * k;
+    o.N = fma(f, I, o.N);
+    o.Nz += fz * I + f * Ir * rz;
+    o.Np += fp * I + f * Ir * rp;
+    const double fo = f * om;
+    o.M1 += fo;
+    o.M2 = fma(fo, om, o.M2);
+  };
+  if (p - z > 0.0) {
+    const bool whole = p - z > 1.0;
+    const double half = (whole ? 1.0 : p - z) * 0.5, hz = whole ? 0.0 : -0.5;   // dhalf/dp = -hz
+    for (int j = j0; j < kGLN; j += step) {
+      const double s1 = 1.0 + g.s[j], jw = g.jw[j] * (2.0 * kPi);
+      const double r = half * s1, wt = half * jw;
+      // f = r wt: both are half times a constant
+      const double fh = 2.0 * r * jw;
+      add(r, hz * s1, -hz * s1, r * wt, fh * hz, -fh * hz);
+    }
+  }
+  const bool out = z >= p, limb = z + p > 1.0;
+  const double lo = out ? z - p : p - z, hi = limb ? 1.0 : z + p;
+  if (hi > lo) {
+    const double mid = (lo + hi) * 0.5, half = (hi - lo) * 0.5;
+    const double loz = out ? 1.0 : -1.0, h1 = limb ? 0.0 : 1.0;   // dlo/dz = -dlo/dp; dhi/dz = dhi/dp
+    const double mz = 0.5 * (loz + h1), mp = 0.5 * (h1 - loz), hz = 0.5 * (h1 - loz), hp = 0.5 * (h1 + loz);
+    const bool centre = !(z > 1e-300);
+    const double zs = centre ? 1e-300 : z, dzs = centre ? 0.0 : 1.0;
+    const double zp2 = zs * zs - p * p;
+    for (int j = j0; j < kGLN; j += step) {
+      const double s = g.s[j], jw = 2.0 * g.jw[j];
+      const double r = mid + half * s, rz = mz + hz * s, rp = mp + hp * s;
+      const double inv = 1.0 / (2.0 * r * zs);
+      const double c = (r * r + zp2) * inv;
+      double ac = c >= 1.0 ? 0.0 : (c <= -1.0 ? kPi : c), acz = 0.0, acp = 0.0;   // (a NaN stays one)
+      if (c < 1.0 && c > -1.0) {
+        ac = acos(c);
+        const double d = 1.0 - c * c;
+        const double k = d > 0.0 ? -2.0 * inv * rsqrt(d) : 0.0;   // dacos/dc times 2 / (2 r z)
+        acz = k * (r * rz + zs * dzs - c * (rz * zs + r * dzs));
+        acp = k * (r * rp - p - c * rp * zs);
+      }
+      const double ra = r * ac, wt = half * jw;
+      add(r, rz, rp, ra * wt, (rz * ac + r * acz) * wt + ra * (hz * jw), (rp * ac + r * acp) * wt + ra * (hp * jw));
+    }
+  }
+  return o;
+}
 
 // Fraction of the stellar flux blocked by a disk of radius p at separation z
 // (ldmodel.occulted_fraction): 0 unless z < 1 + p and p > 0.
 __device__ __forceinline__ double occulted_fraction(double z, double p, double u1, double u2, const GLTable& g) {
   if (!(p > 0.0) || !(z < 1.0 + p)) return 0.0;
   double M[3];
-  occultation_moments<double>(z, p, g, M);
+  occultation_moments(z, p, g, M);
   return (M[0] - u1 * M[1] - u2 * M[2]) / (kPi * (1.0 - u1 / 3.0 - u2 / 6.0));
 }
 
