@@ -51,7 +51,7 @@ constexpr int kPrepSmallMaxN = 1 << 15;
 constexpr int kSmallBucket = 8;     // entries of buckets up to this size are ranked by their own thread
 constexpr int kSmallBucketSm = 32;  // the same, for buckets in shared memory
 constexpr int kBigBuckets = 512;    // capacity of the list of larger buckets (warp-ranked)
-constexpr int kMaxRounds = 32;      // rounds of the shared-memory prepare path
+constexpr int kMaxRounds = 96;      // rounds of the shared-memory prepare path
 constexpr int kRoundShift = 20;     // hist entries of that path: position | round << kRoundShift
 constexpr int kPosMask = (1 << kRoundShift) - 1;
 constexpr int kPrepStaticSmem = 4096;  // static shared memory of prepare_kernel, rounded up
@@ -252,27 +252,78 @@ __device__ __forceinline__ double fold_phase(double t, double P) {
   return x - (double)(int)x;
 }
 
-// Bucket of a phase from x = phase * NB (exact: NB = scale is a power of
-// two, and |phase| < 1): floor(x), clamped so that out-of-range phases land
-// in the first or last bucket.
-__device__ __forceinline__ int phase_bin(double x, int nb) {
-  int b = (int)x;
-  b = b < 0 ? 0 : b;
-  return b >= nb ? nb - 1 : b;
+// Bucket (y) of a phase and its key within the bucket (x): the bucket is
+// floor(phase * NB), NB a power of two, clamped so that out-of-range phases
+// land in the first or last one; the key is 32 bits of the fraction, rounded
+// down, which never reverses an order.  The key resolves 2^-46 of a turn at
+// 2^14 buckets: phases of samples more than 64 turns from t = 0 are no finer,
+// so that their keys differ wherever they do (a float's 24 bits left ties
+// by the hundred on periods commensurate with the cadence).
+__device__ __forceinline__ uint2 phase_key(double phase, int nb_log2) {
+  const int nb = 1 << nb_log2;
+  const double x = phase * (double)nb;
+  const double b = floor(x);
+  if (!(b >= 0.0)) return make_uint2(0u, 0u);
+  if (b >= (double)nb) return make_uint2(~0u, (unsigned)(nb - 1));
+  return make_uint2(__double2uint_rd((x - b) * 0x1p32), (unsigned)b);
 }
 
+// The same of sample times.  The quotient is the correctly rounded t / P
+// without a division: from the rounded reciprocal r of P, two corrections
+// q += r (t - q P), each remainder a fused multiply-add.  The first leaves q
+// within one unit of the last place, and from such a q the second rounds
+// correctly when r is itself rounded correctly (P. Markstein, IBM J. Res. Dev.
+// 34, 1990, theorem on the final step of division).  Adding 2^52 rounded down
+// then leaves the whole turns, and adding 2^20 / NB to the phase its bucket
+// and key in the sum's two words: no branch and no conversion, so
+// that a thread's samples overlap (the divide's own branch kept them one after
+// the other; 70,000 samples: 0.95 -> 0.88 us a period).  Turn counts outside [2^-200, 2^31) and extreme periods
+// are divided.
+struct FoldKey {
+  double P, r, place;
+  int nb_log2;
+  __device__ __forceinline__ FoldKey(double P_, int nbl) : P(P_), nb_log2(nbl) {
+    r = P_ >= 0x1p-200 && P_ <= 0x1p200 ? __drcp_rn(P_) : __longlong_as_double(0x7ff8000000000000LL);
+    place = __hiloint2double((1023 + 20 - nbl) << 20, 0);
+  }
+  template <int kB>
+  __device__ __forceinline__ void operator()(const double (&t)[kB], uint2 (&w)[kB]) const {
+    double x[kB];
+#pragma unroll
+    for (int u = 0; u < kB; ++u) x[u] = __dmul_rn(t[u], r);
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int u = 0; u < kB; ++u) x[u] = __fma_rn(__fma_rn(-x[u], P, t[u]), r, x[u]);
+#pragma unroll
+    for (int u = 0; u < kB; ++u) {
+      const double z = __dadd_rd(__dsub_rn(x[u], __dsub_rn(__dadd_rd(x[u], 0x1p52), 0x1p52)), place);
+      w[u] = make_uint2((unsigned)__double2loint(z), (unsigned)__double2hiint(z) & 0xfffffu);
+    }
+#pragma unroll
+    for (int u = 0; u < kB; ++u)
+      if ((unsigned)__double2hiint(x[u]) - 0x33700000u >= 0x41e00000u - 0x33700000u)
+        w[u] = phase_key(fold_phase(t[u], P), nb_log2);
+  }
+};
+
 // Strict order of two slots of the same bucket: by phase, then by original
-// index (the order of a stable argsort).  The 32-bit keys are the in-bucket
-// fractions rounded to float, which preserves every strict inequality; equal
-// keys are decided on the exact FP64 phases, recomputed.
-// Slot index words hold the sample index, and for curves of at most
-// kPackedMaxN samples also the bucket in the bits above it (the same for two
-// slots of one bucket, so comparing whole words compares the indices).
+// index (the order of a stable argsort).  Equal keys are decided on the exact
+// FP64 phases, recomputed.
+// Slot index words hold the sample index, and in the bits above it a bucket
+// where there is room (the same for two slots of one bucket, so comparing
+// whole words compares the indices): index_bits is 17 for curves of at most
+// 2^17 samples.
 constexpr int kPackedShift = 17;
 constexpr int kPackedMaxN = 1 << kPackedShift;
+constexpr int kRoundMaxN = (1 << 20) - 1;   // positions of the rounds' hist entries; 12 bits for a bucket of a round
+__host__ __device__ __forceinline__ int index_bits(int n) {
+  int b = kPackedShift;
+  while ((1 << b) < n) ++b;
+  return b;
+}
 __device__ __forceinline__ bool slot_less(uint2 a, uint2 b, const double* __restrict__ t, double P, unsigned imask) {
-  const float fa = __uint_as_float(a.x), fb = __uint_as_float(b.x);
-  if (fa != fb) return fa < fb;
+  if (a.x != b.x) return a.x < b.x;
   const double pa = fold_phase(t[a.y & imask], P), pb = fold_phase(t[b.y & imask], P);
   if (pa != pb) return pa < pb;
   return a.y < b.y;
@@ -282,7 +333,7 @@ __device__ __forceinline__ bool slot_less(uint2 a, uint2 b, const double* __rest
 // original index)), by a whole warp: each lane ranks one entry of a group of
 // 32 against the bucket, streamed 32 entries at a time and broadcast by
 // shuffles.  Used for large buckets, whose O(k^2) comparisons would
-// otherwise fall on single threads.
+// otherwise fall on single threads, where sort_bucket_warp cannot be.
 template <typename Emit>
 __device__ __forceinline__ void rank_bucket_warp(const uint2* __restrict__ slot, int s, int e,
                                                  const double* __restrict__ t, double P, unsigned imask, Emit emit) {
@@ -305,6 +356,74 @@ __device__ __forceinline__ void rank_bucket_warp(const uint2* __restrict__ slot,
   }
 }
 
+// The same by sorting the bucket in place in shared memory, for buckets of a
+// period commensurate with the cadence (hundreds to thousands of samples at a
+// few phases; by comparing all pairs, a division in most, such a period
+// took milliseconds: 800 periods of a 70,000-sample curve, of which a few are
+// so, 2.2 -> 0.84 us each on average).  Each entry becomes one 64-bit word, the fraction of the
+// bucket in fixed point above the ib bits of its index: with 64 - ib bits
+// every phase is exact but those below 2^-10 of the samples before the first
+// turn ends, so that the words sort as a stable argsort does.  A bucket with a
+// fraction that is not exact takes rank_bucket_warp.  A network of
+// ascending comparators (each merge starts with the mirrored pairs) works on any
+// length: pairs that reach past the end are left out.  The slots keep
+// their index words.
+template <typename Emit>
+__device__ __noinline__ void sort_bucket_warp(uint2* __restrict__ slot, int s, int e, int b, int nb_log2, int ib,
+                                              unsigned high, const double* __restrict__ t, double P, Emit emit) {
+  const int lane = threadIdx.x & 31, k = e - s;
+  const unsigned imask = (1u << ib) - 1u;
+  unsigned long long* const w = reinterpret_cast<unsigned long long*>(slot) + s;
+  const double unit = (double)(1ULL << (63 - ib)) * 2.0;
+  bool exact = true;
+  for (int j = lane; j < k; j += 32) {
+    const unsigned i = slot[s + j].y & imask;
+    const double y = (fold_phase(t[i], P) * (double)(1 << nb_log2) - (double)b) * unit;
+    const bool ok = y >= 0.0 && y < unit && y == floor(y);
+    exact = exact && ok;
+    w[j] = (ok ? (unsigned long long)y << ib : 0ULL) | i;
+  }
+  __syncwarp();
+  if (!__all_sync(0xffffffffu, exact)) {
+    for (int j = lane; j < k; j += 32) {
+      const unsigned i = (unsigned)w[j] & imask;
+      slot[s + j] = make_uint2(phase_key(fold_phase(t[i], P), nb_log2).x, i | high);
+    }
+    __syncwarp();
+    rank_bucket_warp(slot, s, e, t, P, imask, emit);
+    return;
+  }
+  auto order = [&](int i, int j) {
+    if (j >= k) return;
+    const unsigned long long x = w[i], y = w[j];
+    if (y < x) {
+      w[i] = y;
+      w[j] = x;
+    }
+  };
+  int half = 1;   // pairs of the padded length
+  while (2 * half < k) half *= 2;
+  for (int p = 1; p <= half; p *= 2) {   // sorted runs of p become runs of 2 p
+    for (int c = lane; c < half; c += 32) {
+      const int i = 2 * c - (c & (p - 1));
+      order(i, i ^ (2 * p - 1));
+    }
+    __syncwarp();
+    for (int q = p / 2; q > 0; q /= 2) {
+      for (int c = lane; c < half; c += 32) {
+        const int i = 2 * c - (c & (q - 1));
+        order(i, i + q);
+      }
+      __syncwarp();
+    }
+  }
+  for (int j = lane; j < k; j += 32) {
+    const unsigned i = (unsigned)w[j] & imask;
+    emit(s + j, (int)i);
+    slot[s + j].y = i | high;
+  }
+}
+
 // Round tables of the shared-memory prepare path.
 struct RoundTables {
   int nrounds;               // rounds; -1: the period takes the global-scatter path
@@ -313,11 +432,12 @@ struct RoundTables {
   int cursor[kMaxRounds];    // append cursors of the round-partitioned sample words
 };
 
-// Shared-memory prepare of one period (curves of at most kPackedMaxN
+// Shared-memory prepare of one period (curves of at most kRoundMaxN
 // samples).  The samples are folded (GPUFun.py:30-41) and counted into NB
 // phase buckets; the buckets are cut greedily into rounds of whole buckets
-// holding at most `cap` samples each; a second fold appends each sample's
-// word (in-bucket key, index | bucket << kPackedShift) to its round's range
+// holding at most `cap` samples each (and no more buckets than the index word
+// has room for); a second fold appends each sample's word (in-bucket key,
+// index | bucket << ib, ib = index_bits(n), of which the low bits stay) to its round's range
 // of the scratch row `stage` (warp-aggregated, so the stores stay nearly
 // coalesced).  Each round then
 //   (a) reads its words (coalesced) into shared-memory slots by bucket,
@@ -329,18 +449,22 @@ struct RoundTables {
 // written nothing, when a single bucket holds more than `cap` samples or more
 // than kMaxRounds rounds would be needed; the caller then takes the global
 // path.  Dynamic shared memory: hist [NB] ints, slots [cap] words.
+// kIndexBits: index_bits(n) where it is kPackedShift (every bucket number fits
+// above it), else 0.
+template <int kIndexBits>
 __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int* nbig, RoundTables& rt,
                                const double* __restrict__ t, int n, double P, int nb_log2, int cap,
                                uint2* __restrict__ stage, int* __restrict__ ord) {
   const int nb = 1 << nb_log2;
-  const double scale = (double)nb;
-  constexpr unsigned imask = (unsigned)(kPackedMaxN - 1);
+  const int ib = kIndexBits ? kIndexBits : index_bits(n);
+  const unsigned imask = (1u << ib) - 1u;
   int* hist = dyn;
   uint2* slots = reinterpret_cast<uint2*>(dyn + nb);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  constexpr int kB = 2;   // elements per thread in flight in each pass (4 and 8 measured slower)
+  constexpr int kB = 3;   // elements per thread in flight in each pass (2 and 4: 5% slower, short curves 8%)
   const int stride = blockDim.x * kB;
 
+  const FoldKey fold(P, nb_log2);
   for (int b = threadIdx.x; b < nb; b += blockDim.x) hist[b] = 0;
   __syncthreads();
   // (1) fold and histogram of buckets
@@ -349,12 +473,14 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
-      tv[u] = i < n ? t[i] : 0.0;
+      tv[u] = i < n ? t[i] : P;   // (a padding of 0 would take the divide)
     }
+    uint2 wd[kB];
+    fold(tv, wd);
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
-      if (i < n) atomicAdd(&hist[phase_bin(fold_phase(tv[u], P) * scale, nb)], 1);
+      if (i < n) atomicAdd(&hist[wd[u].y], 1);
     }
   }
   __syncthreads();
@@ -371,7 +497,7 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
     }
     while (b0 < nb) {
       const int lim = S(b0) + cap;
-      int lo = b0, hi = nb;   // S(lo) <= lim; the answer lies in [lo, hi]
+      int lo = b0, hi = min(nb, b0 + (int)(~0u >> ib) + 1);   // S(lo) <= lim; the answer lies in [lo, hi]
       while (lo < hi) {
         const int step = (hi - lo + 31) >> 5;
         const int x = min(hi, lo + (lane + 1) * step);
@@ -402,6 +528,10 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
   for (int b = threadIdx.x; b < nb; b += blockDim.x)
     hist[b] |= upper_find(0, nr, b, [&](int q) { return (long long)rt.rb[q]; }) << kRoundShift;
   auto H = [&](int b) { return hist[b] & kPosMask; };
+  // the bucket of a word of the round from b0 on, from its low bits
+  auto bucket_of = [&](unsigned y, int b0) { 
+    return kIndexBits ? (int)(y >> ib) : b0 + (int)(((y >> ib) - (unsigned)b0) & (~0u >> ib));
+  };
   __syncthreads();
   // (3) fold again; each sample's word to its round's range of the scratch
   //     row (the loop runs over whole warps for the warp-wide match)
@@ -410,19 +540,15 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + lane + u * blockDim.x;
-      tv[u] = i < n ? t[i] : 0.0;
+      tv[u] = i < n ? t[i] : P;   // (a padding of 0 would take the divide)
     }
+    uint2 wds[kB];
+    fold(tv, wds);
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + lane + u * blockDim.x;
-      int r = -1;
-      uint2 wd = make_uint2(0u, 0u);
-      if (i < n) {
-        const double x = fold_phase(tv[u], P) * scale;
-        const int b = phase_bin(x, nb);
-        wd = make_uint2(__float_as_uint((float)(x - (double)b)), (unsigned)i | ((unsigned)b << kPackedShift));
-        r = hist[b] >> kRoundShift;
-      }
+      const int r = i < n ? hist[wds[u].y] >> kRoundShift : -1;
+      const uint2 wd = make_uint2(wds[u].x, (unsigned)i | wds[u].y << ib);
       const unsigned peers = __match_any_sync(0xffffffffu, r);
       const int leader = __ffs(peers) - 1;
       int pos = 0;
@@ -449,7 +575,7 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
       for (int u = 0; u < kB; ++u) {
         const int q = q0 + u * blockDim.x;
         if (q < cnt) {
-          const int b = (int)(wd[u].y >> kPackedShift);
+          const int b = bucket_of(wd[u].y, b0);
           const int sl = (atomicAdd(&hist[b], 1) & kPosMask) - rs;
           if ((unsigned)sl < (unsigned)cnt) slots[sl] = wd[u];   // always true: the counts of pass (1)
         }
@@ -485,8 +611,9 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
     if (warp_ranked)
       for (int q = wid; q < nbg; q += nwarp) {
         const int b = big[q];
-        rank_bucket_warp(slots, (b == 0 ? 0 : H(b - 1)) - rs, H(b) - rs, t, P, imask, emit);
+        sort_bucket_warp(slots, (b == 0 ? 0 : H(b - 1)) - rs, H(b) - rs, b, nb_log2, ib, (unsigned)b << ib, t, P, emit);
       }
+    if (warp_ranked && nbg > 0) __syncthreads();   // the sorted slots' index words are back
     for (int j0 = threadIdx.x; j0 < cnt; j0 += stride) {
       int pos[kB], idx[kB];
 #pragma unroll
@@ -496,7 +623,7 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
         idx[u] = 0;
         if (j < cnt) {
           const uint2 sj = slots[j];
-          const int b = (int)(sj.y >> kPackedShift);
+          const int b = bucket_of(sj.y, b0);
           const int s = (b == 0 ? 0 : H(b - 1)) - rs;
           const int e = H(b) - rs;
           idx[u] = (int)(sj.y & imask);
@@ -505,17 +632,17 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
           } else if (e - s <= kSmallBucketSm || !warp_ranked) {
             // entries of smaller key, and of equal key (itself included);
             // equal keys, rare, are then ordered on the exact phases
-            const float kj = __uint_as_float(sj.x);
+            const unsigned kj = sj.x;
             int lt = 0, eq = 0;
 #pragma unroll 4
             for (int m = s; m < e; ++m) {
-              const float km = __uint_as_float(slots[m].x);
+              const unsigned km = slots[m].x;
               lt += km < kj;
               eq += km == kj;
             }
             if (eq > 1)
               for (int m = s; m < e; ++m)
-                if (m != j && __uint_as_float(slots[m].x) == kj) lt += slot_less(slots[m], sj, t, P, imask);
+                if (m != j && slots[m].x == kj) lt += slot_less(slots[m], sj, t, P, imask);
             pos[u] = s + lt;
           }
         }
@@ -552,20 +679,26 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
   const int n = C.n;
   const int nb_log2 = C.nb_log2;
   const int nb = 1 << nb_log2;
-  const double scale = (double)nb;
   const bool packed = n <= kPackedMaxN && nb_log2 <= 32 - kPackedShift;
   const unsigned imask = packed ? (unsigned)(kPackedMaxN - 1) : 0xffffffffu;
   const double P = C.periods[R.pidx0 + local];
   uint2* slot = scr_slot + R.slot_off - runs[0].slot_off + (size_t)local * n;
   int* ord = order + R.slot_off + (size_t)local * n;
-  constexpr int kB = 4;   // elements per thread in flight in each pass
+  constexpr int kB = 3;   // elements per thread in flight in each pass (2 and 4: 5% slower, short curves 8%)
   const int stride = blockDim.x * kB;
   __shared__ RoundTables rt;
-  if (C.rnb_log2 > 0 && prepare_rounds(hist, wtmp_i, big, &nbig, rt, t, n, P, C.rnb_log2, C.rcap, slot, ord)) return;
+  if (C.rnb_log2 > 0) {
+    const bool done =
+        n <= kPackedMaxN
+            ? prepare_rounds<kPackedShift>(hist, wtmp_i, big, &nbig, rt, t, n, P, C.rnb_log2, C.rcap, slot, ord)
+            : prepare_rounds<0>(hist, wtmp_i, big, &nbig, rt, t, n, P, C.rnb_log2, C.rcap, slot, ord);
+    if (done) return;
+  }
   // global path: buckets scattered through the scratch row
 
   for (int b = threadIdx.x; b < nb; b += blockDim.x) hist[b] = 0;
   if (threadIdx.x == 0) nbig = 0;
+  const FoldKey fold(P, nb_log2);
   __syncthreads();
   // (1) fold and histogram of buckets
   for (int i0 = threadIdx.x; i0 < n; i0 += stride) {
@@ -573,12 +706,14 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
-      tv[u] = i < n ? t[i] : 0.0;
+      tv[u] = i < n ? t[i] : P;   // (a padding of 0 would take the divide)
     }
+    uint2 wd[kB];
+    fold(tv, wd);
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
-      if (i < n) atomicAdd(&hist[phase_bin(fold_phase(tv[u], P) * scale, nb)], 1);
+      if (i < n) atomicAdd(&hist[wd[u].y], 1);
     }
   }
   __syncthreads();
@@ -590,17 +725,18 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
-      tv[u] = i < n ? t[i] : 0.0;
+      tv[u] = i < n ? t[i] : P;   // (a padding of 0 would take the divide)
     }
+    uint2 wd[kB];
+    fold(tv, wd);
 #pragma unroll
     for (int u = 0; u < kB; ++u) {
       const int i = i0 + u * blockDim.x;
       if (i < n) {
-        const double x = fold_phase(tv[u], P) * scale;
-        const int b = phase_bin(x, nb);
+        const uint2 at = wd[u];
+        const int b = (int)at.y;
         const int s = atomicAdd(&hist[b], 1);
-        const float f = (float)(x - (double)b);
-        slot[s] = make_uint2(__float_as_uint(f), (unsigned)i | (packed ? (unsigned)b << kPackedShift : 0u));
+        slot[s] = make_uint2(at.x, (unsigned)i | (packed ? (unsigned)b << kPackedShift : 0u));
       }
     }
   }
@@ -924,14 +1060,15 @@ static int nb_log2_for(int n, int shift) {
 // Shared-memory prepare path of a curve of n samples: NB = 2^(ceil(log2 n) -
 // 2) buckets (at most 2^14, about four samples a bucket), and the largest
 // round capacity that fits the CTA's shared memory next to them (8 bytes a
-// sample: the slot word).  Off (0) for curves beyond the packed slot words or
-// when fewer than 1,024 samples fit a round.
+// sample: the slot word).  Off (0) for curves beyond kRoundMaxN (the words'
+// scatter through global memory, 6.6 us a period of 160,000 samples, takes 2.9
+// in rounds) or when fewer than 1,024 samples fit a round.
 template <typename Real>
 static void rounds_params(CurveDev<Real>& C, int smem_optin) {
   C.rnb_log2 = 0;
   C.rcap = 0;
   const int n = C.n;
-  if (n < 1 || n > kPackedMaxN) return;
+  if (n < 1 || n > kRoundMaxN) return;
   int k = 1;
   while ((1 << k) < n) ++k;
   const int nbl = std::max(1, std::min(14, k - 2));
