@@ -15,6 +15,8 @@ constexpr int kCoarseCap = 2240;                 // prefix values kept at every 
 constexpr int kCoarseStep = 24;                  // g wanted when the range may be split
 constexpr int kTaskGroupsMain = 4, kTaskGroupsAll = 8;   // groups of 32 starts of one task (its queue entries fit a byte)
 constexpr int kSplitW = 1024;                    // wider windows are summed by the whole CTA
+constexpr int kTogether = 4;                     // overlapping ones summed together, FP64
+constexpr int kStage = 4096;                     // samples of theirs in shared memory at a time
 constexpr int kProbe = 16;                       // all-starts pass: first sweep over every (width / kProbe)-th start
 constexpr int kList = 4096;                      // starts of a CTA that wait for their sums, main pass
 constexpr int kListAll = 16384;                  // and all-starts pass
@@ -29,6 +31,8 @@ constexpr int kBlockSlots = 2048;                // blocks of a CTA
 __host__ __device__ __forceinline__ int skew(int p) { return p + (p >> 5); }
 constexpr int kRingWords = kRing + kRing / 32;
 constexpr int kCoarseWords = kCoarseCap + kCoarseCap / 32;
+constexpr int kPartWords = kTogether * (kChiThreads / 32) * 6;   // words of their warps' sums, before the samples
+static_assert(kPartWords % 4 == 0 && kPartWords + 4 * kStage <= 4 * kRingWords, "");
 constexpr size_t kChiSmemRing = 4 * sizeof(float) * kRingWords;
 constexpr size_t kChiSmemCoarse = 3 * sizeof(float) * kCoarseWords;
 // Dynamic shared memory: the rings, the coarse arrays, and per duration of the
@@ -308,6 +312,72 @@ __device__ __noinline__ void evaluate(const Exact<Real>& x, int u, int k) {
                                     x.trows + x.trow_off[x.dur[u]]));
 }
 
+// The parts, one a warp, of the sums of up to kTogether wide windows (>
+// kSplitW) by the CTA, each in part_sums' order.  What bounds a wide window is
+// its scattered (v, w) reads, a sector each (24,000 clocks for 8,000 samples with two
+// CTAs on the SM); the waiting starts lie around the same few dips, so the
+// samples go through shared memory once for all.
+__device__ __noinline__ void group_sums(const Exact<double>& x, const int2* which, int cnt, double2* stage,
+                                        Sums<double>* parts) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int k[kTogether], w[kTogether], lo = 0x7fffffff, hi = 0;
+  const double2* trow[kTogether];
+  Sums<double> sum[kTogether];
+#pragma unroll
+  for (int q = 0; q < kTogether; ++q) {
+    const int u = q < cnt ? which[q].x : -1;
+    k[q] = u >= 0 ? which[q].y : 0;
+    w[q] = u >= 0 ? (int)(x.wsk[u] & 0xffff) : 0;
+    trow[q] = x.trows + (u >= 0 ? x.trow_off[x.dur[u]] : 0);
+    sum[q] = Sums<double>{0.0, 0.0, 0.0};
+    if (u >= 0) {
+      lo = min(lo, k[q]);
+      hi = max(hi, k[q] + w[q]);
+    }
+  }
+  for (int c0 = lo; c0 < hi; c0 += kStage) {
+    const int len = min(kStage, hi - c0);
+    constexpr int kDeep = 6;
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < len; i0 += kDeep * kChiThreads) {
+      int idx[kDeep];
+#pragma unroll
+      for (int q = 0; q < kDeep; ++q) {
+        const int i = i0 + q * kChiThreads;
+        idx[q] = i < len ? x.fold.order[wrap_pos(c0 + i, x.fold.n)] : 0;
+      }
+      double2 g[kDeep];
+#pragma unroll
+      for (int q = 0; q < kDeep; ++q) g[q] = x.fold.vw[min(max(idx[q], 0), x.fold.n - 1)];
+#pragma unroll
+      for (int q = 0; q < kDeep; ++q) {
+        const int i = i0 + q * kChiThreads;
+        if (i < len) stage[i] = g[q];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTogether; ++q) {
+      const int from = c0 - k[q], to = min(w[q], from + len);
+      int i = threadIdx.x;
+      if (from > i) i += (from - i + kChiThreads - 1) / kChiThreads * kChiThreads;
+#pragma unroll 4
+      for (; i < to; i += kChiThreads) {
+        const double2 g = stage[i - from], t = trow[q][i];
+        sum[q].S += g.x;
+        sum[q].B = fma(t.x, g.x * g.y, sum[q].B);
+        sum[q].C = fma(t.y, g.y, sum[q].C);
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kTogether; ++q) {
+    if (q >= cnt) break;
+    const Sums<double> t{warp_sum(sum[q].S), warp_sum(sum[q].B), warp_sum(sum[q].C)};
+    if (lane == 0) parts[q * kChiWarps + wid] = t;
+  }
+}
+
 // One CTA per (period, range of starts).
 //
 // What bounds the stage: with every passing start summed it was the FMA pipe
@@ -346,7 +416,8 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   __shared__ ScreenRow row_sm[kChiWarps][2];
   __shared__ int list_n, tau_key, next_task, nring_sm, low_key, go_sm, redo_n, picked[2];
   __shared__ short pick[kChiThreads];
-  __shared__ Sums<Real> part[kChiWarps];
+  __shared__ double part_s[kChiWarps];
+  __shared__ int2 together[kTogether];          // union position (-1: ruled out) and start
   __shared__ unsigned maxbits[4];
   __shared__ double carry_v, wtot_v[kChiWarps];
   __shared__ float carry[3], wtot[kChiWarps][3];
@@ -1041,6 +1112,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         // this turn's entries of the next kChiThreads: narrow windows from the front of pick, wide from its end
         __syncthreads();
         if (threadIdx.x < 2) picked[threadIdx.x] = 0;
+        if (threadIdx.x == 0 && ntiles > 1) atomicMin(&tau_key, atomicMin(tau_all, *(volatile int*)&tau_key));
         __syncthreads();
         const int i = c0 + threadIdx.x;
         if (i < total) {
@@ -1083,44 +1155,81 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
             if (lane == 0) go = !over_tau(x.lb);   // one lane's view of tau for the warp
             if (__shfl_sync(0xffffffffu, go, 0)) evaluate<Real>(ex, x.u, x.k);
           }
-          for (int j = 0; j < nw; ++j) {   // the CTA together (a warp alone: 100,000 clocks for 10,000 samples)
-            const Waiting x = list[c0 + pick[kChiThreads - 1 - j]];
-            const int w = (int)(wsk[x.u] & 0xffff), s = (int)(wsk[x.u] >> 16);
-            const bool alone = sizeof(Real) == 4 && (s < 32 || s > kRingWords * 2);
-            __syncthreads();
-            if (threadIdx.x == 0) go_sm = !over_tau(x.lb);
-            __syncthreads();
-            if (!go_sm) continue;
-            if (alone) {
-              if (wid == 0) evaluate<Real>(ex, x.u, x.k);
-              continue;
+          // the CTA together (a warp alone: 100,000 clocks for 10,000 samples)
+          auto entry = [&](int j) { return list[c0 + pick[kChiThreads - 1 - j]]; };
+          if constexpr (sizeof(Real) == 8) {
+            // in order of their starts, up to kTogether whose windows overlap at a time
+            if (nw > 1) {
+              int* const keys = reinterpret_cast<int*>(dyn_f);   // the rings are free by now
+              const int j = threadIdx.x;
+              const short at = pick[kChiThreads - 1 - min(j, nw - 1)];
+              __syncthreads();
+              if (j < nw) keys[j] = list[c0 + at].k;
+              __syncthreads();
+              if (j < nw) {
+                int rank = 0;
+                for (int q = 0; q < nw; ++q) rank += keys[q] < keys[j] || (keys[q] == keys[j] && q < j);
+                pick[kChiThreads - 1 - rank] = at;
+              }
             }
-            const R2* __restrict__ trow = ex.trows + ex.trow_off[dur[x.u]];
-            if constexpr (sizeof(Real) == 8) {
-              const Sums<double> mine = part_sums(ex.fold, x.k, w, trow, 32 * wid, kChiThreads);
-              if (lane == 0) part[wid] = mine;
+            for (int j = 0; j < nw;) {
               __syncthreads();
               if (wid == 0) {
+                Waiting x{0.f, 0, 0};
+                int w = 0, go = 0;
+                if (lane < kTogether && j + lane < nw) {
+                  x = entry(j + lane);
+                  w = (int)(wsk[x.u] & 0xffff);
+                  go = !over_tau(x.lb);
+                }
+                int cnt = 1, end = __shfl_sync(0xffffffffu, x.k + w, 0);
+                for (; cnt < min(kTogether, nw - j); ++cnt) {
+                  if (__shfl_sync(0xffffffffu, x.k, cnt) >= end) break;
+                  end = max(end, __shfl_sync(0xffffffffu, x.k + w, cnt));
+                }
+                if (lane < cnt) together[lane] = make_int2(go ? x.u : -1, x.k);
+                if (lane == 0) go_sm = cnt;
+              }
+              __syncthreads();
+              const int cnt = go_sm;
+              Sums<double>* const parts = reinterpret_cast<Sums<double>*>(dyn_f);
+              group_sums(ex, together, cnt, reinterpret_cast<double2*>(dyn_f + kPartWords), parts);
+              __syncthreads();
+              if (wid < cnt && together[wid].x >= 0) {
                 Sums<double> t{0.0, 0.0, 0.0};
                 for (int p = 0; p < kChiWarps; ++p) {
-                  t.S += part[p].S;
-                  t.B += part[p].B;
-                  t.C += part[p].C;
+                  t.S += parts[wid * kChiWarps + p].S;
+                  t.B += parts[wid * kChiWarps + p].B;
+                  t.C += parts[wid * kChiWarps + p].C;
                 }
-                settle<Real>(ex, x.u, x.k, t);
+                settle<Real>(ex, together[wid].x, together[wid].y, t);
               }
-            } else {
-              float2* const prs = reinterpret_cast<float2*>(dyn_f);   // the rings are free by now
+              j += cnt;
+            }
+          } else {
+            for (int j = 0; j < nw; ++j) {
+              const Waiting x = entry(j);
+              const int w = (int)(wsk[x.u] & 0xffff), s = (int)(wsk[x.u] >> 16);
+              __syncthreads();
+              if (threadIdx.x == 0) go_sm = !over_tau(x.lb);
+              __syncthreads();
+              if (!go_sm) continue;
+              if (s < 32 || s > kRingWords * 2) {
+                if (wid == 0) evaluate<Real>(ex, x.u, x.k);
+                continue;
+              }
+              const R2* __restrict__ trow = ex.trows + ex.trow_off[dur[x.u]];
+              float2* const prs = reinterpret_cast<float2*>(dyn_f);
               double S = 0.0;
               for (int rho = threadIdx.x; rho < s; rho += kChiThreads) prs[rho] = offset_sum(ex.fold, x.k, w, s, rho, trow, S);
               S = warp_sum(S);
-              if (lane == 0) part[wid].S = S;
+              if (lane == 0) part_s[wid] = S;
               __syncthreads();
               if (wid == 0) {
                 float2 acc = make_float2(0.f, 0.f);
                 for (int rho = lane; rho < s; rho += 32) add_pair(acc, prs[rho]);
                 S = 0.0;
-                for (int p = 0; p < kChiWarps; ++p) S += part[p].S;
+                for (int p = 0; p < kChiWarps; ++p) S += part_s[p];
                 settle<Real>(ex, x.u, x.k, Sums<Real>{S, (Real)warp_sum(acc.x), (Real)warp_sum(acc.y)});
               }
             }

@@ -1,0 +1,35 @@
+"""Windows that the CTA sums together: widths around the split (1,024), around
+the samples in shared memory at a time (4,096) and beyond two of those, on a
+curve with dips (their windows overlap) and on one where every start ties
+(windows far apart, many more than are summed together).
+
+Bars: FP64 chi2 within 1e-9 relative of the FP64 oracle, identical locations
+where the minimum is unique, and the same bits with and without neighbours.
+"""
+import numpy as np
+import pytest
+
+import tls_oracle as O
+from test_gpu_bounds import _case, _search
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("n,widths", [
+    (9001, [1024, 1025, 1031, 1409]),
+    (20000, [1025, 2049, 4095, 4096, 4097, 4480]),
+    (26001, [3000, 8191, 8192, 8193, 9000]),
+])
+def test_wide_windows_match_the_oracle(cuda, n, widths, flat):
+    t, y, dy, widths, tm, ov, maxd = _case(n, widths, seed=n, dy=not flat, flat=flat)
+    P = np.array([0.61, 1.7, 3.4])
+    c, l = _search(t, y, dy, widths, tm, ov, P, False, "fp64", 1)
+    c_ref, l_ref = O.search_periods(O.NumpyBackend(), P, t, y, dy, widths, tm, ov, maxd, 1e-5, 8, 1)
+    np.testing.assert_allclose(c, c_ref, rtol=1e-9)
+    if not flat:
+        np.testing.assert_array_equal(l, l_ref)
+    for i, p in enumerate(P):
+        one, lone = _search(t, y, dy, widths, tm, ov, np.array([p]), False, "fp64", 1)
+        assert one[0] == c[i]
+        assert flat or lone[0] == l[i]
