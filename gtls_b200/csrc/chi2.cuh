@@ -19,12 +19,12 @@ constexpr int kTogether = 4;                     // overlapping ones summed toge
 constexpr int kStage = 4096;                     // samples of theirs in shared memory at a time
 constexpr int kProbe = 16;                       // all-starts pass: first sweep over every (width / kProbe)-th start
 constexpr int kList = 4096;                      // starts of a CTA that wait for their sums, main pass
-constexpr int kListAll = 16384;                  // and all-starts pass
+constexpr int kListAll = 8192;                   // and all-starts pass, whose starts come from blocks:
+constexpr int kBlockTable = 24576;               // blocks of a CTA's starts and durations (a multiple of three)
 constexpr int kRedo = 256;                       // tasks of a CTA that found the list full
 constexpr int kBlockStarts = 64;                 // all-starts pass: consecutive starts bounded together from their samples
 constexpr int kBlockSamples = 2048;              // samples of their windows in shared memory at a time
-constexpr int kBlockMinW = 128;                  // for widths from here on
-constexpr int kBlockSlots = 2048;                // blocks of a CTA
+constexpr int kBlockSlots = 2048;                // blocks of a CTA taken up at a time
 
 // Arrays of prefix values are skewed by one word per 32, so that starts a
 // power of two apart fall into different banks.
@@ -67,11 +67,15 @@ struct Waiting {
   int k, u;
 };
 
+// Per CTA: the list, the tasks that found it full, and (all starts) the blocks.
+constexpr int list_entries(bool all) { return (all ? kListAll + kBlockTable / 3 : kList) + kRedo; }
+static_assert(sizeof(Waiting) == 3 * sizeof(int), "");
+
 struct Chi2Args {
   int nruns;
   double depth_min;
   float* vpre;              // rows of the prefix of v (CTAs of curves with a coarse prefix)
-  Waiting* list;            // [chunk CTAs * (kList or kListAll, and kRedo)]
+  Waiting* list;            // [chunk CTAs * list_entries(all)]
   int* tau;                 // [chunk periods] smallest upper bound so far, shared by a period's CTAs
   double* part_v;           // [chunk CTAs]
   long long* part_loc;      // [chunk CTAs]
@@ -383,25 +387,28 @@ __device__ __noinline__ void group_sums(const Exact<double>& x, const int2* whic
 // What bounds the stage: with every passing start summed it was the FMA pipe
 // and the latency of the records' reads (6.0 us a period on a 70,000-sample
 // curve with 66 durations); with the bounds first (screen.cuh) it is issue
-// slots and barriers.
+// slots and barriers (2.7 us).
 //
-//  * The CTA walks its range in batches of 2,560 samples: every thread takes
-//    five folded samples (order, then the (v, w) pair: no records are written
+//  * The CTA walks its range in batches of 2,688 samples: every thread takes
+//    seven folded samples (order, then the (v, w) pair: no records are written
 //    to memory), the block scans v, u, w - wbar and u^2 - qbar, and the prefix
 //    values go into a ring of 4,096 samples in shared memory (and u, w, u^2 at
 //    every g-th sample into a coarse array, and v into a row in memory, for
 //    widths the ring does not hold).
-//  * After each batch the warps screen the 2,560 starts it completes, for every
+//  * After each batch the warps screen the 2,688 starts it completes, for every
 //    duration of the union of at most kRingMaxW samples: the depth test of 128
 //    starts, the passing ones packed 32 to a group, a lower bound each, and
 //    both bounds from more cells for those not ruled out.  The smallest upper
-//    bound so far (tau) rules out most; the rest are listed.  Wider durations
+//    bound so far (tau) rules out most; the rest are listed (all starts: their
+//    blocks are marked, and those bounded again).  Wider durations
 //    follow at the end from the coarse array.
-//  * The listed starts still at or below tau get their exact sums, a warp
-//    each, the most promising first (each result lowers tau).
+//  * The listed starts still at or below tau get their exact sums, a warp each
+//    (windows of more than 1,024 samples the CTA), the most promising first
+//    (each result lowers tau).
 //
-// 512 threads and 113 KB, two CTAs to an SM, so that one's barriers and scans
-// overlap the other's screening.
+// 384 threads of 80 registers and at most 110 KB, two CTAs to an SM, so that one's
+// barriers and scans overlap the other's screening (512 threads of 64
+// registers spill in the screening: 5.9 us).
 template <typename Real, bool kAll>
 __global__ void __launch_bounds__(kChiThreads, 2)
 chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, const int* __restrict__ order,
@@ -465,7 +472,21 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   const ScreenCell* __restrict__ scells = C.scells;
   const int* __restrict__ sends = C.sends;
   constexpr int kCap = kAll ? kListAll : kList;
-  Waiting* const list = a.list + (size_t)cta * (kCap + kRedo);
+  Waiting* const list = a.list + (size_t)cta * list_entries(kAll);
+  // all starts: the smallest lower bound (as float_key) of every block, kBlockStarts
+  // starts of 2^bgroup neighbouring union positions
+  int* const btable = reinterpret_cast<int*>(list + kCap + kRedo);
+  const int nblk = (k1 - k0 + kBlockStarts - 1) / kBlockStarts;
+  int bgroup = 0;
+  if constexpr (kAll)
+    while ((long long)nblk * (((ucnt - 1) >> bgroup) + 1) > kBlockTable) ++bgroup;
+  const int bpos = ((ucnt - 1) >> bgroup) + 1;   // groups of positions
+  constexpr int kNoBlock = 0x7fffffff;
+  auto to_block = [&](int u, int k, float lb) {
+    atomicMin(&btable[(k - k0) / kBlockStarts * bpos + (u >> bgroup)], float_key(lb));
+  };
+  if constexpr (kAll)
+    for (int i = threadIdx.x; i < nblk * bpos; i += kChiThreads) btable[i] = kNoBlock;
   int* const tau_all = a.tau + (R.item0 + local);
   // FP32 exact sums round by up to (w + 8) half ulps of their absolute sum
   auto gamma_of = [&](int w) { return kGammaF + (sizeof(Real) == 4 ? (float)(w + 8) * 1.2e-7f : 0.f); };
@@ -814,7 +835,9 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           if (lane == 0 && ub < *(volatile int*)&tau_key) atomicMin(&tau_key, ub);
           __syncwarp();
           left = __ballot_sync(0xffffffffu, on && (probe ? certain : true) && (!certain || !over_tau(lb)));
-          if (left) {
+          if (kAll && !probe) {
+            if (left >> lane & 1) to_block(u, k, certain ? lb : -INFINITY);
+          } else if (left) {
             int base = 0;
             if (lane == 0) base = atomicAdd(&list_n, __popc(left));
             const int pos = __shfl_sync(0xffffffffu, base, 0) + __popc(left & ((1u << lane) - 1u));
@@ -856,7 +879,10 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         if (lane == 0) {
           if (cert && sb.ub < INFINITY && float_key(sb.ub) < *(volatile int*)&tau_key)
             atomicMin(&tau_key, float_key(sb.ub));
-          if (cert ? !over_tau(sb.lb) : !probe) {
+          if (!(cert ? !over_tau(sb.lb) : !probe)) {
+          } else if (kAll && !probe) {
+            to_block(u, ks, cert ? sb.lb : -INFINITY);
+          } else {
             pos = atomicAdd(&list_n, 1);
             if (pos < kCap) list[pos] = Waiting{cert ? sb.lb : -INFINITY, ks, u};
           }
@@ -951,149 +977,141 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
 
     if (kAll && !probe) {
       // Around a broad peak thousands of neighbouring starts stay (up to 22,000
-      // in one CTA of a 70,000-sample curve, 300 ms of single sums).  They go
-      // together: blocks of 64 consecutive starts of a width are bounded from
-      // their samples themselves, in FP32, so closely that few are left.
-      int* const slot_key = reinterpret_cast<int*>(dyn_f);            // the rings are free by now
-      int* const slot_lb = slot_key + kBlockSlots;
-      short* const blocks = reinterpret_cast<short*>(slot_lb + kBlockSlots);
-      float* const bv = reinterpret_cast<float*>(blocks + kBlockSlots);                       // v, (u, w) and (s, s^2)
+      // in one CTA of a 70,000-sample curve, and on some curves ten times that).
+      // The screening marks their blocks, 64 consecutive starts of a width, in a table
+      // that cannot overflow; a block's starts are bounded together from
+      // their samples themselves, in FP32, so closely that few are left.  (As a
+      // list of starts, of which a full one left all starts of the CTA to be summed, some
+      // curves took 0.1 to 1.5 s for 200 periods.)
+      int* const block_at = reinterpret_cast<int*>(dyn_f);            // the rings are free by now
+      int* const block_lb = block_at + kBlockSlots;
+      float* const bv = reinterpret_cast<float*>(block_lb + kBlockSlots);                     // v, (u, w) and (s, s^2)
       float2* const buw = reinterpret_cast<float2*>(bv + kBlockSamples + kBlockStarts);
       float2* const bt = buw + kBlockSamples + kBlockStarts;
       float* const bpart = bv;                                        // [warp][5][kBlockStarts], after the samples
-      static_assert(kBlockSlots * 10 + (kBlockSamples + kBlockStarts) * 12 + kBlockSamples * 8 <= 4 * 4 * kRingWords, "");
+      static_assert(kBlockSlots * 8 + (kBlockSamples + kBlockStarts) * 12 + kBlockSamples * 8 <= 4 * 4 * kRingWords, "");
       static_assert(kChiWarps * 5 * kBlockStarts <= 3 * (kBlockSamples + kBlockStarts) + 2 * kBlockSamples, "");
-      for (int i = threadIdx.x; i < kBlockSlots; i += kChiThreads) {
-        slot_key[i] = -1;
-        slot_lb[i] = 0x7f800000;
-      }
-      if (threadIdx.x == 0) picked[0] = 0;
-      __syncthreads();
-      const int listed = min(list_n, kCap);
-      for (int i = threadIdx.x; i < listed; i += kChiThreads) {
-        const Waiting x = list[i];
-        if ((int)(wsk[x.u] & 0xffff) < kBlockMinW || x.lb == -INFINITY) continue;   // on its own
-        bool taken = over_tau(x.lb);
-        if (!taken) {
-          const int key = (x.k - k0) / kBlockStarts * GTLS_MAX_DURATIONS + x.u;
-          unsigned h = ((unsigned)key * 2654435761u) >> 21;   // 11 bits: kBlockSlots
-          for (int tries = 0; tries < 64 && !taken; ++tries, h = (h + 1) & (kBlockSlots - 1)) {
-            const int was = atomicCAS(&slot_key[h], -1, key);
-            if (was == -1) blocks[atomicAdd(&picked[0], 1)] = (short)h;
-            if (was == -1 || was == key) {
-              atomicMin(&slot_lb[h], float_key(x.lb));
-              taken = true;
-            }
-          }
+      if (threadIdx.x == 0) list_n = 0;
+      for (bool more = true; more;) {
+        if (threadIdx.x == 0) picked[0] = 0;
+        __syncthreads();
+        float lo = INFINITY;
+        for (int i = threadIdx.x; i < nblk * bpos; i += kChiThreads) {
+          const int key = __ldcg(btable + i);
+          if (key == kNoBlock || over_tau(key_float(key))) continue;
+          const int pos = atomicAdd(&picked[0], 1);
+          if (pos >= kBlockSlots) continue;
+          block_at[pos] = i;
+          block_lb[pos] = key;
+          btable[i] = kNoBlock;
+          if (key_float(key) > -INFINITY) lo = fminf(lo, key_float(key));
         }
-        if (taken) list[i].k = -1;
-      }
-      __syncthreads();
-      const int nblocks = picked[0];
-      float lo = INFINITY;
-      for (int j = threadIdx.x; j < nblocks; j += kChiThreads) lo = fminf(lo, key_float(slot_lb[blocks[j]]));
-      const int low = __reduce_min_sync(0xffffffffu, float_key(lo));
-      if (lane == 0) atomicMin(&low_key, low);
-      if (threadIdx.x == 0) list_n = listed;
-      __syncthreads();
-      const float cut = key_float(low_key) + 0.25f * (key_float(tau_key) - key_float(low_key));
-      __syncthreads();
-      if (threadIdx.x == 0) low_key = 0x7f800000;
-      for (int j = 0; j < 2 * nblocks; ++j) {   // the lowest quarter first, then the others
-        const int h = blocks[j < nblocks ? j : j - nblocks];
-        const float blb = key_float(slot_lb[h]);
-        if ((blb > cut) != (j >= nblocks)) continue;
+        const int low = __reduce_min_sync(0xffffffffu, float_key(lo));
+        if (lane == 0) atomicMin(&low_key, low);
         __syncthreads();
-        if (threadIdx.x == 0) go_sm = !over_tau(blb);
+        more = picked[0] > kBlockSlots;
+        const int nblocks = min(picked[0], kBlockSlots);
+        const float cut = key_float(low_key) + 0.25f * (key_float(tau_key) - key_float(low_key));
         __syncthreads();
-        if (!go_sm) continue;
-        const int u = slot_key[h] % GTLS_MAX_DURATIONS, kb = k0 + slot_key[h] / GTLS_MAX_DURATIONS * kBlockStarts;
-        const int d = dur[u], w = (int)(wsk[u] & 0xffff);
-        const R2* __restrict__ trow = ex.trows + ex.trow_off[d];
-        // lane's starts kb + lane and kb + 32 + lane, each warp a slice of the window
-        float2 bc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        float sv[2] = {0.f, 0.f}, av[2] = {0.f, 0.f}, qu[2] = {0.f, 0.f};
-        for (int c = 0; c < w; c += kBlockSamples) {
-          const int len = min(kBlockSamples, w - c);
-          __syncthreads();
-          {
-            constexpr int kPer = (kBlockSamples + kBlockStarts + kChiThreads - 1) / kChiThreads;
-            int idx[kPer];
+        if (threadIdx.x == 0) low_key = 0x7f800000;
+        for (int j = 0; j < 2 * nblocks; ++j) {   // the lowest quarter first, then the others
+          const int h = j < nblocks ? j : j - nblocks;
+          const float blb = key_float(block_lb[h]);
+          if ((blb > cut) != (j >= nblocks)) continue;
+          const int u0 = block_at[h] % bpos << bgroup, kb = k0 + block_at[h] / bpos * kBlockStarts;
+          for (int u = u0; u < min(ucnt, u0 + (1 << bgroup)); ++u) {
+            __syncthreads();
+            if (threadIdx.x == 0) go_sm = !over_tau(blb);
+            __syncthreads();
+            if (!go_sm) break;
+            const int d = dur[u], w = (int)(wsk[u] & 0xffff);
+            const R2* __restrict__ trow = ex.trows + ex.trow_off[d];
+            // lane's starts kb + lane and kb + 32 + lane, each warp a slice of the window
+            float2 bc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            float sv[2] = {0.f, 0.f}, av[2] = {0.f, 0.f}, qu[2] = {0.f, 0.f};
+            for (int c = 0; c < w; c += kBlockSamples) {
+              const int len = min(kBlockSamples, w - c);
+              __syncthreads();
+              {
+                constexpr int kPer = (kBlockSamples + kBlockStarts + kChiThreads - 1) / kChiThreads;
+                int idx[kPer];
 #pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-              const int i = threadIdx.x + q * kChiThreads;
-              idx[q] = i < len + kBlockStarts ? ex.fold.order[wrap_pos(kb + c + i, n)] : -1;
-            }
+                for (int q = 0; q < kPer; ++q) {
+                  const int i = threadIdx.x + q * kChiThreads;
+                  idx[q] = i < len + kBlockStarts ? ex.fold.order[wrap_pos(kb + c + i, n)] : -1;
+                }
 #pragma unroll
-            for (int q = 0; q < kPer; ++q) {
-              const int i = threadIdx.x + q * kChiThreads;
-              if (idx[q] < 0) continue;
-              const double2 x = ex.fold.vw[min(idx[q], n - 1)];
-              const double v = x.x * cc.vscale;
-              bv[i] = (float)v;
-              buw[i] = make_float2((float)(v * x.y) * (float)cc.wscale, (float)x.y * (float)cc.wscale);
-            }
-          }
-          for (int i = threadIdx.x; i < len; i += kChiThreads) bt[i] = make_float2((float)trow[c + i].x, (float)trow[c + i].y);
-          __syncthreads();
-          const int slice = (len + kChiWarps - 1) / kChiWarps;
-          const int i1 = min(len, (wid + 1) * slice);
+                for (int q = 0; q < kPer; ++q) {
+                  const int i = threadIdx.x + q * kChiThreads;
+                  if (idx[q] < 0) continue;
+                  const double2 x = ex.fold.vw[min(idx[q], n - 1)];
+                  const double v = x.x * cc.vscale;
+                  bv[i] = (float)v;
+                  buw[i] = make_float2((float)(v * x.y) * (float)cc.wscale, (float)x.y * (float)cc.wscale);
+                }
+              }
+              for (int i = threadIdx.x; i < len; i += kChiThreads) bt[i] = make_float2((float)trow[c + i].x, (float)trow[c + i].y);
+              __syncthreads();
+              const int slice = (len + kChiWarps - 1) / kChiWarps;
+              const int i1 = min(len, (wid + 1) * slice);
 #pragma unroll 4
-          for (int i = wid * slice; i < i1; ++i) {
-            const float2 t = bt[i];
+              for (int i = wid * slice; i < i1; ++i) {
+                const float2 t = bt[i];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                  const float2 x = buw[i + lane + 32 * b];
+                  const float v = bv[i + lane + 32 * b];
+                  fma_pair(t, x, bc[b]);
+                  qu[b] = fmaf(x.x, x.x, qu[b]);
+                  sv[b] += v;
+                  av[b] += fabsf(v);
+                }
+              }
+            }
+            __syncthreads();
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
-              const float2 x = buw[i + lane + 32 * b];
-              const float v = bv[i + lane + 32 * b];
-              fma_pair(t, x, bc[b]);
-              qu[b] = fmaf(x.x, x.x, qu[b]);
-              sv[b] += v;
-              av[b] += fabsf(v);
+              float* const to = bpart + wid * 5 * kBlockStarts + lane + 32 * b;
+              to[0] = bc[b].x;
+              to[kBlockStarts] = bc[b].y;
+              to[2 * kBlockStarts] = qu[b];
+              to[3 * kBlockStarts] = sv[b];
+              to[4 * kBlockStarts] = av[b];
+            }
+            __syncthreads();
+            if (threadIdx.x < kBlockStarts) {   // two whole warps
+              float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+              for (int p = 0; p < kChiWarps; ++p)
+#pragma unroll
+                for (int f = 0; f < 5; ++f) x[f] += bpart[(p * 5 + f) * kBlockStarts + threadIdx.x];
+              const int k = kb + (int)threadIdx.x;
+              // a sum of at most (w / kBlockSamples + 1) * 171 terms per warp, then of the warps
+              const float roundf = (float)((w / kBlockSamples + 1) * (kBlockSamples / kChiWarps + 1) + kChiWarps + 8) * 1.2e-7f;
+              ScreenRow row = srows[2 * d];
+              row.asum = row.smn = row.smx = row.lmn = row.lmx = 0.f;
+              CellSums cs;
+              cs.B = x[0];
+              cs.cl = cs.cu = x[1];
+              const float m = -x[3] * row.inv_w;
+              const float em = (roundf * x[4]) * row.inv_w + 4e-7f * fabsf(m) + 2e-7f * fabsf(dthr);
+              const StartBounds sb = start_bounds<true>(cs, row, m, em, x[2] * (1.f + 2.f * roundf), 0.f, false,
+                                                        gamma_of(w) + roundf, ScreenErr{0.f, 0.f, 0.f, 0.f});
+              const bool mine = k < k1 && !(m + em <= dthr), certain = m - em > dthr;
+              if (mine && certain && sb.ub < INFINITY) atomicMin(&tau_key, float_key(sb.ub));
+              __syncwarp();
+              const bool stays = mine && (!certain || !over_tau(sb.lb));
+              int pos = 0;
+              if (stays) {
+                pos = atomicAdd(&list_n, 1);
+                if (pos < kCap) list[pos] = Waiting{certain ? sb.lb : -INFINITY, k, u};
+              }
+              unsigned over = __ballot_sync(0xffffffffu, stays && pos >= kCap);
+              for (; over; over &= over - 1) evaluate<Real>(ex, u, __shfl_sync(0xffffffffu, k, __ffs(over) - 1));
             }
           }
         }
         __syncthreads();
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          float* const to = bpart + wid * 5 * kBlockStarts + lane + 32 * b;
-          to[0] = bc[b].x;
-          to[kBlockStarts] = bc[b].y;
-          to[2 * kBlockStarts] = qu[b];
-          to[3 * kBlockStarts] = sv[b];
-          to[4 * kBlockStarts] = av[b];
-        }
-        __syncthreads();
-        if (threadIdx.x < kBlockStarts) {   // two whole warps
-          float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-          for (int p = 0; p < kChiWarps; ++p)
-#pragma unroll
-            for (int f = 0; f < 5; ++f) x[f] += bpart[(p * 5 + f) * kBlockStarts + threadIdx.x];
-          const int k = kb + (int)threadIdx.x;
-          // a sum of at most (w / kBlockSamples + 1) * 171 terms per warp, then of the warps
-          const float roundf = (float)((w / kBlockSamples + 1) * (kBlockSamples / kChiWarps + 1) + kChiWarps + 8) * 1.2e-7f;
-          ScreenRow row = srows[2 * d];
-          row.asum = row.smn = row.smx = row.lmn = row.lmx = 0.f;
-          CellSums cs;
-          cs.B = x[0];
-          cs.cl = cs.cu = x[1];
-          const float m = -x[3] * row.inv_w;
-          const float em = (roundf * x[4]) * row.inv_w + 4e-7f * fabsf(m) + 2e-7f * fabsf(dthr);
-          const StartBounds sb = start_bounds<true>(cs, row, m, em, x[2] * (1.f + 2.f * roundf), 0.f, false,
-                                                    gamma_of(w) + roundf, ScreenErr{0.f, 0.f, 0.f, 0.f});
-          const bool mine = k < k1 && !(m + em <= dthr), certain = m - em > dthr;
-          if (mine && certain && sb.ub < INFINITY) atomicMin(&tau_key, float_key(sb.ub));
-          __syncwarp();
-          const bool stays = mine && (!certain || !over_tau(sb.lb));
-          int pos = 0;
-          if (stays) {
-            pos = atomicAdd(&list_n, 1);
-            if (pos < kCap) list[pos] = Waiting{certain ? sb.lb : -INFINITY, k, u};
-          }
-          unsigned over = __ballot_sync(0xffffffffu, stays && pos >= kCap);
-          for (; over; over &= over - 1) evaluate<Real>(ex, u, __shfl_sync(0xffffffffu, k, __ffs(over) - 1));
-        }
       }
-      __syncthreads();
     }
     // the listed starts that can still be the minimum, the most promising first:
     // those of the lowest quarter between the smallest lower bound and tau;
@@ -1236,7 +1254,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           }
         }
       }
-    if (!probe && redo_n > 0) {   // the list was full: every start of the tasks that found it so (of all, if those are too many)
+    if (!kAll && redo_n > 0) {   // the list was full: every start of the tasks that found it so (of all, if those are too many)
       const bool every = redo_n > kRedo;
       for (int t = 0; t < (every ? ucnt : redo_n); ++t) {
         const int u = every ? t : list[kCap + t].u;

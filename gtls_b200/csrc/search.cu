@@ -1135,7 +1135,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
                       double depth_min, int flags, gtls_timing* tm, cudaStream_t st) {
   using R2 = typename Tr<Real>::R2;
   const bool all = precision_pass == GTLS_PASS_ALL;
-  const size_t list_cap = (all ? kListAll : kList) + kRedo;
+  const size_t list_cap = list_entries(all);
   bool& allowed = sizeof(Real) == 8 ? ctx->smem_set_fp64 : ctx->smem_set_fp32;
   if (!allowed) {
     GTLS_TRY_CUDA(ctx, allow_smem<Real>(ctx->smem_optin));

@@ -33,3 +33,19 @@ def test_wide_windows_match_the_oracle(cuda, n, widths, flat):
         one, lone = _search(t, y, dy, widths, tm, ov, np.array([p]), False, "fp64", 1)
         assert one[0] == c[i]
         assert flat or lone[0] == l[i]
+
+
+@pytest.mark.parametrize("flat", [False, True])
+@pytest.mark.parametrize("n,durations", [(8300, 190), (8300, 200), (3000, 64)])
+def test_blocks_of_all_starts_match_the_oracle(cuda, n, durations, flat):
+    """All starts of 64 to 200 durations: blocks of one and of two durations
+    (the table holds 192 of 128 blocks), and with every start tying more blocks
+    than are taken up at a time."""
+    t, y, dy, widths, tm, ov, maxd = _case(n, list(range(9, 9 + durations)), seed=n, dy=not flat, flat=flat)
+    P = np.array([1.7])
+    c_ref, l_ref = O.search_periods(O.NumpyBackend(), P, t, y, dy, widths, tm, ov, maxd, 1e-5, 8, 1, noskip=True)
+    for precision, rtol in (("fp64", 1e-9), ("fp32", 2e-6)):
+        c, l = _search(t, y, dy, widths, tm, ov, P, True, precision, 1)
+        np.testing.assert_allclose(c, c_ref, rtol=rtol)
+        if precision == "fp64" and not flat:
+            np.testing.assert_array_equal(l, l_ref)
