@@ -222,9 +222,11 @@ def pipe_object(timings, chi2_ms, precision):
     ``dense``: every evaluated (start, template sample), whether or not the
     start's window passes the depth test; ``active``: the starts that pass it,
     the only sums that enter the result (the reference's kernel runs its
-    in-transit loop for these alone, GPUFun.py:409-424); ``issued``: what the
-    kernel executed (register groups of consecutive starts covering the
-    passing ones, padded template blocks)."""
+    in-transit loop for these alone, GPUFun.py:409-424); ``issued``: the
+    multiply-adds of the starts whose exact sums the kernel forms.  It rules the others
+    out by bounds from prefix sums, whose arithmetic is not counted, so
+    ``issued`` is a small part of ``active`` and its share of the pipe says
+    little about the kernel's speed."""
     peak = 148 * (64 if precision == "fp64" else 128) * 2 * 1.965e9 / 1e12
     sec = chi2_ms * 1e-3
     out = {"unit": "TFLOP/s", "fp_pipe": "fp64" if precision == "fp64" else "fp32", "nominal_peak": peak,

@@ -1,9 +1,9 @@
-// The arithmetic core of the chi2 kernel: record/template pair types and the
-// register-blocked correlations of a template row with the folded records
-// (B and C sums of kR consecutive starts).  Host-callable as well, so that
-// the summation orders can be checked on the CPU (the device build uses the
-// packed two-lane FP32 instructions, the host build two scalar FMAs with the
-// same IEEE rounding).
+// Record and template pair types of the chi2 kernel, and the summation orders
+// of a start's sums written as register-blocked correlations of a template row
+// with the folded records.  The kernel sums single starts in those orders
+// (chi2.cuh); the correlations are the host-callable statement of them that the
+// CPU checks run (the device build uses the packed two-lane FP32 instructions,
+// the host build two scalar FMAs with the same IEEE rounding).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -17,12 +17,9 @@ constexpr int kR = 9;            // starts per register block (odd: conflict-fre
 template <typename Real> struct Tr;
 template <> struct Tr<double> {
   using R2 = double2;   // (u, w) record / (s, s^2) template pair
-  using Pv = double;    // prefix of v
 };
-static_assert(sizeof(float2) == sizeof(double), "float-float prefix shares the FP64 slot");
 template <> struct Tr<float> {
   using R2 = float2;
-  using Pv = float2;    // (hi, lo) float-float prefix of v
 };
 
 // (b, c) += (t.x * x.x, t.y * x.y) for an accumulator pair (B, C): one
@@ -60,99 +57,12 @@ __host__ __device__ __forceinline__ R2 zero_pair() {
   return z;
 }
 
-// Correlate template offset rho of kR consecutive starts with the tile:
-//   acc[r].x (B) += sum_{q<Q} T[q*s + rho] * u[base + (r+q)*s],  acc[r].y (C) likewise with (T^2, w)
-// where base = jb*s + rho - k0 addresses start block jb.  A sliding window of
-// kR records in registers gives one shared-memory load and one template load
-// per kR multiply-add pairs (slot of record q+r is (q+r) % kR; the q loop is
-// unrolled by kR so every slot index is a constant).  Template rows are zero
-// at and beyond w.  Loads past the tile are clamped to its last record: for a
-// start inside the tile they only meet those zero template entries, and the
-// sums of starts past the tile are discarded.
-template <typename Real, bool kTwoLevel>
-__host__ __device__ __forceinline__ void correlate(const typename Tr<Real>::R2* __restrict__ tile, int L, int base, int s,
-                                          const typename Tr<Real>::R2* __restrict__ trow, int rho, int Q,
-                                          typename Tr<Real>::R2 (&acc)[kR]) {
-  using R2 = typename Tr<Real>::R2;
-  R2 xs[kR];
-  const int last = L - 1;
-#pragma unroll
-  for (int i = 0; i < kR - 1; ++i) xs[i] = tile[min(base + i * s, last)];
-  R2 pr[kR];
-#pragma unroll
-  for (int r = 0; r < kR; ++r) pr[r] = kTwoLevel ? zero_pair<R2>() : acc[r];
-  int pos = base + (kR - 1) * s;
-  int toff = rho;
-  R2 tnext = trow[toff];
-  for (int q0 = 0; q0 < Q; q0 += kR) {
-#pragma unroll
-    for (int qq = 0; qq < kR; ++qq) {
-      if (q0 + qq >= Q) break;
-      xs[(qq + kR - 1) % kR] = tile[min(pos, last)];
-      const R2 tq = tnext;
-      pos += s;
-      toff += s;
-      tnext = trow[toff];   // next template entry (rows carry one zero block past Q)
-#pragma unroll
-      for (int r = 0; r < kR; ++r) {
-        const R2 x = xs[(qq + r) % kR];
-        fma_pair(tq, x, pr[r]);
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < kR; ++r) {
-    if (kTwoLevel)
-      add_pair(acc[r], pr[r]);
-    else
-      acc[r] = pr[r];
-  }
-}
-
-// correlate() for skip 1 (every start: the all-starts pass and widths up to
-// the skip point) and a group whose kR starts all lie in the tile: no
-// clamping (the reads stay inside the tile and its zeroed pad), whole blocks
-// of kR template entries (entries past Q are zero), consecutive records and
-// template entries addressed with constant offsets from block pointers.  The
-// sums are formed in exactly the order of correlate() with skip 1 (entries
-// past Q add exact zeros), so a start's value does not depend on which of
-// the two paths the tile boundaries send it through.
-template <typename Real, bool kTwoLevel>
-__host__ __device__ __forceinline__ void correlate_s1(const typename Tr<Real>::R2* __restrict__ tile, int base,
-                                             const typename Tr<Real>::R2* __restrict__ trow, int Qr,
-                                             typename Tr<Real>::R2 (&acc)[kR]) {
-  using R2 = typename Tr<Real>::R2;
-  R2 xs[kR];
-  const R2* xp = tile + base;
-#pragma unroll
-  for (int i = 0; i < kR - 1; ++i) xs[i] = xp[i];
-  R2 pr[kR];
-#pragma unroll
-  for (int r = 0; r < kR; ++r) pr[r] = kTwoLevel ? zero_pair<R2>() : acc[r];
-  for (int q0 = 0; q0 < Qr; q0 += kR) {
-    const R2* xb = xp + q0 + kR - 1;
-    const R2* tb = trow + q0;
-#pragma unroll
-    for (int qq = 0; qq < kR; ++qq) {
-      xs[(qq + kR - 1) % kR] = xb[qq];
-      const R2 tq = tb[qq];
-#pragma unroll
-      for (int r = 0; r < kR; ++r) fma_pair(tq, xs[(qq + r) % kR], pr[r]);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < kR; ++r) {
-    if (kTwoLevel)
-      add_pair(acc[r], pr[r]);
-    else
-      acc[r] = pr[r];
-  }
-}
-
-// Same sums for the lanes-split path: the kR template entries of one block of
-// kR template offsets are loaded together first (kR loads in flight), then the
-// 2*kR-1 records they touch stream through once.  kClamp: clamp record reads
-// to the tile (needed only for tasks whose reads may pass its end).
+// Correlate template offset rho of kR consecutive starts with the records:
+//   acc[r].x (B) += sum_{q<Q} T[q*s + rho] * u[base + (r+q)*s],  acc[r].y (C) likewise with (T^2, w).
+// The kR template entries of one block of kR template offsets are loaded
+// together first, then the 2*kR-1 records they touch stream through once.
+// kClamp: clamp record reads to the records' end (needed only where reads may
+// pass it: they meet zero template entries).
 template <typename Real, bool kTwoLevel, bool kClamp>
 __host__ __device__ __forceinline__ void correlate_pre(const typename Tr<Real>::R2* __restrict__ tile, int L, int base,
                                               int s, const typename Tr<Real>::R2* __restrict__ trow, int rho,

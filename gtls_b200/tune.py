@@ -1,16 +1,14 @@
 """Autotuning of the search's launch shapes on the caller's own data.
 
-The tile of starts per chi2 CTA, where the chi2 kernel reads the folded
-records from (a shared-memory tile, or global memory through a large L1),
-and the number of phase buckets of the global-scatter fold ordering change
-only the time of a search, never its result (every chi2 value and argmin
-location is the same; ``tests/test_gpu_tune.py``).  Which setting is fastest
-depends on the curves: the tile against the longest duration (halo re-reads
-versus work per CTA; in the FP64 form on a 70,000-sample, 8,400-width curve
-the records read through L1, in tiles of 10,240 starts, beat the staged tile
-by 7.5%), the bucket count against how clustered the folded phases are (it
-matters only for curves above 2^17 samples, which take the global-scatter
-ordering).  ``autotune`` times the main pass of a sample of the trial
+The largest range of starts of a chi2 CTA and the number of phase buckets of
+the global-scatter fold ordering change only the time of a search, never its
+result (every chi2 value and argmin location is the same;
+``tests/test_gpu_tune.py``).  At the default caps the library splits the starts by its own
+rule, from the samples and the longest duration; another cap is taken as it
+is: larger ranges read fewer samples twice, smaller ones make more CTAs.  The
+bucket count matters only for curves of 2^20 samples and more, which take the
+global-scatter ordering.  ``records_global`` has no effect any more and is kept for
+callers that set it.  ``autotune`` times the main pass of a sample of the trial
 periods under each candidate setting, with the library's own CUDA-event
 stage timing, and keeps the fastest for the context (``gtls_set_tuning``).
 Results are cached per (precision, samples rounded to a power of two,
@@ -25,7 +23,7 @@ from . import _lib
 TILE_CAPS = {"fp32": (8192, 12288, 16384, 24576), "fp64": (4096, 8192, 10240, 12288)}
 BUCKET_SHIFTS = (0, -1)
 RECORDS_GLOBAL = (0, 1)
-PACKED_MAX_N = 1 << 17   # curves up to this many samples order their phases in shared memory
+PACKED_MAX_N = 1 << 17   # longer curves try the bucket counts too
 DEFAULT_CAP = {"fp32": 16384, "fp64": 8192}
 MARGIN = 0.02   # a setting must beat the default by this fraction to be chosen
 _CACHE = {}
@@ -36,7 +34,7 @@ def _key(precision, n, maxd):
 
 
 def autotune(run_main_pass, precision, n, maxd, device=0, repeats=2):
-    """Pick the fastest (tile cap, records mode, bucket shift) for ``precision``.
+    """Pick the fastest (tile cap, ``records_global``, bucket shift) for ``precision``.
 
     ``run_main_pass(timing)`` runs the main pass of a representative sample
     of periods and fills the ``_lib.Timing`` it is given.  Returns the chosen

@@ -90,8 +90,8 @@ typedef struct gtls_tuning {
                                  [256, 65536]; 0, or 16384 = the library's own split (by the
                                  curve's samples and longest duration)                       */
   int32_t tile_cap_fp64;      /* the same for the FP64 form; 0, or 8192 = the library's own split */
-  int32_t bucket_shift;       /* phase buckets of the global-scatter fold ordering (curves above
-                                 2^17 samples, and periods whose phases cluster beyond what the
+  int32_t bucket_shift;       /* phase buckets of the global-scatter fold ordering (curves of
+                                 2^20 samples and more, and periods whose phases cluster beyond what the
                                  shared-memory ordering holds) = 2^min(15, ceil(log2 N) + shift),
                                  shift in [-3, 0] (0 = default)                               */
   int32_t records_global;     /* 0 or 1, kept for callers: the folded records are read through L2
