@@ -683,7 +683,7 @@ def bench_cfg3(args):
     """cfg3: the mixed-precision form over 64 seeded cfg1-shaped curves.
 
     Every curve is searched with the FP32-compensated main pass (precision
-    "fp32": FP32 chi2 and template sums, float-float prefix sums, FP64 fold,
+    "fp32": FP32 chi2 and template sums, FP64 window means, FP64 fold,
     FP64 re-search of the 200 candidates and 5 harmonics) and with the plain
     FP64 form, whose chi2 matches the FP64 oracle within 1e-9 relative (the
     GPU parity tests).  Reports throughput of both and the FP32 form's error

@@ -10,8 +10,8 @@ The per-curve steps between the passes (outlier mask, spectra, candidate
 choice) and the host statistics of the best period stay per curve.
 
 The reference has no batched form; it searches one curve per ``gtls``
-object.  ``precision`` defaults to "fp32" here (FP32 chi2 with float-float
-prefix sums in the main pass and the candidate re-search, then an FP64
+object.  ``precision`` defaults to "fp32" here (FP32 chi2 with FP64
+window means in the main pass and the candidate re-search, then an FP64
 re-check of each curve's best 32 candidates; harmonics and the best period in
 FP64).
 """

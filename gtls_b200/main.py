@@ -9,7 +9,7 @@ batch-aligned period ranges, one host thread per device; every chi2 value is
 the unsharded one), and runs the rest on the first of them.  ``distributed``
 (below) does the same with one process per GPU started by torchrun.
 Extra keywords: ``precision`` ("fp64" plain FP64 search, default; "fp32" FP32
-chi2 with float-float prefix sums in the main pass and the candidate
+chi2 with FP64 window means in the main pass and the candidate
 re-search, then an FP64 re-check of the 32 best candidates),
 ``batch_periods`` (periods per duration-union batch; default: the reference's
 free-memory formula, core.py:620-628), ``distributed`` (shard the main pass
