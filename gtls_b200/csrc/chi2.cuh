@@ -1082,6 +1082,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
               to[4 * kBlockStarts] = av[b];
             }
             __syncthreads();
+            bool stays = false;
             if (threadIdx.x < kBlockStarts) {   // two whole warps
               float x[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
               for (int p = 0; p < kChiWarps; ++p)
@@ -1102,14 +1103,67 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
               const bool mine = k < k1 && !(m + em <= dthr), certain = m - em > dthr;
               if (mine && certain && sb.ub < INFINITY) atomicMin(&tau_key, float_key(sb.ub));
               __syncwarp();
-              const bool stays = mine && (!certain || !over_tau(sb.lb));
-              int pos = 0;
-              if (stays) {
-                pos = atomicAdd(&list_n, 1);
-                if (pos < kCap) list[pos] = Waiting{certain ? sb.lb : -INFINITY, k, u};
+              stays = mine && (!certain || !over_tau(sb.lb));
+              if constexpr (sizeof(Real) == 8) {
+                int pos = 0;
+                if (stays) {
+                  pos = atomicAdd(&list_n, 1);
+                  if (pos < kCap) list[pos] = Waiting{certain ? sb.lb : -INFINITY, k, u};
+                }
+                unsigned over = __ballot_sync(0xffffffffu, stays && pos >= kCap);
+                for (; over; over &= over - 1) evaluate<Real>(ex, u, __shfl_sync(0xffffffffu, k, __ffs(over) - 1));
               }
-              unsigned over = __ballot_sync(0xffffffffu, stays && pos >= kCap);
-              for (; over; over &= over - 1) evaluate<Real>(ex, u, __shfl_sync(0xffffffffu, k, __ffs(over) - 1));
+            }
+            if constexpr (sizeof(Real) == 4) {
+              // FP32 bounds carry the chains' own rounding, 0.3% at 24,000 samples, and
+              // whole blocks stay (15 s for 161 periods of 163,000 samples when
+              // they went through the list): their chains run here,
+              // a lane each, over the samples in shared memory.
+              if (!__syncthreads_or(stays)) continue;
+              double* const cv = reinterpret_cast<double*>(bv);
+              float2* const cuw = reinterpret_cast<float2*>(cv + kBlockSamples + kBlockStarts);
+              float2* const ct = cuw + kBlockSamples + kBlockStarts;
+              static_assert(kBlockSlots * 8 + (kBlockSamples + kBlockStarts) * 16 + kBlockSamples * 8 <= 4 * 4 * kRingWords, "");
+              double S = 0.0;
+              float2 pr = make_float2(0.f, 0.f);
+              for (int c = 0; c < w; c += kBlockSamples) {
+                const int len = min(kBlockSamples, w - c);
+                __syncthreads();
+#pragma unroll 6
+                for (int i = threadIdx.x; i < len + kBlockStarts; i += kChiThreads) {
+                  const double2 x = folded_at(ex.fold, kb + c + i);
+                  cv[i] = x.x;
+                  cuw[i] = record_of(x, 0.f);
+                }
+                for (int i = threadIdx.x; i < len; i += kChiThreads) ct[i] = make_float2((float)trow[c + i].x, (float)trow[c + i].y);
+                __syncthreads();
+                if (threadIdx.x < kBlockStarts) {
+#pragma unroll 8
+                  for (int i = 0; i < len; ++i) {
+                    S += cv[i + threadIdx.x];
+                    fma_pair(ct[i], cuw[i + threadIdx.x], pr);
+                  }
+                }
+              }
+              if (threadIdx.x < kBlockStarts) {
+                Best best = red[wid];
+                __syncwarp();
+                if (stays) {
+                  const float inv_w = 1.f / (float)w;
+                  const int k = kb + (int)threadIdx.x;
+                  const double delta = eval_mean<float>(best, -(float)S * inv_w, (float)ex.overshoot[d], pr.x, pr.y, 1,
+                                                        a.depth_min, cc.ebase, (double)n, (long long)u * n + k);
+                  if (delta < INFINITY) atomicMin(&tau_key, float_key(__double2float_ru(delta * cc.dscale)));
+                  if (a.work) atomicAdd(&work_sm[1], 2ULL * (unsigned)w);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                  const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
+                  const long long l = __shfl_xor_sync(0xffffffffu, best.loc, o);
+                  best_update(best, v, l);
+                }
+                if (lane == 0) red[wid] = best;
+              }
             }
           }
         }

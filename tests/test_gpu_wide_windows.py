@@ -20,18 +20,21 @@ pytestmark = pytest.mark.gpu
     (9001, [1024, 1025, 1031, 1409]),
     (20000, [1025, 2049, 4095, 4096, 4097, 4480]),
     (26001, [3000, 8191, 8192, 8193, 9000]),
+    (28500, [4095, 4096, 4097, 4200]),      # all of them valid at P = 0.61: at most 0.15 n
+    (56001, [8191, 8192, 8193]),
 ])
 def test_wide_windows_match_the_oracle(cuda, n, widths, flat):
     t, y, dy, widths, tm, ov, maxd = _case(n, widths, seed=n, dy=not flat, flat=flat)
     P = np.array([0.61, 1.7, 3.4])
     c, l = _search(t, y, dy, widths, tm, ov, P, False, "fp64", 1)
     c_ref, l_ref = O.search_periods(O.NumpyBackend(), P, t, y, dy, widths, tm, ov, maxd, 1e-5, 8, 1)
+    assert np.isfinite(c[0])
     np.testing.assert_allclose(c, c_ref, rtol=1e-9)
     if not flat:
         np.testing.assert_array_equal(l, l_ref)
     for i, p in enumerate(P):
         one, lone = _search(t, y, dy, widths, tm, ov, np.array([p]), False, "fp64", 1)
-        assert one[0] == c[i]
+        assert one[0] == c[i] or np.isnan([one[0], c[i]]).all()   # no valid duration: NaN
         assert flat or lone[0] == l[i]
 
 
@@ -49,3 +52,17 @@ def test_blocks_of_all_starts_match_the_oracle(cuda, n, durations, flat):
         np.testing.assert_allclose(c, c_ref, rtol=rtol)
         if precision == "fp64" and not flat:
             np.testing.assert_array_equal(l, l_ref)
+
+
+@pytest.mark.parametrize("n,widths", [(14500, [2047, 2048, 2049]), (28500, [2000, 4095, 4097, 4200])])
+def test_wide_chains_of_all_starts_match_the_oracle(cuda, n, widths):
+    """FP32, every start: the blocks' chains over samples in shared memory
+    (2,048 at a time), and the same bits with and without neighbours."""
+    t, y, dy, widths, tm, ov, maxd = _case(n, widths, seed=n)
+    P = np.array([0.61, 0.7])
+    c, _ = _search(t, y, dy, widths, tm, ov, P, True, "fp32", 1)
+    c_ref, _ = O.search_periods(O.NumpyBackend(), P, t, y, dy, widths, tm, ov, maxd, 1e-5, 8, 1, noskip=True)
+    assert np.isfinite(c).all()
+    np.testing.assert_allclose(c, c_ref, rtol=2e-6)
+    for i, p in enumerate(P):
+        assert _search(t, y, dy, widths, tm, ov, np.array([p]), True, "fp32", 1)[0][0] == c[i]
