@@ -1100,7 +1100,9 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
               const float em = (roundf * x[4]) * row.inv_w + 4e-7f * fabsf(m) + 2e-7f * fabsf(dthr);
               const StartBounds sb = start_bounds<true>(cs, row, m, em, x[2] * (1.f + 2.f * roundf), 0.f, false,
                                                         gamma_of(w) + roundf, ScreenErr{0.f, 0.f, 0.f, 0.f});
-              const bool mine = k < k1 && !(m + em <= dthr), certain = m - em > dthr;
+              // (a start that only its samples settle carries n like those that the screening settles)
+              const bool fails = m + em <= dthr, mine = k < k1 && !fails, certain = m - em > dthr;
+              if (k < k1 && fails) atomicMin(&sent_sm, (long long)u * n + k);
               if (mine && certain && sb.ub < INFINITY) atomicMin(&tau_key, float_key(sb.ub));
               __syncwarp();
               stays = mine && (!certain || !over_tau(sb.lb));
