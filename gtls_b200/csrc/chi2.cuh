@@ -482,8 +482,8 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     while ((long long)nblk * (((ucnt - 1) >> bgroup) + 1) > kBlockTable) ++bgroup;
   const int bpos = ((ucnt - 1) >> bgroup) + 1;   // groups of positions
   constexpr int kNoBlock = 0x7fffffff;
-  auto to_block = [&](int u, int k, float lb) {
-    atomicMin(&btable[(k - k0) / kBlockStarts * bpos + (u >> bgroup)], float_key(lb));
+  auto to_block = [&](int u, int k, float lb) {   // a NaN's key may be the empty block's
+    atomicMin(&btable[(k - k0) / kBlockStarts * bpos + (u >> bgroup)], float_key(lb == lb ? lb : -INFINITY));
   };
   if constexpr (kAll)
     for (int i = threadIdx.x; i < nblk * bpos; i += kChiThreads) btable[i] = kNoBlock;
@@ -597,7 +597,6 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const int cnt = fetched;
     const int q0 = ld + (int)threadIdx.x * kItems;   // item i is prefix value q0 + i + 1
     const int have = min(kItems, cnt - (int)threadIdx.x * kItems);
-    const float wscale = (float)cc.wscale;
     const int* __restrict__ ord = ex.fold.order;
     const double2* __restrict__ vw = ex.fold.vw;
     if (k0 + q0 + kBatch < n)   // the next batch's indices: into L2
@@ -607,8 +606,9 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       v[i] = gq[i].x * cc.vscale;
-      const float wf = (float)gq[i].y * wscale;
-      uu[i] = (float)(v[i] * gq[i].y) * wscale;
+      const double w = gq[i].y * cc.wscale;   // scaled in FP64: a weight itself may be beyond FP32
+      const float wf = (float)w;
+      uu[i] = (float)(v[i] * w);
       ww[i] = i < have ? wf - cc.wbar : 0.f;
       sv += v[i];
       su += uu[i];
@@ -1048,9 +1048,9 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
                   const int i = threadIdx.x + q * kChiThreads;
                   if (idx[q] < 0) continue;
                   const double2 x = ex.fold.vw[min(idx[q], n - 1)];
-                  const double v = x.x * cc.vscale;
+                  const double v = x.x * cc.vscale, sw = x.y * cc.wscale;
                   bv[i] = (float)v;
-                  buw[i] = make_float2((float)(v * x.y) * (float)cc.wscale, (float)x.y * (float)cc.wscale);
+                  buw[i] = make_float2((float)(v * sw), (float)sw);
                 }
               }
               for (int i = threadIdx.x; i < len; i += kChiThreads) bt[i] = make_float2((float)trow[c + i].x, (float)trow[c + i].y);

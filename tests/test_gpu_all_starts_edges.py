@@ -3,8 +3,10 @@
 * A start whose window mean lies within the screening's rounding of the depth
   threshold is decided by its block of samples; where it fails there it still
   carries the value n (GPUFun.py:407,437).
+* Uncertainties far from one: the weights alone are beyond FP32.
 
-Bars: the value n exactly, and the location of the only start that has it.
+Bars: the value n exactly, and the location of the only start that has it;
+chi2 times a power of two exactly, and the same locations.
 """
 import numpy as np
 import pytest
@@ -47,3 +49,23 @@ def test_a_start_just_below_the_threshold_has_the_value_n(cuda, at, precision):
     c, l = _search(t, y, np.full(n, 0.0101 / 10.0), [1, 2, 3], 1000.0, _lib.GTLS_PASS_ALL, precision)
     assert c[0] == n
     assert l[0] == at
+
+
+@pytest.mark.parametrize("bits", [73, -70])
+@pytest.mark.parametrize("pass_", ["GTLS_PASS_MAIN", "GTLS_PASS_ALL"])
+def test_scaled_uncertainties_scale_chi2(cuda, pass_, bits):
+    """dy divided by 2^bits multiplies every weight, and so E and every delta,
+    by 4^bits without a rounding (weights of 1e50 and 1e-36).  Every start passes
+    the depth test and none is skipped, so that n is no candidate.  (The first
+    sweep of the all-starts pass looks at every second start and more.)"""
+    from gtls_b200 import _lib
+    n = 9000
+    rng = np.random.default_rng(5)
+    t = 1.0 + np.arange(n) * 1e-3
+    sigma = rng.uniform(0.5e-3, 1.5e-3, n)
+    y = 1.0 - 0.05 + sigma * rng.standard_normal(n)
+    args = ([35, 60, 101], np.array([0.7, 1000.0]), getattr(_lib, pass_), "fp64", 200)
+    c0, l0 = _search(t, y, sigma, *args)
+    c1, l1 = _search(t, y, sigma * 2.0 ** -bits, *args)
+    np.testing.assert_array_equal(c1, c0 * 4.0 ** bits)
+    np.testing.assert_array_equal(l1, l0)
