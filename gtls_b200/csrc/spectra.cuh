@@ -27,10 +27,11 @@ int spectra_launch(const double* chi2, const uint8_t* mask, long long n, int k, 
                    double* power, SpecScratch s, cudaStream_t st);
 
 // Window of the running median for an oversampling factor: 30 times it, made
-// odd (stats.py:108-112); 0 when that is no whole number of at least 1.
+// odd (stats.py:108-112); 0 when that is no whole number of at least 1.  (Up to
+// 4e18, so that twice the window is still a 64-bit number.)
 inline long long spectra_window(double oversampling_factor) {
   const double kd = oversampling_factor * 30;
-  if (!(kd >= 1 && kd <= 1e15) || kd != (double)(long long)kd) return 0;
+  if (!(kd >= 1 && kd <= 4e18) || kd != (double)(long long)kd) return 0;
   const long long k = (long long)kd;
   return k + 1 - k % 2;
 }
