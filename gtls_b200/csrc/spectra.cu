@@ -72,9 +72,9 @@ __global__ void __launch_bounds__(kSpecThreads) spec_min_kernel(const double* __
 }
 
 // 2: SR = min / chi2 and its sum
-__global__ void __launch_bounds__(kSpecThreads) spec_sr_kernel(const double* __restrict__ chi2,
+__global__ void __launch_bounds__(kSpecThreads) spec_sr_kernel(const double* chi2,
                                                                const uint8_t* __restrict__ mask, long long n,
-                                                               double* __restrict__ sr, SpecScratch s) {
+                                                               double* sr, SpecScratch s) {
   __shared__ double sh[32];
   const double mn = reduce_parts(s.part, gridDim.x, INFINITY, OpMin(), sh);
   double sum = 0;
@@ -121,10 +121,10 @@ __device__ double raw_scale(const SpecScratch& s, int parts, double* sde_raw, do
   return *sde_raw / mx;
 }
 
-// 4: raw power, for spectra too short for a running median or with a window too wide for the tiles of spec_median_kernel
-__global__ void __launch_bounds__(kSpecThreads) spec_raw_kernel(const double* __restrict__ sr, long long n,
-                                                                double* __restrict__ praw, double* __restrict__ power,
-                                                                SpecScratch s) {
+// 4: raw power, for spectra too short for a running median, with a window too
+// wide for the tiles of spec_median_kernel, or with outputs that share an array
+__global__ void __launch_bounds__(kSpecThreads) spec_raw_kernel(const double* sr, long long n, double* praw,
+                                                                double* power, SpecScratch s) {
   __shared__ double sh[32];
   double sde_raw;
   const double scale = raw_scale(s, gridDim.x, &sde_raw, sh), mean = s.state->mean_sr;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(M) spec_median_kernel(const double* __restrict
   }
 }
 
-// The running median for windows beyond the tiles: a thread per row ranks its
+// The running median where the tiles are not used: a thread per row ranks its
 // window by all pairs.
 __global__ void running_median_kernel(const double* __restrict__ praw, const uint8_t* __restrict__ mask,
                                       long long n, int k, double* __restrict__ med) {
@@ -314,10 +314,10 @@ __global__ void running_median_kernel(const double* __restrict__ praw, const uin
 }
 
 // power = power_raw - median (rows as above) and its sum
-__global__ void __launch_bounds__(kSpecThreads) spec_detrend_kernel(const double* __restrict__ praw,
+__global__ void __launch_bounds__(kSpecThreads) spec_detrend_kernel(const double* praw,
                                                                     const uint8_t* __restrict__ mask, long long n,
                                                                     int k, const double* __restrict__ med,
-                                                                    double* __restrict__ power, SpecScratch s) {
+                                                                    double* power, SpecScratch s) {
   __shared__ double sh[32];
   const long long rows = n - k + 1, front = (n - rows) / 2;
   double sum = 0;
@@ -378,14 +378,18 @@ int spectra_launch(const double* chi2, const uint8_t* mask, long long n, int k, 
   }
   const long long rows = n - k + 1;
   int parts = ctas;
+  // A caller that wants only some of the outputs may pass one array for several.
+  // The tiles read sr beyond their own places and write both powers, so
+  // they need three; the passes over whole arrays below read and write one place each.
+  const bool apart = sr != praw && sr != power && praw != power;
   auto tiles = [&](int m) { return (int)std::min<long long>(kSpecCtas, (rows + m - k) / (m - k + 1)); };
-  if (k <= 128) {
+  if (apart && k <= 128) {
     parts = tiles(256);
     spec_median_kernel<256><<<parts, 256, 0, st>>>(sr, mask, n, k, ctas, praw, power, s);
-  } else if (k <= 256) {
+  } else if (apart && k <= 256) {
     parts = tiles(512);
     spec_median_kernel<512><<<parts, 512, 0, st>>>(sr, mask, n, k, ctas, praw, power, s);
-  } else if (k <= 512) {
+  } else if (apart && k <= 512) {
     parts = tiles(1024);
     spec_median_kernel<1024><<<parts, 1024, 0, st>>>(sr, mask, n, k, ctas, praw, power, s);
   } else {

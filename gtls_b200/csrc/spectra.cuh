@@ -18,7 +18,7 @@ constexpr size_t kSpecParts = 6 * (size_t)kSpecCtas; // partial results of the l
 struct SpecScratch {
   double* part;       // [kSpecParts]
   SpecState* state;
-  double* med;        // [n], read and written for windows of more than 512 periods only
+  double* med;        // [n], read and written only where the median's tiles are not used
 };
 
 // Launches the spectra of n periods with a running median over k (none when n
