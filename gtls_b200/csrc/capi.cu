@@ -14,6 +14,8 @@ namespace gtls {
 
 static thread_local std::string g_create_error;
 
+constexpr size_t kPoolKeep = (size_t)64 << 20;   // bytes of a context's pool kept between calls (it grows by 32 MB at a time)
+
 int fail(gtls_ctx* ctx, int code, const std::string& msg) {
   if (ctx) ctx->err = msg;
   else g_create_error = msg;
@@ -145,8 +147,22 @@ int gtls_ctx_create(int device, gtls_ctx** out) {
   e = cudaGetDeviceProperties(&prop, device);
   if (e != cudaSuccess) return fail(nullptr, GTLS_E_CUDA, cudaGetErrorString(e));
   if (prop.major < 10) return fail(nullptr, GTLS_E_DEVICE, "gtls_b200 is built for sm_100a (B200)");
+  // keeps what its calls gave back, up to kPoolKeep, for the next ones
+  cudaMemPoolProps pp = {};
+  pp.allocType = cudaMemAllocationTypePinned;
+  pp.location.type = cudaMemLocationTypeDevice;
+  pp.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  unsigned long long keep = kPoolKeep;
+  e = cudaMemPoolCreate(&pool, &pp);
+  if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) {
+    if (pool) cudaMemPoolDestroy(pool);
+    return fail(nullptr, GTLS_E_CUDA, std::string("memory pool: ") + cudaGetErrorString(e));
+  }
   gtls_ctx* c = new gtls_ctx();
   c->device = device;
+  c->pool = pool;
   c->num_sms = prop.multiProcessorCount;
   c->smem_optin = (int)prop.sharedMemPerBlockOptin;
   *out = c;
@@ -158,6 +174,7 @@ int gtls_ctx_destroy(gtls_ctx* ctx) {
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();
   if (ctx->arena) cudaFree(ctx->arena);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   delete ctx;
   return GTLS_OK;
 }

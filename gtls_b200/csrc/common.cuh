@@ -19,6 +19,7 @@ struct gtls_ctx {
   std::string err;
   void* arena = nullptr;       // scratch arena (grows on demand)
   size_t arena_bytes = 0;
+  cudaMemPool_t pool = nullptr;  // scratch of calls that do not wait for their kernels
   long long launches = 0;      // kernels launched through this context
   size_t chunk_budget = (size_t)8 << 30;   // per-chunk scratch of a search, bytes
   int tile_cap_fp32 = gtls::kTileCapFp32;   // launch-shape tuning (gtls_set_tuning); results do not depend on it
