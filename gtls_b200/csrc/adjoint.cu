@@ -165,7 +165,8 @@ __device__ void block_sum(double (&v)[K], double* sh) {
 // chi2 of the curves (kGrad false: one value each) or its gradient (six).
 //
 // Some 2% of the samples are in transit and cost 96 quadrature nodes each, the
-// others nothing but their residual (none in the gradient).  A CTA therefore
+// others nothing but their residual (in the gradient a look whether it is finite:
+// 3% of the time).  A CTA therefore
 // looks at up to kAdjRound samples with one multiply-add each, lists those that
 // may be in transit, and then evaluates the list, four lanes to a sample, so
 // that a transit's neighbouring samples are spread over all its lanes.  On 1,024
@@ -217,10 +218,8 @@ __global__ void __launch_bounds__(kAdjThreads) model_kernel(const double* __rest
       for (int u = 0; u < kAdjItems; ++u) {
         const int i = i0 + 32 * u + lane;
         tv[u] = i < s1 ? tc[r0 + i] : 0.0;
-        if (!kGrad) {
-          yv[u] = i < s1 ? yc[r0 + i] : 1.0;
-          wv[u] = i < s1 ? wc[r0 + i] : 0.0;
-        }
+        yv[u] = i < s1 ? yc[r0 + i] : 1.0;
+        wv[u] = i < s1 ? wc[r0 + i] : 0.0;
       }
 #pragma unroll
       for (int u = 0; u < kAdjItems; ++u) {
@@ -229,9 +228,9 @@ __global__ void __launch_bounds__(kAdjThreads) model_kernel(const double* __rest
         const unsigned m = __ballot_sync(0xffffffffu, in);
         if (in) list[wid * kAdjSeg + hits + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(i - s0);
         hits += __popc(m);
-        if (!kGrad && i < s1 && !in) {
+        if (i < s1 && !in) {   // (the gradient: 0, or NaN where the residual is not finite)
           const double res = yv[u] - 1.0;
-          acc[0] += wv[u] * res * res;
+          acc[0] += wv[u] * res * (kGrad ? 0.0 : res);
         }
       }
     }
@@ -261,6 +260,11 @@ __global__ void __launch_bounds__(kAdjThreads) model_kernel(const double* __rest
       }
     }
     __syncthreads();
+  }
+  if constexpr (kGrad) {
+    const double bad = acc[0] - acc[0];   // NaN if anything was
+#pragma unroll
+    for (int k = 1; k < 6; ++k) acc[k] += bad;
   }
   block_sum<kOut>(acc, sh);
   if (threadIdx.x < kOut) part[(size_t)blockIdx.x * kOut + threadIdx.x] = sh[kOut * 32 + threadIdx.x];

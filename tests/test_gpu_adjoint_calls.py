@@ -1,8 +1,10 @@
 """How the model chi2 and its gradient may be called: they do not wait for
 their kernels, so they may be captured in a graph that outlives whatever the
-context does afterwards, and may overlap on several streams.
+context does afterwards, and may overlap on several streams.  And samples that
+are not finite: chi2 and the whole gradient of their curve are NaN, in transit or out.
 
-Bars: the same bits as the calls made alone.
+Bars: the same bits as the calls made alone; NaN where the model's own formula
+gives it, the other curves' bits unchanged.
 """
 import ctypes
 
@@ -97,3 +99,18 @@ def test_calls_overlap_on_two_streams_of_one_context(fresh):
     torch.cuda.synchronize()
     for s, (c, gr) in zip(sets, want):
         assert torch.equal(s["chi2"], c) and torch.equal(s["grad"], gr)
+
+
+@pytest.mark.parametrize("key,value", [("y", float("nan")), ("y", float("inf")), ("w", float("nan")), ("w", float("inf"))])
+@pytest.mark.parametrize("sample", [0, 4999, 9999])   # of the second curve; all out of transit
+def test_a_sample_that_is_not_finite_shows_in_the_gradient(cuda, key, value, sample):
+    s = _set(3, 10000, 4)
+    s["p"][:, 1] = 100.0 + 1.9
+    q = ((s["t"][10000 + sample] - s["p"][1, 1]) / s["p"][1, 0]).item()
+    assert abs(q - round(q)) * 2.3 > 0.11   # the sample lies outside every transit
+    c0, g0 = _alone(s)
+    s[key][10000 + sample] = value
+    c1, g1 = _alone(s)
+    assert g1[1].isnan().all() and not c1[1].isfinite()
+    for i in (0, 2):
+        assert c1[i] == c0[i] and (g1[i] == g0[i]).all()
