@@ -1130,6 +1130,18 @@ struct Upload {
   }
 };
 
+// Scratch of one period: slots and fold order, and per CTA a row of the prefix
+// of v (curves with a coarse prefix), its list and its result; and the row.
+static size_t v_stride(int tile, int max_width) {
+  const int coarse = coarse_step(tile, max_width);
+  return coarse > 0 ? ((size_t)tile + max_width + 2 * coarse + 8) / 8 * 8 : 0;
+}
+static size_t period_bytes(int n, int max_width, int tile, bool all) {
+  const size_t ctas = ((size_t)n + tile - 1) / tile;
+  return (size_t)n * (sizeof(uint2) + sizeof(int)) +
+         ctas * (sizeof(float) * v_stride(tile, max_width) + list_entries(all) * sizeof(Waiting) + 16) + 4;
+}
+
 template <typename Real>
 static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int precision_pass, int skip_point,
                       double depth_min, int flags, gtls_timing* tm, cudaStream_t st) {
@@ -1189,7 +1201,12 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
   const long long per = np_total > 0 && ctas < want ? std::max<long long>(1, (want + (peaked ? np_total - 1 : 0)) / np_total) : 1;
   for (int c = 0; c < n_curves; ++c) {
     const long long tiles = std::max<long long>(cd[c].ntiles, std::min<long long>(per, (ch[c].n + 511) / 512));
-    const long long tile = ((ch[c].n + tiles - 1) / tiles + 31) / 32 * 32;
+    long long tile = ((ch[c].n + tiles - 1) / tiles + 31) / 32 * 32;
+    // A period that does not fit the scratch budget so is cut into fewer
+    // ranges; as one range it takes less than the budget it is refused under (below).
+    const long long widest = std::min<long long>(((long long)ch[c].n + 31) / 32 * 32, all ? kBlockTable * kBlockStarts : 1 << 26);
+    while (tile < widest && period_bytes(ch[c].n, ch[c].max_width, (int)tile, all) > ctx->chunk_budget)
+      tile = std::min(widest, 2 * tile);
     cd[c].tile = (int)tile;
     cd[c].ntiles = (int)((ch[c].n + tile - 1) / tile);
   }
@@ -1247,7 +1264,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     C.max_width = maxd;
     C.batch = h.batch;
     C.nbatch = (int)((h.np + h.batch - 1) / h.batch);
-    C.vstride = C.coarse > 0 ? (C.tile + maxd + 2 * C.coarse + 8) / 8 * 8 : 0;
+    C.vstride = (int)v_stride(C.tile, maxd);
     C.nb_log2 = nb_log2_for(n, ctx->bucket_shift);
     rounds_params(C, ctx->smem_optin);
     C.span = h.span;
@@ -1288,10 +1305,8 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     };
     for (int c = 0; c < n_curves; ++c) {
       const CurveDev<Real>& C = cd[c];
-      const size_t per = (size_t)C.n * (sizeof(uint2) + sizeof(int)) +
-                         (size_t)C.ntiles * (sizeof(float) * C.vstride + list_cap * sizeof(Waiting) + 16) + 4;
-      // the smallest budget a period is accepted with (as documented: slots, a
-      // record and a prefix value per sample and wrapped sample)
+      const size_t per = period_bytes(C.n, C.maxd, C.tile, all);
+      // the smallest budget a period is accepted with (as documented)
       const size_t least = (size_t)C.n * 8 + (size_t)(C.n + C.maxd + 1) * (sizeof(R2) + 8);
       long long p = 0;
       // one prepare shape per chunk
@@ -1299,7 +1314,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
       if (C.np > 0 && mode != -1 && mode != cmode) close_chunk();
       while (p < C.np) {
         long long fit = (long long)((budget > bytes ? budget - bytes : 0) / per);
-        if (items == 0) fit = budget < least ? 0 : std::max<long long>(fit, 1);
+        if (budget < least) fit = 0;
         fit = std::min<long long>(fit, (long long)INT32_MAX - items);
         fit = std::min<long long>(fit, ((1LL << 31) - 1 - tiles) / C.ntiles);
         if (fit <= 0) {

@@ -74,9 +74,12 @@ int gtls_decode_status(int32_t word, char* msg, size_t cap);
 int64_t gtls_launch_count(const gtls_ctx* ctx);
 
 /* Bytes of per-chunk scratch a search may use (sort slots, fold order, lists
- * of starts; default 8 GiB).  A period is accepted from 48 bytes a sample on.  Periods are processed in chunks that fit it;
- * results do not depend on it.  No counterpart in the reference, whose
- * batch size comes from the free-memory formula of core.py:620-628.
+ * of starts; default 8 GiB; a curve's own arrays come on top).  Periods are
+ * processed in chunks that fit it, a period that does not in fewer and longer
+ * ranges of starts; results do not depend on it.  Below 8 n + (n + max_width +
+ * 1) x 24 bytes (FP32: x 16) a search is refused with GTLS_E_RANGE.  No
+ * counterpart in the reference, whose batch size comes from the free-memory
+ * formula of core.py:620-628.
  * bytes must be >= 1 MiB. */
 int gtls_set_chunk_budget(gtls_ctx* ctx, uint64_t bytes);
 
