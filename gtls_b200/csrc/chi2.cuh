@@ -26,6 +26,13 @@ constexpr int kBlockStarts = 64;                 // all-starts pass: consecutive
 constexpr int kBlockSamples = 2048;              // samples of their windows in shared memory at a time
 constexpr int kBlockSlots = 2048;                // blocks of a CTA taken up at a time
 
+// Rounding of a difference of two prefix values, relative to the largest of
+// them: they are summed in FP64 and rounded to FP32 once each.  (Summed in FP32
+// the bound was 2^-16 of the largest; after six flares of 50% it left so many
+// starts that the list ran over: 300 periods of 19,728 samples 18.5 ms, now 0.61,
+// of 70,000 92 and 1.67 ms.  Without flares both take the same time.)
+constexpr float kPrefixErr = 0x1.01p-23f;
+
 // Arrays of prefix values are skewed by one word per 32, so that starts a
 // power of two apart fall into different banks.
 __host__ __device__ __forceinline__ int skew(int p) { return p + (p >> 5); }
@@ -426,8 +433,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   __shared__ double part_s[kChiWarps];
   __shared__ int2 together[kTogether];          // union position (-1: ruled out) and start
   __shared__ unsigned maxbits[4];
-  __shared__ double carry_v, wtot_v[kChiWarps];
-  __shared__ float carry[3], wtot[kChiWarps][3];
+  __shared__ double carry[4], wtot[kChiWarps][4];   // of v, u, w, u^2
   __shared__ Best red[kChiWarps];
   __shared__ long long sent_sm;                 // first start of the range known to fail the depth test
   __shared__ unsigned long long work_sm[2];
@@ -536,12 +542,11 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       list_n = redo_n = 0;
       low_key = 0x7f800000;
       tau_key = 0x7f800000;   // infinity
-      carry_v = 0.0;
       sent_sm = kNone;
       work_sm[0] = work_sm[1] = 0;
     }
     if (lane < 4) maxbits[lane] = 0;
-    if (lane < 3) carry[lane] = 0.f;
+    if (lane < 4) carry[lane] = 0.0;
   } else if (wid == 4 && lane < (int)(sizeof(CurveConst) / 4)) {
     reinterpret_cast<int*>(&cc)[lane] = reinterpret_cast<const int*>(C.cst)[lane];
   } else if (wid == 1 && lane < 4) {
@@ -601,27 +606,30 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const double2* __restrict__ vw = ex.fold.vw;
     if (k0 + q0 + kBatch < n)   // the next batch's indices: into L2
       asm volatile("prefetch.global.L2 [%0];" ::"l"(ord + k0 + q0 + kBatch));
-    double v[kItems], sv = 0.0;
-    float uu[kItems], ww[kItems], su = 0.f, sw = 0.f, sq = 0.f;
+    // u, w - wbar and u^2 - qbar of an item, scaled in FP64 (a weight itself may be beyond FP32)
+    auto item = [&](int i, double& v, double& u, double& w, double& q) {
+      v = gq[i].x * cc.vscale;
+      w = gq[i].y * cc.wscale;
+      u = v * w;
+      q = fma(u, u, -(double)cc.qbar);
+      w -= (double)cc.wbar;
+      if (i >= have) w = q = 0.0;
+    };
+    double sv = 0.0, su = 0.0, sw = 0.0, sq = 0.0;
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
-      v[i] = gq[i].x * cc.vscale;
-      const double w = gq[i].y * cc.wscale;   // scaled in FP64: a weight itself may be beyond FP32
-      const float wf = (float)w;
-      uu[i] = (float)(v[i] * w);
-      ww[i] = i < have ? wf - cc.wbar : 0.f;
-      sv += v[i];
-      su += uu[i];
-      sw += ww[i];
-      if (i < have) sq += fmaf(uu[i], uu[i], -cc.qbar);
+      double v, u, w, q;
+      item(i, v, u, w, q);
+      sv += v;
+      su += u;
+      sw += w;
+      sq += q;
     }
-    double xv = sv;
-    float xu = su, xw = sw, xq = sq;
+    double xv = sv, xu = su, xw = sw, xq = sq;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const double yv = __shfl_up_sync(0xffffffffu, xv, o);
-      const float yu = __shfl_up_sync(0xffffffffu, xu, o), yw = __shfl_up_sync(0xffffffffu, xw, o),
-                  yq = __shfl_up_sync(0xffffffffu, xq, o);
+      const double yv = __shfl_up_sync(0xffffffffu, xv, o), yu = __shfl_up_sync(0xffffffffu, xu, o),
+                   yw = __shfl_up_sync(0xffffffffu, xw, o), yq = __shfl_up_sync(0xffffffffu, xq, o);
       if (lane >= o) {
         xv += yv;
         xu += yu;
@@ -630,10 +638,10 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       }
     }
     if (lane == 31) {
-      wtot_v[wid] = xv;
-      wtot[wid][0] = xu;
-      wtot[wid][1] = xw;
-      wtot[wid][2] = xq;
+      wtot[wid][0] = xv;
+      wtot[wid][1] = xu;
+      wtot[wid][2] = xw;
+      wtot[wid][3] = xq;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -641,10 +649,10 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       if (ntiles > 1) atomicMin(&tau_key, atomicMin(tau_all, *(volatile int*)&tau_key));
     }
     const bool before = lane < wid;   // kChiWarps <= 32
-    double rv = carry_v + warp_sum(before ? wtot_v[lane] : 0.0) + (xv - sv);
-    float ru = carry[0] + (warp_sum(before ? wtot[lane][0] : 0.f) + (xu - su));
-    float rw = carry[1] + (warp_sum(before ? wtot[lane][1] : 0.f) + (xw - sw));
-    float rq = carry[2] + (warp_sum(before ? wtot[lane][2] : 0.f) + (xq - sq));
+    double rv = carry[0] + warp_sum(before ? wtot[lane][0] : 0.0) + (xv - sv);
+    double ru = carry[1] + warp_sum(before ? wtot[lane][1] : 0.0) + (xu - su);
+    double rw = carry[2] + warp_sum(before ? wtot[lane][2] : 0.0) + (xw - sw);
+    double rq = carry[3] + warp_sum(before ? wtot[lane][3] : 0.0) + (xq - sq);
     float mv = 0.f, mu = 0.f, mw = 0.f, mq = 0.f;
     int cq = 0, cr = 1;   // next coarse step and the items up to it
     if (g > 0) {
@@ -654,27 +662,29 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       if (i < have) {
-        rv += v[i];
-        ru += uu[i];
-        rw += ww[i];
-        rq += fmaf(uu[i], uu[i], -cc.qbar);
-        const float fv = (float)rv;
+        double v, u, w, q;
+        item(i, v, u, w, q);
+        rv += v;
+        ru += u;
+        rw += w;
+        rq += q;
+        const float fv = (float)rv, fu = (float)ru, fw = (float)rw, fq = (float)rq;
         mv = fmaxf(mv, fabsf(fv));
-        mu = fmaxf(mu, fabsf(ru));
-        mw = fmaxf(mw, fabsf(rw));
-        mq = fmaxf(mq, fabsf(rq));
+        mu = fmaxf(mu, fabsf(fu));
+        mw = fmaxf(mw, fabsf(fw));
+        mq = fmaxf(mq, fabsf(fq));
         float* const to = ringV + skew((q0 + i + 1) & (kRing - 1));
         to[0] = fv;
-        to[kRingWords] = ru;
-        to[2 * kRingWords] = rw;
-        to[3 * kRingWords] = rq;
+        to[kRingWords] = fu;
+        to[2 * kRingWords] = fw;
+        to[3 * kRingWords] = fq;
         if (g > 0) {
           vrow[q0 + i + 1] = fv;
           if (i + 1 == cr && cq < kCoarseCap) {   // g >= 8 > kItems: at most one
             float* const tc = coarse + skew(cq);
-            tc[0] = ru;
-            tc[kCoarseWords] = rw;
-            tc[2 * kCoarseWords] = rq;
+            tc[0] = fu;
+            tc[kCoarseWords] = fw;
+            tc[2 * kCoarseWords] = fq;
           }
         }
       }
@@ -687,10 +697,10 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     if (lane < 4) atomicMax(&maxbits[lane], lane == 0 ? r0 : (lane == 1 ? r1 : (lane == 2 ? r2 : r3)));
     __syncthreads();   // the carry has been read by all
     if (threadIdx.x == kChiThreads - 1) {   // the last thread's end is the batch's
-      carry_v = rv;
-      carry[0] = ru;
-      carry[1] = rw;
-      carry[2] = rq;
+      carry[0] = rv;
+      carry[1] = ru;
+      carry[2] = rw;
+      carry[3] = rq;
     }
     ld += cnt;
   };
@@ -735,9 +745,9 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const int d = dur[u];
     const int w = (int)(wsk[u] & 0xffff);
     const float inv_w = row_sm[wid][0].inv_w;
-    const ScreenErr e = screen_err(__uint_as_float(maxbits[0]) * 0x1p-23f, __uint_as_float(maxbits[1]) * cc.prefix_err,
-                                   __uint_as_float(maxbits[2]) * cc.prefix_err,
-                                   __uint_as_float(maxbits[3]) * cc.prefix_err);
+    const ScreenErr e = screen_err(__uint_as_float(maxbits[0]) * kPrefixErr, __uint_as_float(maxbits[1]) * kPrefixErr,
+                                   __uint_as_float(maxbits[2]) * kPrefixErr,
+                                   __uint_as_float(maxbits[3]) * kPrefixErr);
     const float em0 = e.v * inv_w + 2e-7f * fabsf(dthr);
     // depth test on the sum: fails for certain where V(k) - V(k + w) is below this
     const float vmin = (dthr - em0 - 4e-7f * fabsf(dthr)) / inv_w;
@@ -934,8 +944,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     if (kAll) {
       ld = 0;
       if (threadIdx.x == 0) {
-        carry_v = 0.0;
-        carry[0] = carry[1] = carry[2] = 0.f;
+        carry[0] = carry[1] = carry[2] = carry[3] = 0.0;
       } else if (threadIdx.x >= 32 && threadIdx.x < 36) {
         ringV[lane * kRingWords] = 0.f;
       }

@@ -63,7 +63,6 @@ struct CurveConst {
   double ebase;            // sum v^2 w
   double vscale, wscale, dscale;
   float wbar, qbar;        // mean of the scaled w and u^2
-  float prefix_err;        // rounding of a difference of two prefix values, relative to the largest of them
   int uniform;             // all weights equal
 };
 
@@ -97,7 +96,6 @@ struct CurveDev {
   int tile, ntiles, nb_log2;    // starts of a chi2 CTA, CTAs of a period, bucket bits (global-scatter ordering)
   int rnb_log2, rcap;           // shared-memory prepare path: bucket bits and round capacity (0: off)
   int coarse, vstride;          // chi2: step of the coarse prefix (0: none), row of the prefix of v of a CTA
-  int max_cell;                 // longest cell (samples)
   float span;
 };
 
@@ -198,10 +196,6 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     cc.dscale = cc.vscale * cc.vscale * cc.wscale;
     cc.wbar = (float)(red[2][0] * cc.wscale / C.n);
     cc.qbar = (float)(red[3][0] * (cc.vscale * cc.wscale) * (cc.vscale * cc.wscale) / C.n);
-    // a prefix value carries some 20 roundings of a batch's scan, each of at
-    // most the largest prefix value times 2^-23, and one batch's more for each
-    // batch that a cell spans
-    cc.prefix_err = 0x1p-18f * (4.f + C.max_cell / 2048);
     cc.uniform = red[4][0] == red[5][0];
     *C.cst = cc;
   }
@@ -1222,7 +1216,6 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     const int* hw = widths.data() + d_off[c];
     size_t rows = 0, cells = (size_t)D * kLaneCells;
     C.coarse = coarse_step(C.tile, maxd);
-    C.max_cell = 0;
     for (int i = 0; i < D; ++i) {
       const int w = hw[i];
       if (w < 1 || w > maxd || (i > 0 && w <= hw[i - 1]))
@@ -1242,7 +1235,6 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
         if (k == 1) cells += e.size();
         ends.resize(cell_off[c] + cells);
         std::copy(e.begin(), e.end(), ends.begin() + cell_off[c] + r.first);
-        for (size_t q = 0; q < e.size(); ++q) C.max_cell = std::max(C.max_cell, (e[q] - (q ? e[q - 1] : 0)) * g);
       }
     }
     if (maxd > 0xffff) return fail(ctx, GTLS_E_RANGE, "max_width above 65535");
