@@ -74,9 +74,62 @@ struct Waiting {
   int k, u;
 };
 
-// Per CTA: the list, the tasks that found it full, and (all starts) the blocks.
-constexpr int list_entries(bool all) { return (all ? kListAll + kBlockTable / 3 : kList) + kRedo; }
-static_assert(sizeof(Waiting) == 3 * sizeof(int), "");
+// A spike (search.cu) among the samples of a CTA's range: its place in the range.
+struct Spike {
+  int q;
+  float u, w;
+};
+
+// Spikes of part of the range, and the rounding of sums over them.
+struct NearSpikes {
+  const Spike* at;
+  int n, uniform;
+  float err;
+};
+__device__ __forceinline__ NearSpikes near_spikes(const Spike* spikes, int from, int end, int uniform) {
+  NearSpikes s;
+  s.at = spikes + from;
+  s.n = min(end, kSpikes) - from;
+  s.uniform = uniform;
+  s.err = end > kSpikes ? INFINITY : 1.2e-7f * (float)(s.n + 8);   // (there are no more, by their choice)
+  return s;
+}
+// One spike that a window holds, where the template is t = (s, s^2).
+template <typename R2>
+__device__ __forceinline__ void add_spike(CellSums& cs, const NearSpikes& s, const R2& t, float u, float w) {
+  const float b = (float)t.x * u, c = s.uniform ? 0.f : (float)t.y * w;
+  cs.B += b;
+  cs.er = fmaf(fabsf(b), s.err, cs.er);
+  cs.cl = fmaf(c, 1.f - s.err, cs.cl);
+  cs.cu = fmaf(c, 1.f + s.err, cs.cu);
+}
+// Those of the lanes' windows of w samples, which start at q (ascending);
+// returns their sum of u^2.
+template <typename R2>
+__device__ __forceinline__ float add_spikes(CellSums& cs, const NearSpikes& s, const R2* __restrict__ trow, int q, int w) {
+  const int lane = threadIdx.x & 31;
+  const int from = __shfl_sync(0xffffffffu, q, 0), to = __shfl_sync(0xffffffffu, q, 31) + w;
+  float sq = 0.f;
+  for (int i0 = 0; i0 < s.n; i0 += 32) {
+    Spike x{-1, 0.f, 0.f};
+    if (i0 + lane < s.n) x = s.at[i0 + lane];
+    for (unsigned m = __ballot_sync(0xffffffffu, x.q >= from && x.q < to); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const int i = __shfl_sync(0xffffffffu, x.q, src) - q;
+      const float u = __shfl_sync(0xffffffffu, x.u, src), v = __shfl_sync(0xffffffffu, x.w, src);
+      if (i >= 0 && i < w) {
+        add_spike(cs, s, trow[i], u, v);
+        sq = fmaf(u, u, sq);
+      }
+    }
+  }
+  if (s.err == INFINITY) cs.er = INFINITY;
+  return sq;
+}
+
+// Per CTA: the list, the tasks that found it full, (all starts) the blocks, and the spikes.
+constexpr int list_entries(bool all) { return (all ? kListAll + kBlockTable / 3 : kList) + kRedo + kSpikes; }
+static_assert(sizeof(Waiting) == 3 * sizeof(int) && sizeof(Spike) == sizeof(Waiting), "");
 
 struct Chi2Args {
   int nruns;
@@ -437,6 +490,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   __shared__ Best red[kChiWarps];
   __shared__ long long sent_sm;                 // first start of the range known to fail the depth test
   __shared__ unsigned long long work_sm[2];
+  __shared__ int spike_end[4], spike_tot[kChiWarps];   // spikes up to the end of batch b: in [b & 3]
 
   const int cta = blockIdx.x;
   const int ri = upper_find(0, a.nruns, cta, [&](int i) { return (long long)runs[i].tile0; });
@@ -484,15 +538,18 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   int* const btable = reinterpret_cast<int*>(list + kCap + kRedo);
   const int nblk = (k1 - k0 + kBlockStarts - 1) / kBlockStarts;
   int bgroup = 0;
-  if constexpr (kAll)
+  if constexpr (kAll) {
     while ((long long)nblk * (((ucnt - 1) >> bgroup) + 1) > kBlockTable) ++bgroup;
+  }
   const int bpos = ((ucnt - 1) >> bgroup) + 1;   // groups of positions
   constexpr int kNoBlock = 0x7fffffff;
   auto to_block = [&](int u, int k, float lb) {   // a NaN's key may be the empty block's
     atomicMin(&btable[(k - k0) / kBlockStarts * bpos + (u >> bgroup)], float_key(lb == lb ? lb : -INFINITY));
   };
-  if constexpr (kAll)
+  if constexpr (kAll) {
     for (int i = threadIdx.x; i < nblk * bpos; i += kChiThreads) btable[i] = kNoBlock;
+  }
+  Spike* const spikes = reinterpret_cast<Spike*>(list + list_entries(kAll) - kSpikes);
   int* const tau_all = a.tau + (R.item0 + local);
   // FP32 exact sums round by up to (w + 8) half ulps of their absolute sum
   auto gamma_of = [&](int w) { return kGammaF + (sizeof(Real) == 4 ? (float)(w + 8) * 1.2e-7f : 0.f); };
@@ -545,7 +602,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       sent_sm = kNone;
       work_sm[0] = work_sm[1] = 0;
     }
-    if (lane < 4) maxbits[lane] = 0;
+    if (lane < 4) maxbits[lane] = spike_end[lane] = 0;
     if (lane < 4) carry[lane] = 0.0;
   } else if (wid == 4 && lane < (int)(sizeof(CurveConst) / 4)) {
     reinterpret_cast<int*>(&cc)[lane] = reinterpret_cast<const int*>(C.cst)[lane];
@@ -561,6 +618,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   const float dthr = (float)(a.depth_min * cc.vscale);
   // E + delta and n are rounded to doubles: starts that close to tau stay
   const float margin = (float)((fabs(cc.ebase) + (double)n) * cc.dscale * 0x1p-44);
+  const bool spiky = cc.spike_u < INFINITY || cc.spike_w < INFINITY;
   auto over_tau = [&](float lb) { return lb > key_float(*(volatile int*)&tau_key) + margin; };
 
   // (the warp's best exact value lives in red[wid]: few starts get one)
@@ -581,6 +639,11 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   // registers (before the barrier that ends the screening of the batch
   // before, so that a warp that waits there waits for its loads as well),
   // store() adds their prefix values.
+  auto is_spike = [&](const double2& g) {
+    const double w = g.y * cc.wscale;
+    return fabs(g.x * cc.vscale * w) >= cc.spike_u || w > cc.spike_w;
+  };
+  int batches = 0;           // stored so far
   int ld = 0, fetched = 0;   // samples whose prefix values are stored, samples fetched
   double2 gq[kItems];
   auto fetch = [&](int cnt) {
@@ -606,6 +669,31 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const double2* __restrict__ vw = ex.fold.vw;
     if (k0 + q0 + kBatch < n)   // the next batch's indices: into L2
       asm volatile("prefetch.global.L2 [%0];" ::"l"(ord + k0 + q0 + kBatch));
+    ++batches;
+    if (spiky) {   // listed in order; their u and w are 0 in what follows
+      int mine = 0;
+#pragma unroll
+      for (int i = 0; i < kItems; ++i) mine += i < have && is_spike(gq[i]);
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += y;
+      }
+      if (lane == 31) spike_tot[wid] = upto;
+      __syncthreads();
+      int at = spike_end[(batches - 1) & 3] + upto - mine;
+      for (int q = 0; q < wid; ++q) at += spike_tot[q];
+#pragma unroll
+      for (int i = 0; i < kItems; ++i)
+        if (i < have && is_spike(gq[i])) {
+          const double w = gq[i].y * cc.wscale, u = gq[i].x * cc.vscale * w;
+          if (at < kSpikes) spikes[at] = Spike{q0 + i, (float)u, (float)w};
+          ++at;
+          gq[i].y = 0.0;
+        }
+      if (threadIdx.x == kChiThreads - 1) spike_end[batches & 3] = at;
+    }
     // u, w - wbar and u^2 - qbar of an item, scaled in FP64 (a weight itself may be beyond FP32)
     auto item = [&](int i, double& v, double& u, double& w, double& q) {
       v = gq[i].x * cc.vscale;
@@ -737,8 +825,8 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
 
   // screen starts j0 s .. (j1 - 1) s (at most kTaskStarts) of union position u,
   // whose rows are in the warp's buffers; probe: only lower tau
-  auto screen = [&](auto coarse_tag, int u, int s, int j0, int j1, bool probe) {
-    constexpr bool kCoarse = decltype(coarse_tag)::value;
+  auto screen = [&](auto coarse_tag, auto spiky_tag, int u, int s, int j0, int j1, bool probe) {
+    constexpr bool kCoarse = decltype(coarse_tag)::value, kSpiky = decltype(spiky_tag)::value;
     const float* const xU = kCoarse ? coarse : ringU;
     constexpr int kWords = kCoarse ? kCoarseWords : kRingWords;
     auto at = [&](int p) { return xU + skew(kCoarse ? p : p & (kRing - 1)); };
@@ -777,6 +865,12 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     __syncwarp();
     if (a.work && lane == 0 && !probe) atomicAdd(&work_sm[0], (unsigned long long)cnt * 2 * (unsigned)w);
     const float gamma = gamma_of(w);
+    // the spikes that the windows may hold (the ring has samples of the last two batches)
+    NearSpikes near;
+    if constexpr (kSpiky) {
+      const int from = kCoarse ? 0 : spike_end[(batches - 2) & 3];
+      near = near_spikes(spikes, from, spike_end[batches & 3], cc.uniform);
+    }
     for (int b = 0; b < cnt; b += 32) {
       const int k = (j0 + queue[wid][min(b + lane, cnt - 1)]) * s;
       const int q = k - k0;
@@ -803,7 +897,8 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       }
       const float m = (v_at(coarse_tag, q) - v_at(coarse_tag, q + w)) * inv_w;
       const float em = fmaf(3e-7f, fabsf(m), em0);
-      const float qwin = (pq - q00) + (float)(kCoarse ? end * g : w) * cc.qbar + 4.f * e.n2;
+      float qwin = (pq - q00) + (float)(kCoarse ? end * g : w) * cc.qbar + 4.f * e.n2;
+      if constexpr (kSpiky) qwin += add_spikes(cs, near, ex.trows + ex.trow_off[d], q, w);
       float lb = start_bounds<false>(cs, row_sm[wid][0], m, em, qwin, cc.wbar, cc.uniform, gamma, e).lb;
       // too close to the depth threshold to tell: such a start needs its exact value (n, if it fails)
       const bool certain = m - em > dthr;
@@ -838,6 +933,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           __syncwarp();
           cells_sm[wid][lane] = reinterpret_cast<const float4*>(scells + (size_t)d * kLaneCells)[lane];
           __syncwarp();
+          if constexpr (kSpiky) add_spikes(s2, near, ex.trows + ex.trow_off[d], q, w);
           const StartBounds sb = start_bounds<true>(s2, row_sm[wid][1], m, em, qwin, cc.wbar, cc.uniform, gamma, e);
           lb = sb.lb;
           const bool on = left >> lane & 1;
@@ -879,6 +975,14 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           add_cell<kCoarse, true>(s2, c, x1[0] - x0[0], x1[kWords] - x0[kWords], x1[2 * kWords] - x0[2 * kWords], kap,
                                   cc.qbar, e);
         }
+        if constexpr (kSpiky) {
+          const R2* const trow = ex.trows + ex.trow_off[d];
+          if (near.err == INFINITY) s2.er = INFINITY;
+          for (int i = lane; i < near.n; i += 32) {
+            const Spike x = near.at[i];
+            if (x.q >= qs && x.q < qs + w) add_spike(s2, near, trow[x.q - qs], x.u, x.w);
+          }
+        }
         s2.B = warp_sum(s2.B);
         s2.er = warp_sum(s2.er);
         s2.cl = warp_sum(s2.cl);
@@ -915,7 +1019,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     return __shfl_sync(0xffffffffu, tk, 0);
   };
   // all tasks of starts in [t0, t1) for the union positions u_lo .. u_lo + cnt - 1
-  auto run_tasks = [&](auto coarse_tag, int u_lo, int cnt, int t0, int t1, bool probe) {
+  auto run_tasks_of = [&](auto coarse_tag, auto spiky_tag, int u_lo, int cnt, int t0, int t1, bool probe) {
     const int ntask = task_pre[cnt];
     int u = 0, sub = 0;
     auto next = [&]() {   // claims a task and sends for its rows
@@ -935,9 +1039,13 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       more = next();
       const int s = probe ? max(1, (int)(wsk[cu] & 0xffff) / kProbe) : (kAll ? 1 : (int)(wsk[cu] >> 16));
       const int j0 = (t0 + s - 1) / s + csub * kTaskStarts, j1 = min((t1 + s - 1) / s, j0 + kTaskStarts);
-      if (j0 < j1) screen(coarse_tag, cu, s, j0, j1, probe);
+      if (j0 < j1) screen(coarse_tag, spiky_tag, cu, s, j0, j1, probe);
       __syncwarp();
     }
+  };
+  auto run_tasks = [&](auto coarse_tag, int u_lo, int cnt, int t0, int t1, bool probe) {
+    if (spiky) run_tasks_of(coarse_tag, std::true_type{}, u_lo, cnt, t0, t1, probe);
+    else run_tasks_of(coarse_tag, std::false_type{}, u_lo, cnt, t0, t1, probe);
   };
   for (int sweep = kAll ? 0 : 1; sweep < 2; ++sweep) {
     const bool probe = sweep == 0;
@@ -945,6 +1053,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       ld = 0;
       if (threadIdx.x == 0) {
         carry[0] = carry[1] = carry[2] = carry[3] = 0.0;
+        spike_end[0] = spike_end[1] = spike_end[2] = spike_end[3] = 0;
       } else if (threadIdx.x >= 32 && threadIdx.x < 36) {
         ringV[lane * kRingWords] = 0.f;
       }

@@ -62,8 +62,10 @@ constexpr int kPrepStaticSmem = 4096;  // static shared memory of prepare_kernel
 struct CurveConst {
   double ebase;            // sum v^2 w
   double vscale, wscale, dscale;
-  float wbar, qbar;        // mean of the scaled w and u^2
+  double spike_u, spike_w; // samples of larger |u| or w (scaled) are spikes; infinite: none
+  float wbar, qbar;        // mean of the scaled w and u^2, of samples that are no spikes
   int uniform;             // all weights equal
+  int pad;
 };
 
 // Per-light-curve parameters and buffers on the device.  A search covers one
@@ -131,11 +133,13 @@ __device__ __forceinline__ int upper_find(int lo, int hi, long long x, F key) {
 // 70,000 samples); the last of a curve's CTAs adds their parts, in order.
 constexpr int kSetupThreads = 256;
 constexpr int kSetupItems = 1024;
-constexpr int kSetupSums = 6;   // E, sum v^2, sum w, sum u^2, min w, max w
+constexpr int kSetupSums = 8;   // E, sum v^2, sum w, sum u^2, min w, max w, sum |u|^(1/2), sum w^(1/2)
+static_assert(kSetupSums <= kSetupThreads / 32, "a warp adds up each");
 
 __device__ __forceinline__ double sums_join(int k, double x, double y) {
-  return k < 4 ? x + y : (k == 4 ? fmin(x, y) : fmax(x, y));
+  return k == 4 ? fmin(x, y) : (k == 5 ? fmax(x, y) : x + y);
 }
+__device__ __forceinline__ double sums_none(int k) { return k == 4 ? INFINITY : (k == 5 ? -INFINITY : 0.0); }
 
 // Power of two that brings x to [1, 2), or 1 where there is none.
 __device__ __forceinline__ double unit_scale(double x) {
@@ -143,12 +147,93 @@ __device__ __forceinline__ double unit_scale(double x) {
   return exp2(-(double)ilogb(x));
 }
 
+// Spikes.  The bounds of a start (screen.cuh) come from differences of FP32
+// prefix sums, which one sample of a million times the others' |u| (its u^2 a
+// 10^12-fold) or w would leave without a digit for every cell after it: the list of
+// waiting starts ran over, and 300 periods of 70,000 samples with one dy
+// a thousandth of the others took 92 ms (now 1.9; clean 1.8).  Such samples, at most 2
+// kSpikeMax of a curve, are left out of the prefix sums and added to the bounds of the
+// windows that hold them.  The sums round to 2^-23 of the whole (kPrefixErr), so
+// a curve has spikes where sum u^2 is above 2^30 typical ones (a cell's u^2 then
+// rounds by 128 of them, which flares show the bounds to bear) or a weight
+// above 2^20; the typical one is the square of the mean square root, which spikes
+// hardly move.  A sample is a spike from the largest power of two (times the
+// typical |u|) on below which the sum stays within that, or from the smallest
+// that leaves at most kSpikeMax.
+constexpr int kSpikeMax = 256;
+constexpr int kSpikes = 4 * kSpikeMax;   // of a CTA: a window may run once more around the curve
+constexpr double kSpikeSum = 0x1p30, kSpikeW = 0x1p20;
+
+// The curve's thresholds of |u| and w, and its sums 1 to 3 without its spikes,
+// by one CTA (typical_u and typical_w as above).
+template <typename Real>
+__device__ void find_spikes(const CurveDev<Real>& C, double typical_u, double typical_w, double (&sums)[4], double* thr) {
+  constexpr int kBins = 96, kFirst = 4;   // |u| of 2^kFirst typical ones on, by powers of two
+  __shared__ int hist[kBins], heavy;
+  __shared__ double limit[2], red[3][kSetupThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int b = threadIdx.x; b < kBins; b += kSetupThreads) hist[b] = 0;
+  if (threadIdx.x == 0) heavy = 0;
+  __syncthreads();
+  auto sample = [&](int i, double& v, double& w) {
+    v = C.y[i] - 1.0;
+    const double d = C.dy[i];
+    w = 1.0 / (d * d);
+  };
+  for (int i = threadIdx.x; i < C.n; i += kSetupThreads) {
+    double v, w;
+    sample(i, v, w);
+    const double x = fabs(v * w) / typical_u;
+    if (x >= (double)(1 << kFirst)) atomicAdd(&hist[min(kBins - 1, ilogb(x) - kFirst)], 1);
+    if (w > kSpikeW * typical_w) atomicAdd(&heavy, 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int above = 0, j = 0;
+    for (int b = 0; b < kBins; ++b) above += hist[b];
+    double sum = 0.0, unit = (double)(1 << kFirst);
+    for (; j < kBins; ++j, unit *= 2.0) {   // unit: the least |u| of bin j
+      sum += 4.0 * unit * unit * hist[j];
+      if (sum > kSpikeSum && above <= kSpikeMax) break;
+      above -= hist[j];
+    }
+    limit[0] = j < kBins ? typical_u * unit : INFINITY;
+    limit[1] = heavy <= kSpikeMax ? kSpikeW * typical_w : INFINITY;
+  }
+  __syncthreads();
+  double s[3] = {0.0, 0.0, 0.0};
+  for (int i = threadIdx.x; i < C.n; i += kSetupThreads) {
+    double v, w;
+    sample(i, v, w);
+    const double u = v * w;
+    if (fabs(u) >= limit[0] || w > limit[1]) continue;
+    s[0] += v * v;
+    s[1] += w;
+    s[2] += u * u;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+    if (lane == 0) red[k][wid] = s[k];
+  }
+  __syncthreads();
+  thr[0] = limit[0];
+  thr[1] = limit[1];
+  for (int k = 0; k < 3; ++k) {
+    sums[1 + k] = 0.0;
+    for (int q = 0; q < kSetupThreads / 32; ++q) sums[1 + k] += red[k][q];
+  }
+}
+
 template <typename Real>
 __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
   __shared__ double red[kSetupSums][kSetupThreads / 32];
   __shared__ int last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double s[kSetupSums] = {0, 0, 0, 0, INFINITY, -INFINITY};
+  double s[kSetupSums];
+#pragma unroll
+  for (int k = 0; k < kSetupSums; ++k) s[k] = sums_none(k);
   for (int i = blk * kSetupItems + threadIdx.x; i < min(C.n, (blk + 1) * kSetupItems); i += kSetupThreads) {
     const double v = C.y[i] - 1.0;
     const double d = C.dy[i];
@@ -160,6 +245,8 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     s[3] += (v * w) * (v * w);
     s[4] = fmin(s[4], w);
     s[5] = fmax(s[5], w);
+    s[6] += sqrt(fabs(v * w));
+    s[7] += sqrt(w);
   }
 #pragma unroll
   for (int k = 0; k < kSetupSums; ++k) {
@@ -181,21 +268,29 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
   __threadfence();
   if (wid < kSetupSums) {
     const int k = wid;
-    double x = k < 4 ? 0.0 : (k == 4 ? INFINITY : -INFINITY);
+    double x = sums_none(k);
     for (int b = lane; b < nblk; b += 32) x = sums_join(k, x, __ldcg(&C.sums[(size_t)b * kSetupSums + k]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = sums_join(k, x, __shfl_xor_sync(0xffffffffu, x, o));
     if (lane == 0) red[k][0] = x;
   }
   __syncthreads();
+  double sums[4] = {red[0][0], red[1][0], red[2][0], red[3][0]}, thr[2] = {INFINITY, INFINITY};
+  const double root_u = red[6][0] / C.n, root_w = red[7][0] / C.n;
+  const double typical_u = root_u * root_u, typical_w = root_w * root_w;
+  const double spread = sums[3] / typical_u / typical_u;
+  if ((spread > kSpikeSum && spread < INFINITY) || (red[5][0] > kSpikeW * typical_w && red[5][0] < INFINITY))
+    find_spikes(C, typical_u, typical_w, sums, thr);
   if (threadIdx.x == 0) {
     CurveConst cc;
-    cc.ebase = red[0][0];
-    cc.vscale = unit_scale(sqrt(red[1][0] / C.n));
-    cc.wscale = unit_scale(red[2][0] / C.n);
+    cc.ebase = sums[0];
+    cc.vscale = unit_scale(sqrt(sums[1] / C.n));
+    cc.wscale = unit_scale(sums[2] / C.n);
     cc.dscale = cc.vscale * cc.vscale * cc.wscale;
-    cc.wbar = (float)(red[2][0] * cc.wscale / C.n);
-    cc.qbar = (float)(red[3][0] * (cc.vscale * cc.wscale) * (cc.vscale * cc.wscale) / C.n);
+    cc.spike_u = thr[0] * (cc.vscale * cc.wscale);
+    cc.spike_w = thr[1] * cc.wscale;
+    cc.wbar = (float)(sums[2] * cc.wscale / C.n);
+    cc.qbar = (float)(sums[3] * (cc.vscale * cc.wscale) * (cc.vscale * cc.wscale) / C.n);
     cc.uniform = red[4][0] == red[5][0];
     *C.cst = cc;
   }

@@ -1,4 +1,5 @@
-"""Curves whose samples are far from alike, as they come: flares, a glitch.
+"""Curves whose samples are far from alike, as they come: flares, a glitch,
+uncertainties of which a few are far too small.
 The bounds must still rule out most of the starts there (the multiply-adds of
 the starts that are summed, against those of all that pass the depth
 test), and the minimum is the oracle's.
@@ -27,6 +28,13 @@ def _odd(kind, n, widths):
     if kind == "flares":
         for i in rng.integers(100, n - 200, 6):
             y[i:i + 60] += 0.5 * np.exp(-np.arange(60) / 12.0)
+    elif kind == "glitch":
+        y[n // 3] = 50.0
+    elif kind == "sure":         # one sample surer than the others, a million times their weight
+        dy[n // 3] /= 1000.0
+    elif kind == "sure_flat":    # and one of v = 0
+        dy[[n // 3, n // 2]] /= 3000.0
+        y[n // 2] = 1.0
     return t, y, dy, widths, tm, ov, maxd
 
 
@@ -47,7 +55,7 @@ def _widths(lo, hi, ratio):
     return np.unique(np.round(np.geomspace(lo, hi, int(np.log(hi / lo) / np.log(ratio)) + 1)).astype(int))
 
 
-@pytest.mark.parametrize("kind", ["flares"])
+@pytest.mark.parametrize("kind", ["flares", "glitch", "sure", "sure_flat"])
 @pytest.mark.parametrize("all_,n,widths", [
     (False, 19728, _widths(20, 1400, 1.06)),
     (False, 40000, _widths(40, 4500, 1.08)),
