@@ -153,73 +153,93 @@ __device__ __forceinline__ double unit_scale(double x) {
 // waiting starts ran over, and 300 periods of 70,000 samples with one dy
 // a thousandth of the others took 92 ms (now 1.9; clean 1.8).  Such samples, at most 2
 // kSpikeMax of a curve, are left out of the prefix sums and added to the bounds of the
-// windows that hold them.  The sums round to 2^-23 of the whole (kPrefixErr), so
-// a curve has spikes where sum u^2 is above 2^30 typical ones (a cell's u^2 then
-// rounds by 128 of them, which flares show the bounds to bear) or a weight
-// above 2^20; the typical one is the square of the mean square root, which spikes
-// hardly move.  A sample is a spike from the largest power of two (times the
-// typical |u|) on below which the sum stays within that, or from the smallest
-// that leaves at most kSpikeMax.
+// windows that hold them.  The sums round to 2^-23 of the whole (kPrefixErr), so a
+// curve has spikes where its sum of u^2 is so far above that of its samples but the largest
+// kSpikeMax that a cell's u^2 would round by 128 of their mean (flares of 50%,
+// 20 of it, cost 10% more with spikes than without), or where weights are above 2^20 typical ones.
+// A sample is a spike from the largest power of two (times the typical |u|)
+// on below which that rounding is at most 32.  Typical is the square of the mean
+// square root, which spikes hardly move; curves whose sum is below 2^30 typical
+// ones are not looked at.
 constexpr int kSpikeMax = 256;
 constexpr int kSpikes = 4 * kSpikeMax;   // of a CTA: a window may run once more around the curve
-constexpr double kSpikeSum = 0x1p30, kSpikeW = 0x1p20;
+constexpr double kSpikeSum = 0x1p30, kSpikeRest = 0x1p28, kSpikeW = 0x1p20;
 
-// The curve's thresholds of |u| and w, and its sums 1 to 3 without its spikes,
-// by one CTA (typical_u and typical_w as above).
+// The curve's thresholds of |u| and w (infinite: none), and where there are
+// any its sums 1 to 3 (kSetupSums) without its spikes, by one CTA.
 template <typename Real>
-__device__ void find_spikes(const CurveDev<Real>& C, double typical_u, double typical_w, double (&sums)[4], double* thr) {
+__device__ void find_spikes(const CurveDev<Real>& C, double typical_u, double typical_w, double (&sums)[4],
+                            double (&thr)[2]) {
   constexpr int kBins = 96, kFirst = 4;   // |u| of 2^kFirst typical ones on, by powers of two
   __shared__ int hist[kBins], heavy;
-  __shared__ double limit[2], red[3][kSetupThreads / 32];
+  __shared__ double bin_q[kBins], limit[2], red[3][kSetupThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int b = threadIdx.x; b < kBins; b += kSetupThreads) hist[b] = 0;
+  const double inv_u = 1.0 / typical_u;
+  auto sum_over = [&](double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  for (int b = threadIdx.x; b < kBins; b += kSetupThreads) {
+    hist[b] = 0;
+    bin_q[b] = 0.0;
+  }
   if (threadIdx.x == 0) heavy = 0;
   __syncthreads();
-  auto sample = [&](int i, double& v, double& w) {
-    v = C.y[i] - 1.0;
-    const double d = C.dy[i];
-    w = 1.0 / (d * d);
-  };
+  double low_q = 0.0;
+#pragma unroll 4
   for (int i = threadIdx.x; i < C.n; i += kSetupThreads) {
-    double v, w;
-    sample(i, v, w);
-    const double x = fabs(v * w) / typical_u;
-    if (x >= (double)(1 << kFirst)) atomicAdd(&hist[min(kBins - 1, ilogb(x) - kFirst)], 1);
-    if (w > kSpikeW * typical_w) atomicAdd(&heavy, 1);
+    const double2 g = __ldcg(&C.vw[i]);
+    const double u = fabs(g.x * g.y), x = u * inv_u;
+    if (x >= (double)(1 << kFirst)) {
+      const int b = min(kBins - 1, ilogb(x) - kFirst);
+      atomicAdd(&hist[b], 1);
+      atomicAdd(&bin_q[b], u * u);
+    } else {
+      low_q += u * u;
+    }
+    if (g.y > kSpikeW * typical_w) atomicAdd(&heavy, 1);
   }
+  low_q = sum_over(low_q);
+  if (lane == 0) red[0][wid] = low_q;
   __syncthreads();
   if (threadIdx.x == 0) {
+    double rest = 0.0, unit = (double)(1 << kFirst);   // unit: the least |u| of bin j, in typical ones
+    for (int q = 0; q < kSetupThreads / 32; ++q) rest += red[0][q];
     int above = 0, j = 0;
     for (int b = 0; b < kBins; ++b) above += hist[b];
-    double sum = 0.0, unit = (double)(1 << kFirst);
-    for (; j < kBins; ++j, unit *= 2.0) {   // unit: the least |u| of bin j
-      sum += 4.0 * unit * unit * hist[j];
-      if (sum > kSpikeSum && above <= kSpikeMax) break;
+    for (; above > kSpikeMax; ++j, unit *= 2.0) {
       above -= hist[j];
+      rest += bin_q[j];
     }
-    limit[0] = j < kBins ? typical_u * unit : INFINITY;
-    limit[1] = heavy <= kSpikeMax ? kSpikeW * typical_w : INFINITY;
-  }
-  __syncthreads();
-  double s[3] = {0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < C.n; i += kSetupThreads) {
-    double v, w;
-    sample(i, v, w);
-    const double u = v * w;
-    if (fabs(u) >= limit[0] || w > limit[1]) continue;
-    s[0] += v * v;
-    s[1] += w;
-    s[2] += u * u;
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
-    if (lane == 0) red[k][wid] = s[k];
+    limit[0] = INFINITY;
+    if (sums[3] * C.n > kSpikeSum * rest) {
+      double below = rest;
+      for (; j < kBins && (below + bin_q[j]) * C.n <= kSpikeRest * rest; ++j, unit *= 2.0) below += bin_q[j];
+      limit[0] = typical_u * unit;
+    }
+    limit[1] = heavy > 0 && heavy <= kSpikeMax ? kSpikeW * typical_w : INFINITY;
   }
   __syncthreads();
   thr[0] = limit[0];
   thr[1] = limit[1];
+  if (thr[0] == INFINITY && thr[1] == INFINITY) return;
+  double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int i = threadIdx.x; i < C.n; i += kSetupThreads) {
+    const double2 g = __ldcg(&C.vw[i]);
+    const double u = g.x * g.y;
+    if (fabs(u) >= thr[0] || g.y > thr[1]) continue;
+    s[0] += g.x * g.x;
+    s[1] += g.y;
+    s[2] += u * u;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    s[k] = sum_over(s[k]);
+    if (lane == 0) red[k][wid] = s[k];
+  }
+  __syncthreads();
   for (int k = 0; k < 3; ++k) {
     sums[1 + k] = 0.0;
     for (int q = 0; q < kSetupThreads / 32; ++q) sums[1 + k] += red[k][q];
@@ -262,7 +282,10 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(C.arrived, 1) == nblk - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();   // the CTA's (v, w) as well
+    last = atomicAdd(C.arrived, 1) == nblk - 1;
+  }
   __syncthreads();
   if (!last) return;
   __threadfence();
