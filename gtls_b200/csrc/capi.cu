@@ -156,13 +156,16 @@ int gtls_ctx_create(int device, gtls_ctx** out) {
   unsigned long long keep = kPoolKeep;
   e = cudaMemPoolCreate(&pool, &pp);
   if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  int* any_late = nullptr;
+  if (e == cudaSuccess) e = cudaHostAlloc(&any_late, sizeof(int), cudaHostAllocMapped);
   if (e != cudaSuccess) {
     if (pool) cudaMemPoolDestroy(pool);
-    return fail(nullptr, GTLS_E_CUDA, std::string("memory pool: ") + cudaGetErrorString(e));
+    return fail(nullptr, GTLS_E_CUDA, std::string("memory of a context: ") + cudaGetErrorString(e));
   }
   gtls_ctx* c = new gtls_ctx();
   c->device = device;
   c->pool = pool;
+  c->any_late = any_late;
   c->num_sms = prop.multiProcessorCount;
   c->smem_optin = (int)prop.sharedMemPerBlockOptin;
   *out = c;
@@ -175,6 +178,7 @@ int gtls_ctx_destroy(gtls_ctx* ctx) {
   cudaDeviceSynchronize();
   if (ctx->arena) cudaFree(ctx->arena);
   if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+  if (ctx->any_late) cudaFreeHost(ctx->any_late);
   delete ctx;
   return GTLS_OK;
 }

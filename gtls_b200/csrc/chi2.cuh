@@ -21,7 +21,6 @@ constexpr int kProbe = 16;                       // all-starts pass: first sweep
 constexpr int kList = 4096;                      // starts of a CTA that wait for their sums, main pass
 constexpr int kListAll = 8192;                   // and all-starts pass, whose starts come from blocks:
 constexpr int kBlockTable = 24576;               // blocks of a CTA's starts and durations (a multiple of three)
-constexpr int kRedo = 256;                       // tasks of a CTA that found the list full
 constexpr int kBlockStarts = 64;                 // all-starts pass: consecutive starts bounded together from their samples
 constexpr int kBlockSamples = 2048;              // samples of their windows in shared memory at a time
 constexpr int kBlockSlots = 2048;                // blocks of a CTA taken up at a time
@@ -127,8 +126,8 @@ __device__ __forceinline__ float add_spikes(CellSums& cs, const NearSpikes& s, c
   return sq;
 }
 
-// Per CTA: the list, the tasks that found it full, (all starts) the blocks, and the spikes.
-constexpr int list_entries(bool all) { return (all ? kListAll + kBlockTable / 3 : kList) + kRedo + kSpikes; }
+// Per CTA, in units of list entries: the list, (all starts) the blocks, and the spikes.
+constexpr int list_entries(bool all) { return (all ? kListAll + kBlockTable / 3 : kList) + kSpikes; }
 static_assert(sizeof(Waiting) == 3 * sizeof(int) && sizeof(Spike) == sizeof(Waiting), "");
 
 struct Chi2Args {
@@ -140,6 +139,7 @@ struct Chi2Args {
   double* part_v;           // [chunk CTAs]
   long long* part_loc;      // [chunk CTAs]
   unsigned long long* work; // NULL, or [2]: multiply-adds of the starts passing the depth test, and executed
+  int* any_late;            // set where a list ran over (host memory)
 };
 
 // Order-preserving map of a float to an int (for atomicMin).
@@ -469,7 +469,14 @@ __device__ __noinline__ void group_sums(const Exact<double>& x, const int2* whic
 // 384 threads of 80 registers and at most 110 KB, two CTAs to an SM, so that one's
 // barriers and scans overlap the other's screening (512 threads of 64
 // registers spill in the screening: 5.9 us).
-template <typename Real, bool kAll>
+//
+// A list that runs over (main pass) marks its period; what it found is not the
+// minimum then.  Such periods are searched again, by the kLate form, which works
+// the list off as it goes: after each batch and as many durations as the list holds
+// the starts of, from the former minimum as the first tau.  (With all starts of
+// the tasks that found the list full summed instead, whatever their depth and bounds, 300
+// periods of 19,728 samples of one value and uneven weights took 32 ms.)
+template <typename Real, bool kAll, bool kLate = false>
 __global__ void __launch_bounds__(kChiThreads, 2)
 chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, const int* __restrict__ order,
             Chi2Args a) {
@@ -481,7 +488,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   __shared__ unsigned char queue[kChiWarps][kTaskStarts];
   __shared__ float4 cells_sm[kChiWarps][2 * kLaneCells];
   __shared__ ScreenRow row_sm[kChiWarps][2];
-  __shared__ int list_n, tau_key, next_task, nring_sm, low_key, go_sm, redo_n, picked[2];
+  __shared__ int list_n, tau_key, next_task, nring_sm, low_key, go_sm, picked[2];
   __shared__ short pick[kChiThreads];
   __shared__ double part_s[kChiWarps];
   __shared__ int2 together[kTogether];          // union position (-1: ruled out) and start
@@ -499,6 +506,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   const int ntiles = C.ntiles;
   const int local = (cta - R.tile0) / ntiles;
   const int tix = (cta - R.tile0) - local * ntiles;
+  if (kLate && !C.late[R.pidx0 + local]) return;
   const int bidx = (int)((R.pidx0 + local) / C.batch);   // union batch of the period
   const int n = C.n;
   const int ucnt = C.union_cnt[bidx];
@@ -535,7 +543,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   Waiting* const list = a.list + (size_t)cta * list_entries(kAll);
   // all starts: the smallest lower bound (as float_key) of every block, kBlockStarts
   // starts of 2^bgroup neighbouring union positions
-  int* const btable = reinterpret_cast<int*>(list + kCap + kRedo);
+  int* const btable = reinterpret_cast<int*>(list + kCap);
   const int nblk = (k1 - k0 + kBlockStarts - 1) / kBlockStarts;
   int bgroup = 0;
   if constexpr (kAll) {
@@ -596,7 +604,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     count_tasks(0, nr, kBatch, false);
     if (lane == 0) {
       nring_sm = nr;
-      list_n = redo_n = 0;
+      list_n = 0;
       low_key = 0x7f800000;
       tau_key = 0x7f800000;   // infinity
       sent_sm = kNone;
@@ -619,6 +627,12 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   // E + delta and n are rounded to doubles: starts that close to tau stay
   const float margin = (float)((fabs(cc.ebase) + (double)n) * cc.dscale * 0x1p-44);
   const bool spiky = cc.spike_u < INFINITY || cc.spike_w < INFINITY;
+  if constexpr (kLate) {
+    if (threadIdx.x == 0) {   // (read after the next barriers)
+      const double x = (C.chi2_out[R.pidx0 + local] - cc.ebase) * cc.dscale;
+      if (x < INFINITY) tau_key = float_key(__double2float_ru(x));
+    }
+  }
   auto over_tau = [&](float lb) { return lb > key_float(*(volatile int*)&tau_key) + margin; };
 
   // (the warp's best exact value lives in red[wid]: few starts get one)
@@ -799,16 +813,6 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     else return ringV[skew(q & (kRing - 1))];
   };
 
-  // A full list: the task goes down for the sums of all its starts.  (Nothing
-  // is summed from within the screening: a call there costs it 30 registers,
-  // and 20% of its time in spills.)
-  auto redo = [&](int u, int k) {
-    if (lane == 0) {
-      const int pos = atomicAdd(&redo_n, 1);
-      if (pos < kRedo) list[kCap + pos] = Waiting{0.f, k, u};
-    }
-  };
-
   // a duration's rows and first table of cells, on their way to the warp's
   // buffers row_sm and cells_sm (.w of a cell's first half is its end)
   int row_part = 0;
@@ -863,7 +867,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       }
     }
     __syncwarp();
-    if (a.work && lane == 0 && !probe) atomicAdd(&work_sm[0], (unsigned long long)cnt * 2 * (unsigned)w);
+    if (a.work && lane == 0 && !probe && !kLate) atomicAdd(&work_sm[0], (unsigned long long)cnt * 2 * (unsigned)w);
     const float gamma = gamma_of(w);
     // the spikes that the windows may hold (the ring has samples of the last two batches)
     NearSpikes near;
@@ -949,7 +953,6 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
             const int pos = __shfl_sync(0xffffffffu, base, 0) + __popc(left & ((1u << lane) - 1u));
             const bool keep = left >> lane & 1;
             if (keep && pos < kCap) list[pos] = Waiting{certain ? lb : -INFINITY, k, u};
-            if (__any_sync(0xffffffffu, keep && pos >= kCap) && !probe) redo(u, j0 * s);
           }
           break;
         }
@@ -989,19 +992,17 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         s2.cu = warp_sum(s2.cu);
         const StartBounds sb = start_bounds<true>(s2, row2, ms, ems, __shfl_sync(0xffffffffu, qwin, src), cc.wbar,
                                                   cc.uniform, gamma, e);
-        int pos = -1;   // all of lane 0's making
-        if (lane == 0) {
+        if (lane == 0) {   // (it makes all of it)
           if (cert && sb.ub < INFINITY && float_key(sb.ub) < *(volatile int*)&tau_key)
             atomicMin(&tau_key, float_key(sb.ub));
           if (!(cert ? !over_tau(sb.lb) : !probe)) {
           } else if (kAll && !probe) {
             to_block(u, ks, cert ? sb.lb : -INFINITY);
           } else {
-            pos = atomicAdd(&list_n, 1);
+            const int pos = atomicAdd(&list_n, 1);
             if (pos < kCap) list[pos] = Waiting{cert ? sb.lb : -INFINITY, ks, u};
           }
         }
-        if (pos >= kCap && !probe) redo(u, j0 * s);
         left &= __ballot_sync(0xffffffffu, !certain || !over_tau(lb));
       }
     }
@@ -1047,6 +1048,172 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     if (spiky) run_tasks_of(coarse_tag, std::true_type{}, u_lo, cnt, t0, t1, probe);
     else run_tasks_of(coarse_tag, std::false_type{}, u_lo, cnt, t0, t1, probe);
   };
+  // The listed starts that can still be the minimum, the most promising first:
+  // those of the lowest quarter between the smallest lower bound and tau;
+  // their values then rule out most others.  The CTA's wide windows go through
+  // the rings' memory, unless that is in use.
+  auto work_off = [&](bool probe, bool ring_live) {
+    const int total = min(list_n, kCap);
+    float lo = INFINITY;
+    for (int i = threadIdx.x; i < total; i += kChiThreads)
+      if (list[i].k >= 0) lo = fminf(lo, list[i].lb);
+    const int low = __reduce_min_sync(0xffffffffu, float_key(lo));
+    if (lane == 0) atomicMin(&low_key, low);
+    __syncthreads();
+    const float first = key_float(low_key);
+    const float cut = first + 0.25f * (key_float(tau_key) - first);   // NaN or infinite: nothing is put off
+    for (int turn = 0; turn < (probe ? 1 : 2); ++turn)   // (the probe: the lowest quarter only)
+      for (int c0 = 0; c0 < total; c0 += kChiThreads) {
+        // this turn's entries of the next kChiThreads: narrow windows from the front of pick, wide from its end
+        __syncthreads();
+        if (threadIdx.x < 2) picked[threadIdx.x] = 0;
+        if (threadIdx.x == 0 && ntiles > 1) atomicMin(&tau_key, atomicMin(tau_all, *(volatile int*)&tau_key));
+        __syncthreads();
+        const int i = c0 + threadIdx.x;
+        if (i < total) {
+          const Waiting x = list[i];
+          if (x.k >= 0 && (x.lb > cut) == (turn == 1) && !over_tau(x.lb)) {
+            const bool wide = (int)(wsk[x.u] & 0xffff) > kSplitW && !(kAll && sizeof(Real) == 4) && !ring_live;
+            const int at = atomicAdd(&picked[wide], 1);
+            pick[wide ? kChiThreads - 1 - at : at] = (short)threadIdx.x;
+          }
+        }
+        __syncthreads();
+        const int nn = picked[0], nw = picked[1];
+        if constexpr (kAll && sizeof(Real) == 4) {
+          // every start's sum is one chain over its window: a lane each
+          Best best = red[wid];
+          __syncwarp();
+          const int j = threadIdx.x;
+          if (j < nn) {
+            const Waiting x = list[c0 + pick[j]];
+            const int d = dur[x.u], w = (int)(wsk[x.u] & 0xffff);
+            const Sums<float> t = chain_sums(ex.fold, x.k, w, ex.trows + ex.trow_off[d]);
+            const float inv_w = 1.f / (float)w;
+            const double delta = eval_mean<float>(best, -(float)t.S * inv_w, (float)ex.overshoot[d], t.B, t.C, 1, a.depth_min,
+                                                  cc.ebase, (double)n, (long long)x.u * n + x.k);
+            if (delta < INFINITY) atomicMin(&tau_key, float_key(__double2float_ru(delta * cc.dscale)));
+            if (a.work) atomicAdd(&work_sm[1], 2ULL * (unsigned)w);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
+            const long long l = __shfl_xor_sync(0xffffffffu, best.loc, o);
+            best_update(best, v, l);
+          }
+          if (lane == 0) red[wid] = best;
+        } else {
+          for (int j = wid; j < nn; j += kChiWarps) {   // a warp each
+            const Waiting x = list[c0 + pick[j]];
+            int go = 0;
+            if (lane == 0) go = !over_tau(x.lb);   // one lane's view of tau for the warp
+            if (__shfl_sync(0xffffffffu, go, 0)) evaluate<Real>(ex, x.u, x.k);
+          }
+          // the CTA together (a warp alone: 100,000 clocks for 10,000 samples)
+          auto entry = [&](int j) { return list[c0 + pick[kChiThreads - 1 - j]]; };
+          if constexpr (sizeof(Real) == 8) {
+            // in order of their starts, up to kTogether whose windows overlap at a time
+            if (nw > 1) {
+              int* const keys = reinterpret_cast<int*>(dyn_f);   // the rings are free by now
+              const int j = threadIdx.x;
+              const short at = pick[kChiThreads - 1 - min(j, nw - 1)];
+              __syncthreads();
+              if (j < nw) keys[j] = list[c0 + at].k;
+              __syncthreads();
+              if (j < nw) {
+                int rank = 0;
+                for (int q = 0; q < nw; ++q) rank += keys[q] < keys[j] || (keys[q] == keys[j] && q < j);
+                pick[kChiThreads - 1 - rank] = at;
+              }
+            }
+            for (int j = 0; j < nw;) {
+              __syncthreads();
+              if (wid == 0) {
+                Waiting x{0.f, 0, 0};
+                int w = 0, go = 0;
+                if (lane < kTogether && j + lane < nw) {
+                  x = entry(j + lane);
+                  w = (int)(wsk[x.u] & 0xffff);
+                  go = !over_tau(x.lb);
+                }
+                int cnt = 1, end = __shfl_sync(0xffffffffu, x.k + w, 0);
+                for (; cnt < min(kTogether, nw - j); ++cnt) {
+                  if (__shfl_sync(0xffffffffu, x.k, cnt) >= end) break;
+                  end = max(end, __shfl_sync(0xffffffffu, x.k + w, cnt));
+                }
+                if (lane < cnt) together[lane] = make_int2(go ? x.u : -1, x.k);
+                if (lane == 0) go_sm = cnt;
+              }
+              __syncthreads();
+              const int cnt = go_sm;
+              Sums<double>* const parts = reinterpret_cast<Sums<double>*>(dyn_f);
+              group_sums(ex, together, cnt, reinterpret_cast<double2*>(dyn_f + kPartWords), parts);
+              __syncthreads();
+              if (wid < cnt && together[wid].x >= 0) {
+                Sums<double> t{0.0, 0.0, 0.0};
+                for (int p = 0; p < kChiWarps; ++p) {
+                  t.S += parts[wid * kChiWarps + p].S;
+                  t.B += parts[wid * kChiWarps + p].B;
+                  t.C += parts[wid * kChiWarps + p].C;
+                }
+                settle<Real>(ex, together[wid].x, together[wid].y, t);
+              }
+              j += cnt;
+            }
+          } else {
+            for (int j = 0; j < nw; ++j) {
+              const Waiting x = entry(j);
+              const int w = (int)(wsk[x.u] & 0xffff), s = (int)(wsk[x.u] >> 16);
+              __syncthreads();
+              if (threadIdx.x == 0) go_sm = !over_tau(x.lb);
+              __syncthreads();
+              if (!go_sm) continue;
+              if (s < 32 || s > kRingWords * 2) {
+                if (wid == 0) evaluate<Real>(ex, x.u, x.k);
+                continue;
+              }
+              const R2* __restrict__ trow = ex.trows + ex.trow_off[dur[x.u]];
+              float2* const prs = reinterpret_cast<float2*>(dyn_f);
+              double S = 0.0;
+              for (int rho = threadIdx.x; rho < s; rho += kChiThreads) prs[rho] = offset_sum(ex.fold, x.k, w, s, rho, trow, S);
+              S = warp_sum(S);
+              if (lane == 0) part_s[wid] = S;
+              __syncthreads();
+              if (wid == 0) {
+                float2 acc = make_float2(0.f, 0.f);
+                for (int rho = lane; rho < s; rho += 32) add_pair(acc, prs[rho]);
+                S = 0.0;
+                for (int p = 0; p < kChiWarps; ++p) S += part_s[p];
+                settle<Real>(ex, x.u, x.k, Sums<Real>{S, (Real)warp_sum(acc.x), (Real)warp_sum(acc.y)});
+              }
+            }
+          }
+        }
+      }
+  };
+  // kLate: the end of the durations from u0 on of whose starts, one in skip of `starts` samples, the list holds all
+  auto listable = [&](int u0, int end, int starts) {
+    int u1 = u0;
+    for (int room = kCap; u1 < end; ++u1) {
+      room -= starts / (int)(wsk[u1] >> 16) + 1;
+      if (room < 0 && u1 > u0) break;
+    }
+    return u1;
+  };
+  auto run_and_work_off = [&](auto coarse_tag, int u0, int u1, int t0, int t1) {
+    __syncthreads();   // task_pre and the list are free
+    if (wid == 0) count_tasks(u0, u1, t1 - t0, false);
+    if (threadIdx.x == 0) {
+      next_task = 0;
+      list_n = 0;
+      low_key = 0x7f800000;
+    }
+    __syncthreads();
+    run_tasks(coarse_tag, u0, u1 - u0, t0, t1, false);
+    __syncthreads();
+    work_off(false, !decltype(coarse_tag)::value);
+  };
   for (int sweep = kAll ? 0 : 1; sweep < 2; ++sweep) {
     const bool probe = sweep == 0;
     if (kAll) {
@@ -1065,7 +1232,15 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     fetch(min(kBatch, need - ld));
     for (int t0 = k0; t0 < k1; t0 += kBatch) {
       store();
-      run_tasks(std::false_type{}, 0, nring, t0, min(k1, t0 + kBatch), probe);
+      const int t1 = min(k1, t0 + kBatch);
+      if constexpr (kLate) {
+        for (int u0 = 0, u1; u0 < nring; u0 = u1) {
+          u1 = listable(u0, nring, kBatch);
+          run_and_work_off(std::false_type{}, u0, u1, t0, t1);
+        }
+      } else {
+        run_tasks(std::false_type{}, 0, nring, t0, t1, probe);
+      }
       fetch(min(kBatch, need - ld));
       __syncthreads();
     }
@@ -1074,12 +1249,28 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         store();
         fetch(min(kBatch, need - ld));
       }
-      __syncthreads();   // next_task is 0, and task_pre free
-      if (wid == 0) count_tasks(nring, ucnt, k1 - k0, probe);
-      if (threadIdx.x == 0) next_task = 0;
-      __syncthreads();
-      run_tasks(std::true_type{}, nring, ucnt - nring, k0, k1, probe);
-      __syncthreads();
+      if constexpr (kLate) {
+        for (int u0 = nring, u1; u0 < ucnt; u0 = u1) {
+          u1 = listable(u0, ucnt, k1 - k0);
+          // (a single duration's starts may be more than the list holds)
+          const long long part = u1 > u0 + 1 ? k1 - k0 : (long long)(kCap - 1) * (int)(wsk[u0] >> 16);
+          for (long long t0 = k0; t0 < k1; t0 += part)
+            run_and_work_off(std::true_type{}, u0, u1, (int)t0, (int)min((long long)k1, t0 + part));
+        }
+      } else {
+        __syncthreads();   // next_task is 0, and task_pre free
+        if (wid == 0) count_tasks(nring, ucnt, k1 - k0, probe);
+        if (threadIdx.x == 0) next_task = 0;
+        __syncthreads();
+        run_tasks(std::true_type{}, nring, ucnt - nring, k0, k1, probe);
+        __syncthreads();
+      }
+    }
+    if constexpr (!kAll && !kLate) {
+      if (threadIdx.x == 0 && list_n > kCap) {   // C.late was 0
+        C.late[R.pidx0 + local] = 1;
+        *a.any_late = 1;
+      }
     }
     if (threadIdx.x == 0 && !probe) {
       long long sent = sent_sm;
@@ -1290,155 +1481,8 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         __syncthreads();
       }
     }
-    // the listed starts that can still be the minimum, the most promising first:
-    // those of the lowest quarter between the smallest lower bound and tau;
-    // their values then rule out most others
-    const int total = min(list_n, kCap);
-    float lo = INFINITY;
-    for (int i = threadIdx.x; i < total; i += kChiThreads)
-      if (list[i].k >= 0) lo = fminf(lo, list[i].lb);
-    const int low = __reduce_min_sync(0xffffffffu, float_key(lo));
-    if (lane == 0) atomicMin(&low_key, low);
-    __syncthreads();
-    const float first = key_float(low_key);
-    const float cut = first + 0.25f * (key_float(tau_key) - first);   // NaN or infinite: nothing is put off
-    for (int turn = 0; turn < (probe ? 1 : 2); ++turn)   // (the probe: the lowest quarter only)
-      for (int c0 = 0; c0 < total; c0 += kChiThreads) {
-        // this turn's entries of the next kChiThreads: narrow windows from the front of pick, wide from its end
-        __syncthreads();
-        if (threadIdx.x < 2) picked[threadIdx.x] = 0;
-        if (threadIdx.x == 0 && ntiles > 1) atomicMin(&tau_key, atomicMin(tau_all, *(volatile int*)&tau_key));
-        __syncthreads();
-        const int i = c0 + threadIdx.x;
-        if (i < total) {
-          const Waiting x = list[i];
-          if (x.k >= 0 && (x.lb > cut) == (turn == 1) && !over_tau(x.lb)) {
-            const bool wide = (int)(wsk[x.u] & 0xffff) > kSplitW && !(kAll && sizeof(Real) == 4);
-            const int at = atomicAdd(&picked[wide], 1);
-            pick[wide ? kChiThreads - 1 - at : at] = (short)threadIdx.x;
-          }
-        }
-        __syncthreads();
-        const int nn = picked[0], nw = picked[1];
-        if constexpr (kAll && sizeof(Real) == 4) {
-          // every start's sum is one chain over its window: a lane each
-          Best best = red[wid];
-          __syncwarp();
-          const int j = threadIdx.x;
-          if (j < nn) {
-            const Waiting x = list[c0 + pick[j]];
-            const int d = dur[x.u], w = (int)(wsk[x.u] & 0xffff);
-            const Sums<float> t = chain_sums(ex.fold, x.k, w, ex.trows + ex.trow_off[d]);
-            const float inv_w = 1.f / (float)w;
-            const double delta = eval_mean<float>(best, -(float)t.S * inv_w, (float)ex.overshoot[d], t.B, t.C, 1, a.depth_min,
-                                                  cc.ebase, (double)n, (long long)x.u * n + x.k);
-            if (delta < INFINITY) atomicMin(&tau_key, float_key(__double2float_ru(delta * cc.dscale)));
-            if (a.work) atomicAdd(&work_sm[1], 2ULL * (unsigned)w);
-          }
-          __syncwarp();
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            const double v = __shfl_xor_sync(0xffffffffu, best.v, o);
-            const long long l = __shfl_xor_sync(0xffffffffu, best.loc, o);
-            best_update(best, v, l);
-          }
-          if (lane == 0) red[wid] = best;
-        } else {
-          for (int j = wid; j < nn; j += kChiWarps) {   // a warp each
-            const Waiting x = list[c0 + pick[j]];
-            int go = 0;
-            if (lane == 0) go = !over_tau(x.lb);   // one lane's view of tau for the warp
-            if (__shfl_sync(0xffffffffu, go, 0)) evaluate<Real>(ex, x.u, x.k);
-          }
-          // the CTA together (a warp alone: 100,000 clocks for 10,000 samples)
-          auto entry = [&](int j) { return list[c0 + pick[kChiThreads - 1 - j]]; };
-          if constexpr (sizeof(Real) == 8) {
-            // in order of their starts, up to kTogether whose windows overlap at a time
-            if (nw > 1) {
-              int* const keys = reinterpret_cast<int*>(dyn_f);   // the rings are free by now
-              const int j = threadIdx.x;
-              const short at = pick[kChiThreads - 1 - min(j, nw - 1)];
-              __syncthreads();
-              if (j < nw) keys[j] = list[c0 + at].k;
-              __syncthreads();
-              if (j < nw) {
-                int rank = 0;
-                for (int q = 0; q < nw; ++q) rank += keys[q] < keys[j] || (keys[q] == keys[j] && q < j);
-                pick[kChiThreads - 1 - rank] = at;
-              }
-            }
-            for (int j = 0; j < nw;) {
-              __syncthreads();
-              if (wid == 0) {
-                Waiting x{0.f, 0, 0};
-                int w = 0, go = 0;
-                if (lane < kTogether && j + lane < nw) {
-                  x = entry(j + lane);
-                  w = (int)(wsk[x.u] & 0xffff);
-                  go = !over_tau(x.lb);
-                }
-                int cnt = 1, end = __shfl_sync(0xffffffffu, x.k + w, 0);
-                for (; cnt < min(kTogether, nw - j); ++cnt) {
-                  if (__shfl_sync(0xffffffffu, x.k, cnt) >= end) break;
-                  end = max(end, __shfl_sync(0xffffffffu, x.k + w, cnt));
-                }
-                if (lane < cnt) together[lane] = make_int2(go ? x.u : -1, x.k);
-                if (lane == 0) go_sm = cnt;
-              }
-              __syncthreads();
-              const int cnt = go_sm;
-              Sums<double>* const parts = reinterpret_cast<Sums<double>*>(dyn_f);
-              group_sums(ex, together, cnt, reinterpret_cast<double2*>(dyn_f + kPartWords), parts);
-              __syncthreads();
-              if (wid < cnt && together[wid].x >= 0) {
-                Sums<double> t{0.0, 0.0, 0.0};
-                for (int p = 0; p < kChiWarps; ++p) {
-                  t.S += parts[wid * kChiWarps + p].S;
-                  t.B += parts[wid * kChiWarps + p].B;
-                  t.C += parts[wid * kChiWarps + p].C;
-                }
-                settle<Real>(ex, together[wid].x, together[wid].y, t);
-              }
-              j += cnt;
-            }
-          } else {
-            for (int j = 0; j < nw; ++j) {
-              const Waiting x = entry(j);
-              const int w = (int)(wsk[x.u] & 0xffff), s = (int)(wsk[x.u] >> 16);
-              __syncthreads();
-              if (threadIdx.x == 0) go_sm = !over_tau(x.lb);
-              __syncthreads();
-              if (!go_sm) continue;
-              if (s < 32 || s > kRingWords * 2) {
-                if (wid == 0) evaluate<Real>(ex, x.u, x.k);
-                continue;
-              }
-              const R2* __restrict__ trow = ex.trows + ex.trow_off[dur[x.u]];
-              float2* const prs = reinterpret_cast<float2*>(dyn_f);
-              double S = 0.0;
-              for (int rho = threadIdx.x; rho < s; rho += kChiThreads) prs[rho] = offset_sum(ex.fold, x.k, w, s, rho, trow, S);
-              S = warp_sum(S);
-              if (lane == 0) part_s[wid] = S;
-              __syncthreads();
-              if (wid == 0) {
-                float2 acc = make_float2(0.f, 0.f);
-                for (int rho = lane; rho < s; rho += 32) add_pair(acc, prs[rho]);
-                S = 0.0;
-                for (int p = 0; p < kChiWarps; ++p) S += part_s[p];
-                settle<Real>(ex, x.u, x.k, Sums<Real>{S, (Real)warp_sum(acc.x), (Real)warp_sum(acc.y)});
-              }
-            }
-          }
-        }
-      }
-    if (!kAll && redo_n > 0) {   // the list was full: every start of the tasks that found it so (of all, if those are too many)
-      const bool every = redo_n > kRedo;
-      for (int t = 0; t < (every ? ucnt : redo_n); ++t) {
-        const int u = every ? t : list[kCap + t].u;
-        const int s = (int)(wsk[u] >> 16), from = every ? (k0 + s - 1) / s * s : list[kCap + t].k;
-        const int to = every ? k1 : min(k1, from + kTaskStarts * s);
-        for (int k = from + wid * s; k < to; k += kChiWarps * s) evaluate<Real>(ex, u, k);
-      }
+    if constexpr (!kLate) {
+      work_off(probe, false);
     }
     if (kAll && probe) {
       __syncthreads();

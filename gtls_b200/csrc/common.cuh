@@ -26,6 +26,7 @@ struct gtls_ctx {
   int tile_cap_fp64 = gtls::kTileCapFp64;
   int bucket_shift = 0;
   int records_global = 0;      // accepted and reported; the records are always read through L2
+  int* any_late = nullptr;     // host memory the search kernels write: a list of starts ran over
   bool smem_set_fp32 = false, smem_set_fp64 = false;   // the search kernels' shared memory has been allowed
 };
 

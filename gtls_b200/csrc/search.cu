@@ -78,6 +78,7 @@ struct CurveDev {
   const double* periods;        // [np] this curve's trial periods
   double* chi2_out;             // [np]
   int64_t* loc_out;             // [np] or NULL
+  int* late;                    // [np] 1: a list ran over, the period is searched again (scratch)
   double2* vw;                  // [n] (v, w) per original sample (scratch)
   CurveConst* cst;              // sums over the curve (scratch)
   double* sums;                 // [setup blocks * kSetupSums] their parts (scratch)
@@ -776,7 +777,8 @@ __device__ __noinline__ bool prepare_rounds(int* dyn, int* wtmp_i, int* big, int
 template <typename Real, int kThreads = kPrepThreads>
 __global__ void __launch_bounds__(kThreads, kPrepThreads / kThreads)
 prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, int nruns,
-               uint2* __restrict__ scr_slot, int* __restrict__ order, int* __restrict__ tau = nullptr) {
+               uint2* __restrict__ scr_slot, int* __restrict__ order, int* __restrict__ tau = nullptr,
+               bool late = false) {
   extern __shared__ int hist[];
   __shared__ int wtmp_i[32];
   __shared__ int big[kBigBuckets];
@@ -787,6 +789,8 @@ prepare_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ r
   const Run& R = runs[ri];
   const CurveDev<Real>& C = cds[R.curve];
   const int local = item - R.item0;
+  if (late && !C.late[R.pidx0 + local]) return;   // only the periods whose lists ran over
+  if (tau && !late && threadIdx.x == 0) C.late[R.pidx0 + local] = 0;
   const double* __restrict__ t = C.t;
   const int n = C.n;
   const int nb_log2 = C.nb_log2;
@@ -920,7 +924,8 @@ namespace gtls {
 
 template <typename Real>
 __global__ void finish_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs, int nruns,
-                              int count, const double* __restrict__ part_v, const long long* __restrict__ part_loc) {
+                              int count, const double* __restrict__ part_v, const long long* __restrict__ part_loc,
+                              bool late) {
   const int item = blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= count) return;
   const int ri = upper_find(0, nruns, item, [&](int i) { return (long long)runs[i].item0; });
@@ -929,6 +934,7 @@ __global__ void finish_kernel(const CurveDev<Real>* __restrict__ cds, const Run*
   if (C.ntiles == 1) return;   // written by the chi2 kernel
   const int local = item - R.item0;
   const long long pg = R.pidx0 + local;
+  if (late && !C.late[pg]) return;
   Best b{INFINITY, 0x7fffffffffffffffLL};
   if (C.union_cnt[pg / C.batch] == 0) {
     b.v = NAN;
@@ -1225,6 +1231,7 @@ static cudaError_t allow_smem(int optin) {
   set(prepare_kernel<Real>, optin - kPrepStaticSmem);
   set(prepare_kernel<Real, kPrepThreadsSmall>, optin - kPrepStaticSmem);
   set(chi2_kernel<Real, false>, chi);
+  set(chi2_kernel<Real, false, true>, chi);
   set(chi2_kernel<Real, true>, chi);
   return e;
 }
@@ -1478,6 +1485,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     carve_size<double>(total, (size_t)(blk_off[c + 1] - blk_off[c]) * kSetupSums);
     carve_size<int>(total, (size_t)C.nbatch);
     carve_size<int>(total, (size_t)C.nbatch * C.D);
+    carve_size<int>(total, (size_t)C.np);
   }
   carve_size<R2>(total, row_off[n_curves]);
   carve_size<ScreenCell>(total, ends.size());
@@ -1503,6 +1511,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
     C.arrived = reinterpret_cast<int*>(base + at_arrived) + c;
     C.union_cnt = cv.take<int>(C.nbatch);
     C.union_list = cv.take<int>((size_t)C.nbatch * C.D);
+    C.late = cv.take<int>((size_t)C.np);
     C.skips = reinterpret_cast<const int*>(base + at_skips) + d_off[c];
     C.trow_off = reinterpret_cast<const int*>(base + at_trow) + d_off[c];
     C.sends = reinterpret_cast<const int*>(base + at_ends) + cell_off[c];
@@ -1558,39 +1567,50 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
   ca.part_v = part_v;
   ca.part_loc = part_loc;
   ca.work = tm ? work : nullptr;
-  for (int k = 0; k < nchunks; ++k) {
-    const int r0 = chunk_r0[k], nr = chunk_r0[k + 1] - r0;
-    const int items = chunk_items[k], tiles = chunk_tiles[k];
-    cudaEvent_t e3[4];
-    if (tm) {
-      for (auto& e : e3) GTLS_TRY_CUDA(ctx, cudaEventCreate(&e));
-      GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[0], st));
+  ca.any_late = ctx->any_late;
+  *ctx->any_late = 0;
+  auto run_chunks = [&](bool late) -> int {
+    for (int k = 0; k < nchunks; ++k) {
+      const int r0 = chunk_r0[k], nr = chunk_r0[k + 1] - r0;
+      const int items = chunk_items[k], tiles = chunk_tiles[k];
+      cudaEvent_t e3[4];
+      if (tm) {
+        for (auto& e : e3) GTLS_TRY_CUDA(ctx, cudaEventCreate(&e));
+        GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[0], st));
+      }
+      if (chunk_small[k])
+        prepare_kernel<Real, kPrepThreadsSmall><<<items, kPrepThreadsSmall, chunk_smem_prep[k], st>>>(
+            d_cd, d_runs + r0, nr, scr_slot, order, tau, late);
+      else
+        prepare_kernel<Real><<<items, kPrepThreads, chunk_smem_prep[k], st>>>(d_cd, d_runs + r0, nr, scr_slot, order,
+                                                                               tau, late);
+      if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[1], st));
+      ca.nruns = nr;
+      if (all)
+        chi2_kernel<Real, true><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
+      else if (late)
+        chi2_kernel<Real, false, true><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
+      else
+        chi2_kernel<Real, false><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
+      if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[2], st));
+      if (tiles > items) {   // some periods are split
+        finish_kernel<Real><<<(items + 127) / 128, 128, 0, st>>>(d_cd, d_runs + r0, nr, items, part_v, part_loc,
+                                                                late);
+        ctx->launches += 1;
+      }
+      if (tm) {
+        GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[3], st));
+        for (auto& e : e3) evc.push_back(e);
+      }
+      ctx->launches += 2;
+      GTLS_TRY_CUDA(ctx, cudaGetLastError());
     }
-    if (chunk_small[k])
-      prepare_kernel<Real, kPrepThreadsSmall><<<items, kPrepThreadsSmall, chunk_smem_prep[k], st>>>(
-          d_cd, d_runs + r0, nr, scr_slot, order, tau);
-    else
-      prepare_kernel<Real><<<items, kPrepThreads, chunk_smem_prep[k], st>>>(d_cd, d_runs + r0, nr, scr_slot, order,
-                                                                             tau);
-    if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[1], st));
-    ca.nruns = nr;
-    if (all)
-      chi2_kernel<Real, true><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
-    else
-      chi2_kernel<Real, false><<<tiles, kChiThreads, chunk_smem_chi[k], st>>>(d_cd, d_runs + r0, order, ca);
-    if (tm) GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[2], st));
-    if (tiles > items) {   // some periods are split
-      finish_kernel<Real><<<(items + 127) / 128, 128, 0, st>>>(d_cd, d_runs + r0, nr, items, part_v, part_loc);
-      ctx->launches += 1;
-    }
-    if (tm) {
-      GTLS_TRY_CUDA(ctx, cudaEventRecord(e3[3], st));
-      for (auto& e : e3) evc.push_back(e);
-    }
-    ctx->launches += 2;
-    GTLS_TRY_CUDA(ctx, cudaGetLastError());
-  }
-  GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
+    GTLS_TRY_CUDA(ctx, cudaStreamSynchronize(st));
+    return GTLS_OK;
+  };
+  int rc = run_chunks(false);
+  if (rc == GTLS_OK && *static_cast<volatile int*>(ctx->any_late)) rc = run_chunks(true);   // the marked periods alone
+  if (rc != GTLS_OK) return rc;
   if (tm) {
     float ms = 0;
     GTLS_TRY_CUDA(ctx, cudaEventElapsedTime(&ms, ev[0], ev[1]));
@@ -1603,7 +1623,7 @@ static int run_search(gtls_ctx* ctx, const CurveHost* ch, int n_curves, int prec
       GTLS_TRY_CUDA(ctx, cudaEventElapsedTime(&ms, evc[i + 2], evc[i + 3]));
       tm->finish_ms += ms;
     }
-    tm->chunks = (int)(evc.size() / 4);
+    tm->chunks = nchunks;
     for (auto e : evc) cudaEventDestroy(e);
     for (auto e : ev) cudaEventDestroy(e);
     // work counters of the chi2 kernel, from the unions the kernel used

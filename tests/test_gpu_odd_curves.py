@@ -35,6 +35,11 @@ def _odd(kind, n, widths):
     elif kind == "sure_flat":    # and one of v = 0
         dy[[n // 3, n // 2]] /= 3000.0
         y[n // 2] = 1.0
+    elif kind == "glitches":     # more than are left out of the prefix sums, up to 400 times the flux
+        y[rng.integers(0, n, 700)] *= np.exp(rng.uniform(0.0, 6.0, 700))
+    elif kind == "ties":         # every start of a duration has the same value
+        y[:] = 1.0 - 1e-3
+        dy[:] = 1e-3
     return t, y, dy, widths, tm, ov, maxd
 
 
@@ -73,3 +78,21 @@ def test_most_starts_are_ruled_out(cuda, kind, all_, n, widths):
         if precision == "fp64":
             np.testing.assert_array_equal(loc[CHECKED], [r[1] for r in ref])
         assert tm_.chi2_issued_fma <= 0.1 * tm_.chi2_active_fma, (precision, tm_.as_dict())
+
+
+@pytest.mark.parametrize("kind", ["ties", "glitches"])
+@pytest.mark.parametrize("n,widths", [(19728, _widths(20, 1400, 1.06)), (40000, _widths(40, 4500, 1.08))])
+def test_what_the_list_cannot_hold_is_summed_once_at_most(cuda, kind, n, widths):
+    """Where the list of a CTA runs over: starts that all tie (the widest duration
+    rules out the others in the end) and more glitches than are set apart.  Not
+    more is summed than starts that pass."""
+    c = _odd(kind, n, widths)
+    t, y, dy, widths, tm, ov, maxd = c
+    back = O.NumpyBackend()
+    ref = [back.main_pass(t, y, dy, p, widths, tm, ov, maxd, 1e-5, 8) for p in PERIODS[CHECKED]]
+    for precision, rtol in (("fp64", 1e-9), ("fp32", 2e-6)):
+        chi2, loc, tm_ = _run(c, False, precision)
+        np.testing.assert_allclose(chi2[CHECKED], [r[0] for r in ref], rtol=rtol)
+        if precision == "fp64" and kind != "ties":
+            np.testing.assert_array_equal(loc[CHECKED], [r[1] for r in ref])
+        assert tm_.chi2_issued_fma <= (0.1 if kind == "ties" else 1.0) * tm_.chi2_active_fma, (precision, tm_.as_dict())
