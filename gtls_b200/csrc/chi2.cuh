@@ -625,7 +625,11 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   const int nring = nring_sm;
   const float dthr = (float)(a.depth_min * cc.vscale);
   // E + delta and n are rounded to doubles: starts that close to tau stay
-  const float margin = (float)((fabs(cc.ebase) + (double)n) * cc.dscale * 0x1p-44);
+  // (Without a finite E no start that passes has a finite value: none is listed,
+  // and n, where a start fails, is the minimum.)
+  const bool no_value = cc.kind >= kNoValue;
+  const float margin = no_value ? 0.f : (float)((fabs(cc.ebase) + (double)n) * cc.dscale * 0x1p-44);
+  if (no_value && threadIdx.x == 0) tau_key = 0;   // (read after the next barriers)
   const bool spiky = cc.spike_u < INFINITY || cc.spike_w < INFINITY;
   if constexpr (kLate) {
     if (threadIdx.x == 0) {   // (read after the next barriers)
@@ -873,7 +877,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     NearSpikes near;
     if constexpr (kSpiky) {
       const int from = kCoarse ? 0 : spike_end[(batches - 2) & 3];
-      near = near_spikes(spikes, from, spike_end[batches & 3], cc.uniform);
+      near = near_spikes(spikes, from, spike_end[batches & 3], cc.kind & kUniform);
     }
     for (int b = 0; b < cnt; b += 32) {
       const int k = (j0 + queue[wid][min(b + lane, cnt - 1)]) * s;
@@ -903,9 +907,10 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       const float em = fmaf(3e-7f, fabsf(m), em0);
       float qwin = (pq - q00) + (float)(kCoarse ? end * g : w) * cc.qbar + 4.f * e.n2;
       if constexpr (kSpiky) qwin += add_spikes(cs, near, ex.trows + ex.trow_off[d], q, w);
-      float lb = start_bounds<false>(cs, row_sm[wid][0], m, em, qwin, cc.wbar, cc.uniform, gamma, e).lb;
+      float lb = start_bounds<false>(cs, row_sm[wid][0], m, em, qwin, cc.wbar, cc.kind & kUniform, gamma, e).lb;
       // too close to the depth threshold to tell: such a start needs its exact value (n, if it fails)
       const bool certain = m - em > dthr;
+      if (cc.kind >= kNoValue && certain) lb = INFINITY;
       unsigned left = __ballot_sync(0xffffffffu, b + lane < cnt && (!certain || !over_tau(lb)));
       // the starts that are left.  Many (the neighbours of a peak in the
       // all-starts pass, the first ones of a range): the second table for all
@@ -938,7 +943,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           cells_sm[wid][lane] = reinterpret_cast<const float4*>(scells + (size_t)d * kLaneCells)[lane];
           __syncwarp();
           if constexpr (kSpiky) add_spikes(s2, near, ex.trows + ex.trow_off[d], q, w);
-          const StartBounds sb = start_bounds<true>(s2, row_sm[wid][1], m, em, qwin, cc.wbar, cc.uniform, gamma, e);
+          const StartBounds sb = start_bounds<true>(s2, row_sm[wid][1], m, em, qwin, cc.wbar, cc.kind & kUniform, gamma, e);
           lb = sb.lb;
           const bool on = left >> lane & 1;
           const int ub = __reduce_min_sync(0xffffffffu, on && certain && sb.ub < INFINITY ? float_key(sb.ub) : 0x7f800000);
@@ -991,7 +996,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         s2.cl = warp_sum(s2.cl);
         s2.cu = warp_sum(s2.cu);
         const StartBounds sb = start_bounds<true>(s2, row2, ms, ems, __shfl_sync(0xffffffffu, qwin, src), cc.wbar,
-                                                  cc.uniform, gamma, e);
+                                                  cc.kind & kUniform, gamma, e);
         if (lane == 0) {   // (it makes all of it)
           if (cert && sb.ub < INFINITY && float_key(sb.ub) < *(volatile int*)&tau_key)
             atomicMin(&tau_key, float_key(sb.ub));
@@ -1490,6 +1495,20 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         list_n = 0;
         low_key = 0x7f800000;
       }
+    }
+  }
+  __syncthreads();
+  if (no_value && cc.ebase > 0.0 && sent_sm == kNone) {
+    // E is infinite and all starts pass: the first whose sums are finite is
+    // infinite.  Where the narrowest windows have none, with an infinite weight in
+    // each, those that hold one of them whole have none either.
+    const int w0 = (int)(wsk[0] & 0xffff), s0 = kAll ? 1 : (int)(wsk[0] >> 16);
+    for (int u = 0; u < ucnt && (int)(wsk[u] & 0xffff) < w0 + s0; ++u) {
+      const int s = kAll ? 1 : (int)(wsk[u] >> 16);
+      for (int k = (k0 + s - 1) / s * s + wid * s; k < k1 && red[wid].loc == kNone; k += kChiWarps * s)
+        evaluate<Real>(ex, u, k);
+      int found = red[wid].loc != kNone;
+      if (__syncthreads_or(found)) break;
     }
   }
   __syncthreads();

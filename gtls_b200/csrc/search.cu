@@ -64,9 +64,10 @@ struct CurveConst {
   double vscale, wscale, dscale;
   double spike_u, spike_w; // samples of larger |u| or w (scaled) are spikes; infinite: none
   float wbar, qbar;        // mean of the scaled w and u^2, of samples that are no spikes
-  int uniform;             // all weights equal
+  int kind;                // kUniform: all weights equal; kNoValue or more: E is not finite
   int pad;
 };
+constexpr int kUniform = 1, kNoValue = 2;
 
 // Per-light-curve parameters and buffers on the device.  A search covers one
 // or many light curves; every kernel finds its curve through these.
@@ -315,7 +316,7 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     cc.spike_w = thr[1] * cc.wscale;
     cc.wbar = (float)(sums[2] * cc.wscale / C.n);
     cc.qbar = (float)(sums[3] * (cc.vscale * cc.wscale) * (cc.vscale * cc.wscale) / C.n);
-    cc.uniform = red[4][0] == red[5][0];
+    cc.kind = (red[4][0] == red[5][0] ? kUniform : 0) | (fabs(sums[0]) < INFINITY ? 0 : kNoValue);
     *C.cst = cc;
   }
 }
