@@ -683,10 +683,6 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const int cnt = fetched;
     const int q0 = ld + (int)threadIdx.x * kItems;   // item i is prefix value q0 + i + 1
     const int have = min(kItems, cnt - (int)threadIdx.x * kItems);
-    const int* __restrict__ ord = ex.fold.order;
-    const double2* __restrict__ vw = ex.fold.vw;
-    if (k0 + q0 + kBatch < n)   // the next batch's indices: into L2
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(ord + k0 + q0 + kBatch));
     ++batches;
     if (spiky) {   // listed in order; their u and w are 0 in what follows
       int mine = 0;
@@ -712,25 +708,25 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         }
       if (threadIdx.x == kChiThreads - 1) spike_end[batches & 3] = at;
     }
-    // u, w - wbar and u^2 - qbar of an item, scaled in FP64 (a weight itself may be beyond FP32)
-    auto item = [&](int i, double& v, double& u, double& w, double& q) {
+    // v, u and w of an item, scaled in FP64 (a weight itself may be beyond FP32); 0 past the end
+    auto item = [&](int i, double& v, double& u, double& w) {
       v = gq[i].x * cc.vscale;
       w = gq[i].y * cc.wscale;
       u = v * w;
-      q = fma(u, u, -(double)cc.qbar);
-      w -= (double)cc.wbar;
-      if (i >= have) w = q = 0.0;
     };
+    const double qbar = cc.qbar, wbar = cc.wbar;
     double sv = 0.0, su = 0.0, sw = 0.0, sq = 0.0;
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
-      double v, u, w, q;
-      item(i, v, u, w, q);
+      double v, u, w;
+      item(i, v, u, w);
       sv += v;
       su += u;
       sw += w;
-      sq += q;
+      sq = fma(u, u, sq);
     }
+    sw = fma((double)-max(have, 0), wbar, sw);
+    sq = fma((double)-max(have, 0), qbar, sq);
     double xv = sv, xu = su, xw = sw, xq = sq;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -754,11 +750,16 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       next_task = 0;
       if (ntiles > 1) atomicMin(&tau_key, atomicMin(tau_all, *(volatile int*)&tau_key));
     }
-    const bool before = lane < wid;   // kChiWarps <= 32
-    double rv = carry[0] + warp_sum(before ? wtot[lane][0] : 0.0) + (xv - sv);
-    double ru = carry[1] + warp_sum(before ? wtot[lane][1] : 0.0) + (xu - su);
-    double rw = carry[2] + warp_sum(before ? wtot[lane][2] : 0.0) + (xw - sw);
-    double rq = carry[3] + warp_sum(before ? wtot[lane][3] : 0.0) + (xq - sq);
+    // lane 8 f + j adds up field f of warps j and j + 8 before this one; three steps and a broadcast for all four
+    static_assert(kChiWarps <= 16, "");
+    double sum = ((lane & 7) < wid ? wtot[lane & 7][lane >> 3] : 0.0) +
+                 ((lane & 7) + 8 < wid ? wtot[(lane & 7) + 8][lane >> 3] : 0.0);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    double rv = carry[0] + __shfl_sync(0xffffffffu, sum, 0) + (xv - sv);
+    double ru = carry[1] + __shfl_sync(0xffffffffu, sum, 8) + (xu - su);
+    double rw = carry[2] + __shfl_sync(0xffffffffu, sum, 16) + (xw - sw);
+    double rq = carry[3] + __shfl_sync(0xffffffffu, sum, 24) + (xq - sq);
     float mv = 0.f, mu = 0.f, mw = 0.f, mq = 0.f;
     int cq = 0, cr = 1;   // next coarse step and the items up to it
     if (g > 0) {
@@ -768,12 +769,12 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
 #pragma unroll
     for (int i = 0; i < kItems; ++i) {
       if (i < have) {
-        double v, u, w, q;
-        item(i, v, u, w, q);
+        double v, u, w;
+        item(i, v, u, w);
         rv += v;
         ru += u;
-        rw += w;
-        rq += q;
+        rw += w - wbar;
+        rq += fma(u, u, -qbar);
         const float fv = (float)rv, fu = (float)ru, fw = (float)rw, fq = (float)rq;
         mv = fmaxf(mv, fabsf(fv));
         mu = fmaxf(mu, fabsf(fu));
