@@ -559,8 +559,14 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
   }
   Spike* const spikes = reinterpret_cast<Spike*>(list + list_entries(kAll) - kSpikes);
   int* const tau_all = a.tau + (R.item0 + local);
-  // FP32 exact sums round by up to (w + 8) half ulps of their absolute sum
-  auto gamma_of = [&](int w) { return kGammaF + (sizeof(Real) == 4 ? (float)(w + 8) * 1.2e-7f : 0.f); };
+  // FP32 exact sums: a term takes part in as many roundings, of half an ulp of the
+  // absolute sum each, as its offset's run has terms, the offsets' sums are added up
+  // in steps and its factors were rounded (window_sums; every start: one run)
+  auto gamma_of = [&](int w, int s) {
+    if (sizeof(Real) == 8) return kGammaF;
+    const int steps = s >= 32 ? (s + 31) / 32 + 5 : s;
+    return kGammaF + (float)((w + s - 1) / s + steps + 6) * 6e-8f;
+  };
   constexpr long long kNone = 0x7fffffffffffffffLL;
 
   // tasks of one batch (of the whole range for the coarse widths) per union
@@ -873,7 +879,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     }
     __syncwarp();
     if (a.work && lane == 0 && !probe && !kLate) atomicAdd(&work_sm[0], (unsigned long long)cnt * 2 * (unsigned)w);
-    const float gamma = gamma_of(w);
+    const float gamma = gamma_of(w, kAll ? 1 : (int)(wsk[u] >> 16));
     // the spikes that the windows may hold (the ring has samples of the last two batches)
     NearSpikes near;
     if constexpr (kSpiky) {
@@ -1414,7 +1420,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
               const float m = -x[3] * row.inv_w;
               const float em = (roundf * x[4]) * row.inv_w + 4e-7f * fabsf(m) + 2e-7f * fabsf(dthr);
               const StartBounds sb = start_bounds<true>(cs, row, m, em, x[2] * (1.f + 2.f * roundf), 0.f, false,
-                                                        gamma_of(w) + roundf, ScreenErr{0.f, 0.f, 0.f, 0.f});
+                                                        gamma_of(w, 1) + roundf, ScreenErr{0.f, 0.f, 0.f, 0.f});
               // (a start that only its samples settle carries n like those that the screening settles)
               const bool fails = m + em <= dthr, mine = k < k1 && !fails, certain = m - em > dthr;
               if (k < k1 && fails) atomicMin(&sent_sm, (long long)u * n + k);
