@@ -43,13 +43,13 @@ def _odd(kind, n, widths):
     return t, y, dy, widths, tm, ov, maxd
 
 
-def _run(c, all_, precision):
+def _run(c, all_, precision, periods=PERIODS):
     import torch
     from gtls_b200 import _lib
     t, y, dy, widths, tm, ov, maxd = c
     up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda:0")
     tm_ = _lib.Timing()
-    chi2, loc = _lib.search(dict(t=up(t), y=up(y), dy=up(dy), span=float(np.float32(t.max() - t.min()))), up(PERIODS),
+    chi2, loc = _lib.search(dict(t=up(t), y=up(y), dy=up(dy), span=float(np.float32(t.max() - t.min()))), up(periods),
                             dict(widths=up(widths), overshoot=up(ov), templates=up(tm), max_width=maxd), 1e-5, 8, 1,
                             _lib.GTLS_PASS_ALL if all_ else _lib.GTLS_PASS_MAIN, precision, timing=tm_,
                             flags=_lib.GTLS_SEARCH_ALL_DURATIONS)
@@ -107,3 +107,15 @@ def test_fp32_sums_as_few_starts_as_fp64(cuda):
     c[1] = c[1] - 0.01
     tm_ = [_run(c, False, p)[2] for p in ("fp64", "fp32")]
     assert tm_[1].chi2_issued_fma <= 1.02 * tm_[0].chi2_issued_fma, [t.as_dict() for t in tm_]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["ties", "glitches", "flares"])
+def test_a_value_does_not_depend_on_who_sums_it(cuda, kind, precision):
+    """The same period among 300 (whole ranges, and where the list ran over list by
+    list, a warp a window) and alone (short ranges, wide windows by the CTA): the same bits."""
+    n, widths = 19728, _widths(20, 1400, 1.06)
+    c = _odd(kind, n, widths)
+    chi2 = _run(c, False, precision)[0]
+    for i in CHECKED:
+        assert _run(c, False, precision, PERIODS[i:i + 1])[0][0] == chi2[i]
