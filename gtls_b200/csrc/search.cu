@@ -138,6 +138,12 @@ constexpr int kSetupItems = 1024;
 constexpr int kSetupSums = 8;   // E, sum v^2, sum w, sum u^2, min w, max w, sum |u|^(1/2), sum w^(1/2)
 static_assert(kSetupSums <= kSetupThreads / 32, "a warp adds up each");
 
+// Square root of x >= 0 to 6%: the exponent halved and half of the fraction with it
+// (0 becomes 2^-511).
+__device__ __forceinline__ double rough_root(double x) {
+  return __longlong_as_double((__double_as_longlong(x) >> 1) + (1023LL << 51));
+}
+
 __device__ __forceinline__ double sums_join(int k, double x, double y) {
   return k == 4 ? fmin(x, y) : (k == 5 ? fmax(x, y) : x + y);
 }
@@ -170,7 +176,7 @@ constexpr double kSpikeSum = 0x1p30, kSpikeRest = 0x1p28, kSpikeW = 0x1p20;
 // The curve's thresholds of |u| and w (infinite: none), and where there are
 // any its sums 1 to 3 (kSetupSums) without its spikes, by one CTA.
 template <typename Real>
-__device__ void find_spikes(const CurveDev<Real>& C, double typical_u, double typical_w, double (&sums)[4],
+__device__ __noinline__ void find_spikes(const CurveDev<Real>& C, double typical_u, double typical_w, double (&sums)[4],
                             double (&thr)[2]) {
   constexpr int kBins = 96, kFirst = 4;   // |u| of 2^kFirst typical ones on, by powers of two
   __shared__ int hist[kBins], heavy;
@@ -267,8 +273,8 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     s[3] += (v * w) * (v * w);
     s[4] = fmin(s[4], w);
     s[5] = fmax(s[5], w);
-    s[6] += sqrt(fabs(v * w));
-    s[7] += sqrt(w);
+    s[6] += rough_root(fabs(v * w));
+    s[7] += rough_root(w);
   }
 #pragma unroll
   for (int k = 0; k < kSetupSums; ++k) {
@@ -284,10 +290,8 @@ __device__ void curve_setup(const CurveDev<Real>& C, int blk, int nblk) {
     __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();   // the CTA's (v, w) as well
-    last = atomicAdd(C.arrived, 1) == nblk - 1;
-  }
+  // (thread 0's fence above comes after a barrier: it covers the CTA's (v, w) as well)
+  if (threadIdx.x == 0) last = atomicAdd(C.arrived, 1) == nblk - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
