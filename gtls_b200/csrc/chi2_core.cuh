@@ -1,9 +1,10 @@
-// Record and template pair types of the chi2 kernel, and the summation orders
-// of a start's sums written as register-blocked correlations of a template row
-// with the folded records.  The kernel sums single starts in those orders
-// (chi2.cuh); the correlations are the host-callable statement of them that the
-// CPU checks run (the device build uses the packed two-lane FP32 instructions,
-// the host build two scalar FMAs with the same IEEE rounding).
+// Record and template pair types of the chi2 kernel, and the summation order of
+// a start's FP32 sums (products of each offset of a skip block, then the
+// offsets) written as register-blocked correlations of a template row with the
+// folded records.  No kernel calls the correlations: the kernel sums single
+// starts (chi2.cuh), in FP32 in this order, in FP64 in one of its own; they are
+// what the CPU checks of the order run (the device build uses the packed two-lane
+// FP32 instructions, the host build two scalar FMAs with the same IEEE rounding).
 #pragma once
 #include <cuda_runtime.h>
 

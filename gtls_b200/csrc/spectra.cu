@@ -5,9 +5,9 @@
 // Every quantity is a reduction over the spectrum that the next step needs
 // whole (minimum, mean, variance, then the same of the detrended power), so
 // the steps are launches: each writes one partial result per CTA, and every CTA
-// of the next adds those up for itself, in one order.  On 187,850 periods the
-// former single-CTA passes and an all-pairs median per window took 1.28 ms
-// (160 us on 2,592); these take 55 (35).
+// of the next adds those up for itself, in one order.  A call on 187,850 periods
+// with the former single-CTA passes and an all-pairs median per window took 1.28
+// ms (160 us on 2,592); it takes 94 (68), of which the kernels are 55 (35).
 #include <cuda_runtime.h>
 
 #include <algorithm>

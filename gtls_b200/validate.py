@@ -107,8 +107,8 @@ def validate_args(self, kwargs):
     self.rp = kwargs.get("rp", constants.DEFAULT_RP)
     self.a = kwargs.get("a", constants.DEFAULT_A)
     self.T0_fit_margin = kwargs.get("T0_fit_margin", constants.T0_FIT_MARGIN)
-    # precision: "fp64" (plain FP64 search) or "fp32" (FP32 chi2 with
-    # compensated prefix sums; candidates re-evaluated in FP64)
+    # precision: "fp64" (plain FP64 search) or "fp32" (FP32 chi2 with FP64
+    # window means; candidates re-evaluated in FP64)
     self.precision = kwargs.get("precision", "fp64")
     if self.precision not in ("fp64", "fp32"):
         raise ValueError('precision must be "fp64" or "fp32"')

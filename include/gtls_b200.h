@@ -34,12 +34,12 @@ enum gtls_status {
   GTLS_E_CUDA = 2,      /* a CUDA runtime call failed                    */
   GTLS_E_NOMEM = 3,     /* scratch allocation failed                     */
   GTLS_E_RANGE = 4,     /* input outside the supported range             */
-  GTLS_E_DEVICE = 5     /* a kernel reported an error through its status word */
+  GTLS_E_DEVICE = 5     /* the device is not supported, or a device status word was not 0 */
 };
 
 enum gtls_precision {
   GTLS_FP64 = 0,        /* plain FP64 chi2                                */
-  GTLS_FP32 = 1         /* FP32 chi2, compensated FP32 prefix sums, FP64 baseline */
+  GTLS_FP32 = 1         /* FP32 template sums, FP64 window means and baseline */
 };
 
 enum gtls_pass {
@@ -50,7 +50,7 @@ enum gtls_pass {
 typedef struct gtls_ctx gtls_ctx;
 
 /* Create / destroy a context on CUDA device `device`.  The context owns the
- * scratch arena the searches use. */
+ * scratch arena the searches use, and a pool for the calls that do not wait. */
 int gtls_ctx_create(int device, gtls_ctx** out);
 int gtls_ctx_destroy(gtls_ctx* ctx);
 
@@ -262,7 +262,8 @@ int gtls_search_batch(gtls_ctx* ctx, const gtls_batch_desc* desc, void* stream);
  * Spectra of a chi2 array (stats.spectra, stats.py:95-122, with the
  * running median of helpers.py:91-106).  mask may be NULL (nothing masked);
  * masked entries are left out of every min/mean/std/max/median as numpy.ma
- * does.  Outputs sr, power_raw, power: [n]; sde_raw and sde: host scalars.
+ * does.  Outputs sr, power_raw, power: [n] (a caller that wants only the last of
+ * them may pass one array for several); sde_raw and sde: host scalars.
  * kernel = oversampling_factor * 30, made odd.  Synchronises the stream.
  */
 int gtls_spectra(gtls_ctx* ctx, const double* chi2, const uint8_t* mask, int64_t n,
@@ -322,7 +323,10 @@ int gtls_template_cache(gtls_ctx* ctx, const gtls_template_desc* desc, void* str
  * quadrature).  D is the first-to-fourth-contact duration, depth the central
  * depth.  gtls_model_chi2_grad writes grad_params[6c+k] =
  * grad_chi2[c] * dchi2_c/dparam_k, the exact derivative of that discrete
- * formula, recomputing the model instead of storing it.
+ * formula, recomputing the model instead of storing it (NaN where a sample is
+ * not finite).  Both return without waiting for their kernels; their scratch is
+ * allocated in stream order, so calls may overlap on several streams and may be
+ * captured.
  */
 int gtls_model_chi2(gtls_ctx* ctx, const double* t, const double* y, const double* w,
                     const int64_t* curve_off, int32_t n_curves, const double* params,
@@ -341,8 +345,8 @@ int gtls_model_chi2_grad(gtls_ctx* ctx, const double* t, const double* y, const 
  * gtls context (creating one allocates).  Same inputs, outputs and results as
  * gtls_spectra; runs on the current device, needs no context, and calls no
  * allocator: its scratch is a static device array of
- * GTLS_NOALLOC_SCRATCH_BYTES that every GPU loading the library holds until
- * exit.  Limits and rules:
+ * GTLS_NOALLOC_SCRATCH_BYTES, and 28 KB of partial sums after it, that every
+ * GPU loading the library holds until exit.  Limits and rules:
  *   - n <= GTLS_NOALLOC_MAX_PERIODS, else GTLS_E_RANGE (nothing launched);
  *   - all calls on a device share the scratch array, so calls that overlap
  *     on the GPU race; each call writes every scratch value it reads;
