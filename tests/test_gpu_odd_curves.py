@@ -119,3 +119,36 @@ def test_a_value_does_not_depend_on_who_sums_it(cuda, kind, precision):
     chi2 = _run(c, False, precision)[0]
     for i in CHECKED:
         assert _run(c, False, precision, PERIODS[i:i + 1])[0][0] == chi2[i]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_second_searches_in_chunks_and_sets_of_curves(cuda, precision):
+    """Curves of which some have spikes and some periods' lists run over, searched
+    together and in small chunks: the bits of each curve's own search."""
+    import torch
+    from gtls_b200 import _lib
+    kinds = ["flares", "ties", "glitch", "glitches", "sure"]
+    widths = _widths(20, 1400, 1.06)
+    cs = [_odd(k, n, widths) for k, n in zip(kinds, (19728, 15001, 9000, 19728, 12345))]
+    periods = [PERIODS[i::3] for i in range(len(cs))]
+    alone = [_run(c, False, precision, p)[:2] for c, p in zip(cs, periods)]
+    cat = lambda k: torch.from_numpy(np.concatenate([np.ascontiguousarray(c[k]).reshape(-1) for c in cs])).to("cuda:0")
+    off = lambda sizes: np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    curves = dict(t=cat(0), y=cat(1), dy=cat(2), sample_off=off([len(c[0]) for c in cs]),
+                  span=np.array([np.float32(c[0].max() - c[0].min()) for c in cs], dtype=np.float32))
+    tables = dict(widths=cat(3), overshoot=cat(5), templates=cat(4), dur_off=off([len(c[3]) for c in cs]),
+                  tmpl_off=off([c[4].size for c in cs])[:-1], max_width=np.array([c[6] for c in cs], dtype=np.int32))
+    p_off = off([len(p) for p in periods])
+    p_dev = torch.from_numpy(np.concatenate(periods)).to("cuda:0")
+    try:
+        for budget in (8 << 30, 12 << 20):
+            _lib.set_chunk_budget(budget)
+            chi2, loc = _lib.search_batch(curves, p_dev, p_off, tables, 1e-5, 8, np.ones(len(cs), dtype=np.int32),
+                                          _lib.GTLS_PASS_MAIN, precision, flags=_lib.GTLS_SEARCH_ALL_DURATIONS)
+            chi2, loc = chi2.cpu().numpy(), loc.cpu().numpy()
+            for i, (c, l) in enumerate(alone):
+                np.testing.assert_array_equal(chi2[p_off[i]:p_off[i + 1]], c, err_msg=kinds[i])
+                if kinds[i] != "ties":
+                    np.testing.assert_array_equal(loc[p_off[i]:p_off[i + 1]], l, err_msg=kinds[i])
+    finally:
+        _lib.set_chunk_budget(8 << 30)
