@@ -25,13 +25,6 @@ constexpr int kBlockStarts = 64;                 // all-starts pass: consecutive
 constexpr int kBlockSamples = 2048;              // samples of their windows in shared memory at a time
 constexpr int kBlockSlots = 2048;                // blocks of a CTA taken up at a time
 
-// Rounding of a difference of two prefix values, relative to the largest of
-// them: they are summed in FP64 and rounded to FP32 once each.  (Summed in FP32
-// the bound was 2^-16 of the largest; after six flares of 50% it left so many
-// starts that the list ran over: 300 periods of 19,728 samples 18.5 ms, now 0.61,
-// of 70,000 92 and 1.67 ms.  Without flares both take the same time.)
-constexpr float kPrefixErr = 0x1.01p-23f;
-
 // Arrays of prefix values are skewed by one word per 32, so that starts a
 // power of two apart fall into different banks.
 __host__ __device__ __forceinline__ int skew(int p) { return p + (p >> 5); }
@@ -90,17 +83,13 @@ __device__ __forceinline__ NearSpikes near_spikes(const Spike* spikes, int from,
   s.at = spikes + from;
   s.n = min(end, kSpikes) - from;
   s.uniform = uniform;
-  s.err = end > kSpikes ? INFINITY : 1.2e-7f * (float)(s.n + 8);   // (there are no more, by their choice)
+  s.err = end > kSpikes ? INFINITY : spike_err(s.n);   // (there are no more, by their choice)
   return s;
 }
 // One spike that a window holds, where the template is t = (s, s^2).
 template <typename R2>
 __device__ __forceinline__ void add_spike(CellSums& cs, const NearSpikes& s, const R2& t, float u, float w) {
-  const float b = (float)t.x * u, c = s.uniform ? 0.f : (float)t.y * w;
-  cs.B += b;
-  cs.er = fmaf(fabsf(b), s.err, cs.er);
-  cs.cl = fmaf(c, 1.f - s.err, cs.cl);
-  cs.cu = fmaf(c, 1.f + s.err, cs.cu);
+  add_spike(cs, (float)t.x, (float)t.y, u, s.uniform ? 0.f : w, s.err);
 }
 // Those of the lanes' windows of w samples, which start at q (ascending);
 // returns their sum of u^2.

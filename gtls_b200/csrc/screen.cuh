@@ -102,6 +102,13 @@ __host__ __device__ __forceinline__ ScreenErr screen_err(float v, float u, float
   return ScreenErr{v, u, w, fmaf(1026.f * u, u, q + 1e-30f)};
 }
 
+// Rounding of a difference of two prefix values, relative to the largest of
+// them: they are summed in FP64 and rounded to FP32 once each.  (Summed in FP32
+// the bound was 2^-16 of the largest; after six flares of 50% it left so many
+// starts that the list ran over: 300 periods of 19,728 samples 18.5 ms, now 0.61,
+// of 70,000 92 and 1.67 ms.  Without flares both take the same time.)
+constexpr float kPrefixErr = 0x1.01p-23f;
+
 struct StartBounds {
   float lb, ub;
 };
@@ -138,6 +145,19 @@ __host__ __device__ __forceinline__ void add_cell(CellSums& s, const ScreenCell&
   if (kCoarse) s.er = fmaf(c.rb, fabsf(dU) + e.u, s.er);
   s.cl = fmaf(c.mn, dW, s.cl);
   if (kUpper) s.cu = fmaf(c.mx, dW, s.cu);
+}
+
+// A sample that is kept out of the prefix sums (its u and w there are 0) and lies
+// in the window, where the template is s and its square s2: its products, with
+// the rounding of the sums of up to `err`'s count of them.  Where all weights equal wbar,
+// w is 0 here (C is wbar * t2 then).
+__host__ __device__ __forceinline__ float spike_err(int count) { return 1.2e-7f * (float)(count + 8); }
+__host__ __device__ __forceinline__ void add_spike(CellSums& cs, float s, float s2, float u, float w, float err) {
+  const float b = s * u, c = s2 * w;
+  cs.B += b;
+  cs.er = fmaf(fabsf(b), err, cs.er);
+  cs.cl = fmaf(c, 1.f - err, cs.cl);
+  cs.cu = fmaf(c, 1.f + err, cs.cu);
 }
 
 // Bounds of delta (the upper one only with kUpper) for a window of mean depth in [mean - em, mean + em] (scaled
