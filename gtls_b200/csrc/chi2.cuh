@@ -91,28 +91,44 @@ template <typename R2>
 __device__ __forceinline__ void add_spike(CellSums& cs, const NearSpikes& s, const R2& t, float u, float w) {
   add_spike(cs, (float)t.x, (float)t.y, u, s.uniform ? 0.f : w, s.err);
 }
-// Those of the lanes' windows of w samples, which start at q (ascending);
-// returns their sum of u^2.
+// v of a spike, to 3 half ulps; infinite where FP32 does not hold its w (starts
+// whose windows hold it are summed).
+__device__ __forceinline__ float spike_v(const Spike& x) { return x.w > 1e-30f ? x.u / x.w : INFINITY; }
+// Those of the lanes' windows of w samples, which start at q (ascending); returns
+// their sums of v, |v| and u^2.
+struct SpikeSums {
+  float v, av, sq;
+};
 template <typename R2>
-__device__ __forceinline__ float add_spikes(CellSums& cs, const NearSpikes& s, const R2* __restrict__ trow, int q, int w) {
+__device__ __forceinline__ SpikeSums add_spikes(CellSums& cs, const NearSpikes& s, const R2* __restrict__ trow, int q,
+                                                int w) {
   const int lane = threadIdx.x & 31;
   const int from = __shfl_sync(0xffffffffu, q, 0), to = __shfl_sync(0xffffffffu, q, 31) + w;
-  float sq = 0.f;
+  SpikeSums o{0.f, 0.f, 0.f};
   for (int i0 = 0; i0 < s.n; i0 += 32) {
     Spike x{-1, 0.f, 0.f};
     if (i0 + lane < s.n) x = s.at[i0 + lane];
+    const float xv = spike_v(x);
+    __syncwarp();
     for (unsigned m = __ballot_sync(0xffffffffu, x.q >= from && x.q < to); m; m &= m - 1) {
       const int src = __ffs(m) - 1;
       const int i = __shfl_sync(0xffffffffu, x.q, src) - q;
-      const float u = __shfl_sync(0xffffffffu, x.u, src), v = __shfl_sync(0xffffffffu, x.w, src);
+      const float u = __shfl_sync(0xffffffffu, x.u, src), wt = __shfl_sync(0xffffffffu, x.w, src),
+                  v = __shfl_sync(0xffffffffu, xv, src);
       if (i >= 0 && i < w) {
-        add_spike(cs, s, trow[i], u, v);
-        sq = fmaf(u, u, sq);
+        add_spike(cs, s, trow[i], u, wt);
+        o.v += v;
+        o.av += fabsf(v);
+        o.sq = fmaf(u, u, o.sq);
       }
+      __syncwarp();
     }
   }
-  if (s.err == INFINITY) cs.er = INFINITY;
-  return sq;
+  if (s.err == INFINITY) {
+    cs.er = INFINITY;
+    o.av = INFINITY;
+  }
+  return o;
 }
 
 // Per CTA, in units of list entries: the list, (all starts) the blocks, and the spikes.
@@ -683,7 +699,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     const int q0 = ld + (int)threadIdx.x * kItems;   // item i is prefix value q0 + i + 1
     const int have = min(kItems, cnt - (int)threadIdx.x * kItems);
     ++batches;
-    if (spiky) {   // listed in order; their u and w are 0 in what follows
+    if (spiky) {   // listed in order; they are 0 in what follows
       int mine = 0;
 #pragma unroll
       for (int i = 0; i < kItems; ++i) mine += i < have && is_spike(gq[i]);
@@ -703,7 +719,7 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
           const double w = gq[i].y * cc.wscale, u = gq[i].x * cc.vscale * w;
           if (at < kSpikes) spikes[at] = Spike{q0 + i, (float)u, (float)w};
           ++at;
-          gq[i].y = 0.0;
+          gq[i] = make_double2(0.0, 0.0);
         }
       if (threadIdx.x == kChiThreads - 1) spike_end[batches & 3] = at;
     }
@@ -855,6 +871,34 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
       const int q = j * s - k0;   // start within the range
       dv[i] = j < j1 ? v_at(coarse_tag, q) - v_at(coarse_tag, q + w) : -INFINITY;
     }
+    // the spikes that the windows may hold (the ring has samples of the last two batches)
+    NearSpikes near;
+    if constexpr (kSpiky) {
+      const int from = kCoarse ? 0 : spike_end[(batches - 2) & 3];
+      near = near_spikes(spikes, from, spike_end[batches & 3], cc.kind & kUniform);
+    }
+    if constexpr (kSpiky) {   // less their v, with the rounding in the start's favour
+      const int q_lo = j0 * s - k0, q_hi = (j1 - 1) * s - k0 + w;
+      float sv[kTaskGroups] = {};
+      for (int i0 = 0; i0 < near.n; i0 += 32) {
+        Spike x{-1, 0.f, 0.f};
+        if (i0 + lane < near.n) x = near.at[i0 + lane];
+        const float xv = spike_v(x);
+        __syncwarp();
+        for (unsigned m = __ballot_sync(0xffffffffu, x.q >= q_lo && x.q < q_hi); m; m &= m - 1) {
+          const int at_q = __shfl_sync(0xffffffffu, x.q, __ffs(m) - 1);
+          const float v = __shfl_sync(0xffffffffu, xv, __ffs(m) - 1), less = v - fabsf(v) * near.err;
+#pragma unroll
+          for (int i = 0; i < kTaskGroups; ++i) {
+            const int off = at_q - ((j0 + 32 * i + lane) * s - k0);
+            if (off >= 0 && off < w) sv[i] += less;
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kTaskGroups; ++i)
+        if (j0 + 32 * i + lane < j1) dv[i] = near.err < INFINITY && fabsf(sv[i]) < INFINITY ? dv[i] - sv[i] : INFINITY;
+    }
     // a failing start's value n matters at the first one only
     const long long loc0 = (long long)u * n + (long long)j0 * s;
     const bool track = !probe && loc0 < *(volatile long long*)&sent_sm;
@@ -873,12 +917,6 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
     __syncwarp();
     if (a.work && lane == 0 && !probe && !kLate) atomicAdd(&work_sm[0], (unsigned long long)cnt * 2 * (unsigned)w);
     const float gamma = gamma_of(w, kAll ? 1 : (int)(wsk[u] >> 16));
-    // the spikes that the windows may hold (the ring has samples of the last two batches)
-    NearSpikes near;
-    if constexpr (kSpiky) {
-      const int from = kCoarse ? 0 : spike_end[(batches - 2) & 3];
-      near = near_spikes(spikes, from, spike_end[batches & 3], cc.kind & kUniform);
-    }
     for (int b = 0; b < cnt; b += 32) {
       const int k = (j0 + queue[wid][min(b + lane, cnt - 1)]) * s;
       const int q = k - k0;
@@ -903,10 +941,15 @@ chi2_kernel(const CurveDev<Real>* __restrict__ cds, const Run* __restrict__ runs
         pw = nw;
         pq = nq;
       }
-      const float m = (v_at(coarse_tag, q) - v_at(coarse_tag, q + w)) * inv_w;
-      const float em = fmaf(3e-7f, fabsf(m), em0);
+      float m = (v_at(coarse_tag, q) - v_at(coarse_tag, q + w)) * inv_w;
+      float em = fmaf(3e-7f, fabsf(m), em0);
       float qwin = (pq - q00) + (float)(kCoarse ? end * g : w) * cc.qbar + 4.f * e.n2;
-      if constexpr (kSpiky) qwin += add_spikes(cs, near, ex.trows + ex.trow_off[d], q, w);
+      if constexpr (kSpiky) {
+        const SpikeSums o = add_spikes(cs, near, ex.trows + ex.trow_off[d], q, w);
+        m -= o.v * inv_w;
+        em = fmaf(o.av * inv_w, near.err, em) + 3e-7f * fabsf(m);
+        qwin += o.sq;
+      }
       float lb = start_bounds<false>(cs, row_sm[wid][0], m, em, qwin, cc.wbar, cc.kind & kUniform, gamma, e).lb;
       // too close to the depth threshold to tell: such a start needs its exact value (n, if it fails)
       const bool certain = m - em > dthr;

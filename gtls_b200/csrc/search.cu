@@ -159,7 +159,7 @@ __device__ __forceinline__ double unit_scale(double x) {
 // prefix sums, which one sample of a million times the others' |u| (its u^2 a
 // 10^12-fold) or w would leave without a digit for every cell after it: the list of
 // waiting starts ran over, and 300 periods of 70,000 samples with one dy
-// a thousandth of the others took 92 ms (now 1.9; clean 1.8).  Such samples, at most 2
+// a thousandth of the others took 92 ms (now 2.0; clean 1.8).  Such samples, at most 2
 // kSpikeMax of a curve, are left out of the prefix sums and added to the bounds of the
 // windows that hold them.  The sums round to 2^-23 of the whole (kPrefixErr), so a
 // curve has spikes where its sum of u^2 is so far above that of its samples but the largest
@@ -168,8 +168,10 @@ __device__ __forceinline__ double unit_scale(double x) {
 // A sample is a spike from the largest power of two (times the typical |u|)
 // on below which that rounding is at most 32.  Typical is the square of the mean
 // square root, which spikes hardly move; curves whose sum is below 2^30 typical
-// ones are not looked at.
-constexpr int kSpikeMax = 256;
+// ones are not looked at.  1,024, not 256 with their v in the prefix sums: 300 periods of
+// 70,000 samples, 700 of them up to 400 times the flux, 4.3 ms (39; dense sums 2.1);
+// 350 up to 5 times 2.3 (11.4; 2.1); 700 lowered by up to 80% 2.8 (2.1; 3.7).
+constexpr int kSpikeMax = 1024;
 constexpr int kSpikes = 4 * kSpikeMax;   // of a CTA: a window may run once more around the curve
 constexpr double kSpikeSum = 0x1p30, kSpikeRest = 0x1p28, kSpikeW = 0x1p20;
 

@@ -35,8 +35,11 @@ def _odd(kind, n, widths):
     elif kind == "sure_flat":    # and one of v = 0
         dy[[n // 3, n // 2]] /= 3000.0
         y[n // 2] = 1.0
-    elif kind == "glitches":     # more than are left out of the prefix sums, up to 400 times the flux
-        y[rng.integers(0, n, 700)] *= np.exp(rng.uniform(0.0, 6.0, 700))
+    elif kind in ("glitches", "crowd"):   # up to 400 times the flux; a crowd: more than are left out of the prefix sums
+        k = 700 if kind == "glitches" else 6000
+        y[rng.integers(0, n, k)] *= np.exp(rng.uniform(0.0, 6.0, k))
+    elif kind == "lost":         # one sample whose weight FP32 does not hold beside the others'
+        y[n // 3], dy[n // 3] = 1e30, dy[n // 3] * 1e20
     elif kind == "ties":         # every start of a duration has the same value
         y[:] = 1.0 - 1e-3
         dy[:] = 1e-3
@@ -80,12 +83,12 @@ def test_most_starts_are_ruled_out(cuda, kind, all_, n, widths):
         assert tm_.chi2_issued_fma <= 0.1 * tm_.chi2_active_fma, (precision, tm_.as_dict())
 
 
-@pytest.mark.parametrize("kind", ["ties", "glitches"])
+@pytest.mark.parametrize("kind", ["ties", "glitches", "crowd", "lost"])
 @pytest.mark.parametrize("n,widths", [(19728, _widths(20, 1400, 1.06)), (40000, _widths(40, 4500, 1.08))])
 def test_what_the_list_cannot_hold_is_summed_once_at_most(cuda, kind, n, widths):
     """Where the list of a CTA runs over: starts that all tie (the widest duration
-    rules out the others in the end) and more glitches than are set apart.  Not
-    more is summed than starts that pass."""
+    rules out the others in the end), many glitches, more than are set apart, and
+    a sample whose v is known to no window.  Not more is summed than starts that pass."""
     c = _odd(kind, n, widths)
     t, y, dy, widths, tm, ov, maxd = c
     back = O.NumpyBackend()
@@ -110,7 +113,7 @@ def test_fp32_sums_as_few_starts_as_fp64(cuda):
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
-@pytest.mark.parametrize("kind", ["ties", "glitches", "flares"])
+@pytest.mark.parametrize("kind", ["ties", "glitches", "crowd", "flares"])
 def test_a_value_does_not_depend_on_who_sums_it(cuda, kind, precision):
     """The same period among 300 (whole ranges, and where the list ran over list by
     list, a warp a window) and alone (short ranges, wide windows by the CTA): the same bits."""
@@ -127,7 +130,7 @@ def test_second_searches_in_chunks_and_sets_of_curves(cuda, precision):
     together and in small chunks: the bits of each curve's own search."""
     import torch
     from gtls_b200 import _lib
-    kinds = ["flares", "ties", "glitch", "glitches", "sure"]
+    kinds = ["flares", "ties", "glitch", "crowd", "sure"]
     widths = _widths(20, 1400, 1.06)
     cs = [_odd(k, n, widths) for k, n in zip(kinds, (19728, 15001, 9000, 19728, 12345))]
     periods = [PERIODS[i::3] for i in range(len(cs))]
